@@ -234,13 +234,16 @@ int mirt_interp_plan_adjoint(mirt_interp_plan *plan, const void *fm, void *ck, v
  * bitwise deterministic for any choice. */
 int mirt_interp_plan_autotune(mirt_interp_plan *plan, void *stream);
 
-/* Current launch configuration: up to 23 values
+/* Current launch configuration: up to 24 values
  * {T1, T2, T3, spread threads, spread heavy-first order, coil lanes,
  *  gather threads, (unused), gather CTAs, B1, B2, B3, split chunk,
  *  spread tasks, spare tile columns, partial-tile reductions,
  *  spread shared-tile atomics, ownership spread, row-sweep segments (0: off,
  *  -1: balanced team list), row-sweep rows per band, TMA gather,
- *  row-sweep dense-bin patches, staged row sweep mode}. */
+ *  row-sweep dense-bin patches, staged row sweep mode, column lanes of the
+ *  point spread (0: off)}.  The point spread is the default where the sweeps
+ *  are not; mirt_interp_plan_set_sweep, _set_spread and _set_ownership turn
+ *  it off. */
 int mirt_interp_plan_config(mirt_interp_plan *plan, int32_t *out, int32_t n);
 
 /* Adjoint accumulation order.  deterministic = 1 (the default): every

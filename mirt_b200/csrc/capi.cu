@@ -515,6 +515,61 @@ int set_line_sweep3(mirt_interp_plan *P, int nseg, cudaStream_t st) {
   return MIRT_OK;
 }
 
+// Point spread: the split of every base tile from the sort's bins, and the task
+// list, most split tiles first.
+int build_points(mirt_interp_plan *P, cudaStream_t st) {
+  const InterpArgs &a = P->a;
+  Tiling &t = P->t;
+  const int shape = points_shape(a.C);
+  const long long n = points_tiles(a, shape, t.nslice);
+  if (n < 1 || n >= (1ll << 30)) return MIRT_OK;
+  DMem lgd;
+  CK(lgd.alloc(n));
+  CK(P->pt_hdr.alloc(std::max<long long>(a.Mtot, 1) * sizeof(int4)));
+  CK(launch_points_split(a, t, shape, t.nslice, P->bin_start.as<int>(), lgd.as<unsigned char>(),
+                         P->pt_hdr.as<int4>(), st));
+  std::vector<unsigned char> lg(n);
+  CK(cudaMemcpyAsync(lg.data(), lgd.p, n, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  long long cnt[32] = {0};
+  for (unsigned char l : lg) cnt[l] += 1ll << l;
+  long long at[32], total = 0;
+  for (int l = 31; l >= 0; l--) {
+    at[l] = total;
+    total += cnt[l];
+  }
+  if (total >= (1ll << 31)) return MIRT_OK;
+  const int lc = points_cta_log2(shape);
+  std::vector<int4> task(total);
+  long long slots = 0;
+  for (long long i = 0; i < n; i++)
+    for (int k = 0; k < 1 << lg[i]; k++) {
+      int4 e = make_int4((int)i, k | lg[i] << 16, 0, 0);
+      if (lg[i] > lc) {  // the CTAs of a brick are consecutive
+        e.z = (int)slots;
+        e.w = (int)(slots - (k & ((1 << (lg[i] - lc)) - 1)));
+        slots++;
+      }
+      task[at[lg[i]]++] = e;
+    }
+  const size_t nch = points_chunks(shape, a.C);
+  CK(P->pt_task.alloc(std::max<long long>(total, 1) * sizeof(int4)));
+  CK(P->pt_scratch.alloc(slots * nch * points_slot_bytes(shape)));
+  CK(P->pt_count.alloc(slots * nch * sizeof(int)));
+  if (total)
+    CK(cudaMemcpyAsync(P->pt_task.p, task.data(), total * sizeof(int4), cudaMemcpyHostToDevice, st));
+  if (slots) CK(cudaMemsetAsync(P->pt_count.p, 0, slots * nch * sizeof(int), st));
+  CK(cudaStreamSynchronize(st));
+  t.pt_task = P->pt_task.as<int4>();
+  t.n_pt_task = (int)total;
+  t.pt_slots = (int)slots;
+  t.pt_scratch = P->pt_scratch.as<float2>();
+  t.pt_count = P->pt_count.as<int>();
+  t.pt_hdr = P->pt_hdr.as<int4>();
+  P->points_shape = shape;
+  return MIRT_OK;
+}
+
 // Uniform segments: the work queue of their teams.
 int set_uniform_sweep(mirt_interp_plan *P, int nseg, int rows, cudaStream_t st) {
   P->t.sweep = nseg;
@@ -596,6 +651,13 @@ void choose_config(mirt_interp_plan *P) {
   t.own = 0;
   t.sweep = 0;
   t.sweep_rows = 1;
+  t.points = 0;
+  t.pt_task = nullptr;
+  t.n_pt_task = 0;
+  t.pt_hdr = nullptr;
+  t.pt_slots = 0;
+  t.pt_scratch = nullptr;
+  t.pt_count = nullptr;
   t.sorted = nullptr;
   t.slice0 = 0;
   t.pos0 = 0;
@@ -1055,6 +1117,12 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     rc3 = set_line_sweep3(P, 2, st);
     if (rc3) return rc3;
   }
+  // everything else: the point spread
+  if (!P->t.sweep && a.C > 0) {
+    int rc3 = build_points(P, st);
+    if (rc3) return rc3;
+    P->t.points = P->points_shape;
+  }
   return MIRT_OK;
 }
 
@@ -1081,6 +1149,7 @@ struct SpreadCand {
   int threads, padc, atomic, own, sweep, sweep_rows;
   int dense = 0;  // 2D row sweep with dense-bin patches (one-row bands)
   int staged = 0;  // 2D row sweep staged per column (1), reading the caller's samples (2)
+  int points = 0;  // point spread (its column lanes)
 };
 
 // spare columns the J = 6 row update can use (0 elsewhere)
@@ -1336,6 +1405,11 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     for (int nseg : {1, 2, 4, 8})
       cands.push_back(SpreadCand{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0,
                                  nseg, 1});
+  if (P->points_shape) {
+    SpreadCand c{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, 0, 1};
+    c.points = P->points_shape;
+    cands.push_back(c);
+  }
   SpreadCand best{};
   float best_ms = 1e30f;
   int built_rows = 0;  // rows of the team list last built
@@ -1345,6 +1419,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     P->t.sweep_rows = c.sweep_rows;
     P->t.dense_on = c.dense;
     P->t.sweep_staged = c.staged;
+    P->t.points = c.points;
     if (c.sweep < 0 && built_rows != c.sweep_rows) {
       int rc = build_sweep_teams(P, c.sweep_rows, 65536, st);
       if (rc) return rc;
@@ -1369,9 +1444,9 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     if (autotune_log())
       std::fprintf(stderr,
                    "mirt autotune spread: tile %dx%dx%d threads %d padc %d atomic %d own %d "
-                   "sweep %d rows %d dense %d staged %d: %.3f ms\n",
+                   "sweep %d rows %d dense %d staged %d points %d: %.3f ms\n",
                    c.T[0], c.T[1], c.T[2], c.threads, c.padc, c.atomic, c.own, c.sweep,
-                   c.sweep_rows, c.dense, c.staged, ms);
+                   c.sweep_rows, c.dense, c.staged, c.points, ms);
     if (ms < best_ms) {
       best_ms = ms;
       best = c;
@@ -1383,6 +1458,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     P->t.sweep_rows = best.sweep_rows;
     P->t.dense_on = best.dense;
     P->t.sweep_staged = best.staged;
+    P->t.points = best.points;
     if (best.sweep < 0 && built_rows != best.sweep_rows) {
       int rc = build_sweep_teams(P, best.sweep_rows, 65536, st);
       if (rc) return rc;
@@ -1398,7 +1474,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     P->ls.atomic = best.atomic;
   }
   // split size of heavy tiles (sample visits per spread task)
-  if (!P->t.sweep) {
+  if (!P->t.sweep && !P->t.points) {
     int best_chunk = P->split_chunk;
     float bc_ms = 1e30f;
     for (int chunk : {256, 512, 1024, 2048, 4096, 16384}) {
@@ -1483,12 +1559,12 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
 int mirt_interp_plan_config(mirt_interp_plan *P, int32_t *out, int32_t n) {
   if (!P || !out) return fail(MIRT_ERR_ARG, "NULL argument");
   P = launch_plan(P);
-  const int32_t v[23] = {P->t.T[0], P->t.T[1], P->t.T[2], P->ls.threads, P->heavy_first, P->ls.cw,
+  const int32_t v[24] = {P->t.T[0], P->t.T[1], P->t.T[2], P->ls.threads, P->heavy_first, P->ls.cw,
                          P->lg.threads, P->lg.sb, P->lg.grid, P->t.B[0], P->t.B[1], P->t.B[2],
                          P->split_chunk, P->t.ntask, P->t.padc, P->t.nred, P->ls.atomic,
                          P->t.own, P->t.sweep, P->t.sweep_rows, P->gtma, P->t.dense_on,
-                         P->t.sweep_staged};
-  for (int i = 0; i < n && i < 23; i++) out[i] = v[i];
+                         P->t.sweep_staged, P->t.points};
+  for (int i = 0; i < n && i < 24; i++) out[i] = v[i];
   return MIRT_OK;
 }
 
@@ -1536,6 +1612,7 @@ int mirt_interp_plan_set_sweep(mirt_interp_plan *P, int32_t segments, int32_t ro
                                 "chunks of 8, 16 or 32");
     if (segments < 0 || segments > P->a.g.K[0])
       return fail(MIRT_ERR_ARG, "3D line-sweep segments must be in 1..K1 (0: off)");
+    P->t.points = 0;
     if (segments) {
       int rc = sweep_buffer(P);
       if (rc) return rc;
@@ -1550,6 +1627,7 @@ int mirt_interp_plan_set_sweep(mirt_interp_plan *P, int32_t segments, int32_t ro
     return fail(MIRT_ERR_ARG, "row-sweep segments must be in 1..K1 (0: off, -1: balanced)");
   if (segments && rows != 1 && rows != 2 && rows != 4)
     return fail(MIRT_ERR_ARG, "row-sweep rows per band must be 1, 2 or 4");
+  P->t.points = 0;
   if (segments) {
     int rc = sweep_buffer(P);
     if (rc) return rc;
@@ -1597,6 +1675,7 @@ int mirt_interp_plan_set_ownership(mirt_interp_plan *P, int32_t own, void *strea
     return fail(MIRT_ERR_ARG, "ownership spread needs 2D, J = 6, tiles of >= 5 points and an "
                               "even number of tiles (last one >= 5 points) per dimension");
   P->t.own = own ? 1 : 0;
+  P->t.points = 0;
   if (own) {
     P->ls.atomic = 0;
     P->t.sweep = 0;
@@ -1649,6 +1728,7 @@ int mirt_interp_plan_set_spread(mirt_interp_plan *P, const int32_t *T, int32_t t
   P->t.padc = padc;
   P->ls.threads = threads;
   P->t.sweep = 0;
+  P->t.points = 0;
   int rc = set_spread_tiles(P, Tn, st);
   if (rc) return rc;
   CK(cudaStreamSynchronize(st));
@@ -3075,8 +3155,9 @@ int mirt_nufft_config(mirt_nufft *p, int32_t *out, int32_t n) {
   const Tiling &t = p->ip->t;
   // gather: one launch (TMA-staged or plain)
   const int fwd = (p->own_fft ? p->gg.D : 2) + 1;
-  int spread = 1;
-  if (t.sweep != 0) {
+  int spread = 1;  // the point spread: one launch
+  if (t.points && !p->ip->ls.atomic) {
+  } else if (t.sweep != 0) {
     // ordering pass, dense-bin patches (chunk sums, per-bin sums), sweep (and a
     // memset of the queue counters)
     const bool dense = t.ndense > 0 && (a3d(p) || (t.dense_on && t.sweep_rows == 1));

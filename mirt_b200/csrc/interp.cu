@@ -227,6 +227,7 @@ cudaError_t launch_mark_dense(const int *dense_bin, int n, int *dense_of, cudaSt
 cudaError_t launch_spread(const InterpArgs &a, const Tiling &t, const Launch &l,
                           const int *bin_start, const float2 *fm, float2 *ck, cudaStream_t st) {
   if (a.C == 0) return cudaSuccess;
+  if (t.points && !l.atomic) return launch_spread_points(a, t, bin_start, fm, ck, st);
   Launch lc = l;
   detail::Req r{detail::SPREAD, &a, &t, &lc, bin_start, fm, ck, st};
   return dispatch(r);

@@ -105,6 +105,18 @@ struct Tiling {
   const int *dense_part0;
   float2 *patch_part;
   int chunk0, nchunks;
+  // Point spread (spread_points.cu): its lane shape, 8 x column lanes + columns
+  // per lane (0: off), and its tasks (base tile, part | log2 split << 16, slot,
+  // first slot of the brick), most split first.  CTAs that share a brick leave
+  // their sums in pt_slots scratch slots per column chunk; pt_count[first slot]
+  // counts the ones that have (zero between launches).
+  int points;
+  const int4 *pt_task;
+  int n_pt_task;
+  int pt_slots;
+  float2 *pt_scratch;
+  int *pt_count;
+  const int4 *pt_hdr;    // per position: first tap k1, caller's sample index, phase (float bits)
   int color_beg[9];
   int red_beg[9];
   int padc;              // spread: spare columns on each side of a tile row in
@@ -203,6 +215,22 @@ cudaError_t query_gather_grid(const InterpArgs &a, Launch &l);
 // fm[m][c] = sum_taps h * ck   for every sample (forward gather)
 cudaError_t launch_gather(const InterpArgs &a, const Launch &l, const float2 *ck,
                           float2 *fm, cudaStream_t st);
+
+// Point spread (spread_points.cu): the lane shape for C columns, the base tiles
+// of nslice slices (0: the geometry does not fit it), and the log2 split of each
+// of them (from the sort's bins) with the positions' headers.  A tile of split
+// 2^l is 2^l consecutive tasks; points_cta_log2: the l up to which a brick's
+// groups are one CTA's, beyond it 2^(l - points_cta_log2) CTAs share a brick
+int points_cta_log2(int shape);
+size_t points_slot_bytes(int shape);
+int points_chunks(int shape, int C);
+int points_shape(int C);
+long long points_tiles(const InterpArgs &a, int shape, int nslice);
+cudaError_t launch_points_split(const InterpArgs &a, const Tiling &t, int shape, int nslice,
+                                const int *bin_start, unsigned char *lg, int4 *hdr,
+                                cudaStream_t st);
+cudaError_t launch_spread_points(const InterpArgs &a, const Tiling &t, const int *bin_start,
+                                 const float2 *fm, float2 *ck, cudaStream_t st);
 
 // dense_of[dense_bin[i]] = i for i < n (dense_of cleared to -1 first)
 cudaError_t launch_mark_dense(const int *dense_bin, int n, int *dense_of, cudaStream_t st);

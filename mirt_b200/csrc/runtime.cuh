@@ -74,6 +74,8 @@ struct mirt_interp_plan {
   mirt::DMem sweep_teams;  // row-sweep spread: balanced team list (int4 per team)
   std::vector<int4> team_host;  // the same list on the host
   mirt::DMem team_order, team_next;  // row-sweep work queue: heaviest-first order, counter
+  mirt::DMem pt_task, pt_hdr, pt_scratch, pt_count;  // point spread (Tiling)
+  int points_shape = 0;              // its lane shape (0: the plan has none)
   mirt::DMem dense_of, dense_bin, patch;  // the sweeps' dense bins and their patches
   mirt::DMem dense_chunk, dense_part0, patch_part;  // chunks of the patch sums
   std::vector<int> dense_slice;           // first dense bin of each slice (+ total)

@@ -858,3 +858,60 @@ def test_tma_gather_bounded_wait_fault_path():
     ref = oracle.interp_for(ck, h, J, L, tm, K, 0, impl=ref_impl(), nthreads=8)
     assert rel_l2(got, ref) <= FWD_TOL
     plan.close()
+
+
+POINT_CASES = [
+    # K, J, columns, table kind: blocks of four points cut at the grid's end, J = K,
+    # odd and unequal J, every lane shape (1..4, 6, 8, 12, 16, 24, 32 columns a
+    # chunk, idle columns, several chunks)
+    ([64], [6], 1, "cx0"), ([7], [7], 3, "cx0"), ([130], [5], 33, "re1"),
+    ([64, 48], [6, 6], 1, "cx0"), ([63, 50], [6, 6], 2, "re1"), ([6, 6], [6, 6], 4, "cx0"),
+    ([66, 41], [5, 4], 5, "cx0"), ([48, 33], [7, 6], 7, "re0"), ([37, 64], [6, 6], 12, "cx0"),
+    ([40, 44], [6, 6], 15, "re1"), ([45, 38], [6, 6], 24, "cx0"), ([34, 30], [6, 6], 31, "cx0"),
+    ([33, 35], [5, 5], 49, "cx0"),
+    ([20, 18, 16], [6, 6, 6], 1, "cx0"), ([6, 7, 9], [6, 6, 6], 2, "re1"),
+    ([13, 14, 17], [5, 6, 4], 3, "cx0"), ([16, 12, 10], [4, 5, 3], 9, "re0"),
+]
+
+
+@pytest.mark.parametrize("K,J,C,variant", POINT_CASES)
+def test_point_spread_matches_oracle(K, J, C, variant):
+    """The point spread (the default where the sweeps are not): a sparse slice
+    with coordinates that wrap several times, an empty one and one so dense that
+    bricks are shared by the groups of a CTA and by several CTAs; with a
+    per-sample phase; the oracle's adjoint, the same bits on a second call, and
+    the tiled spread's result to FP32 rounding."""
+    import torch
+    D = len(K)
+    rng = np.random.default_rng(sum(K) + 100 * C)
+    L = [256] * D
+    n = [max(2, k // 2) for k in K]
+    if variant == "cx0":
+        h = [mb.minmax_kb_table(n[d], J[d], K[d], L[d]) for d in range(D)]
+    else:
+        h = [mb.newfft_kb_table(J[d], L[d]) for d in range(D)]
+    order = 1 if variant == "re1" else 0
+    tms = [rng.uniform(-3 * max(K), 3 * max(K), (300, D)), np.zeros((0, D)),
+           rng.uniform(-1.5, 1.5, (4000, D))]
+    moff = np.concatenate([[0], np.cumsum([len(t) for t in tms])])
+    tm = np.concatenate(tms)
+    ph = np.exp(1j * rng.uniform(0, 6, len(tm)))
+    plan = mb.InterpPlan(K, J, L, h, tm, C, order=order, slice_moff=moff, phase=ph)
+    assert plan.config()["spread_points"] > 0
+    fm = rng.standard_normal((len(tm), C)) + 1j * rng.standard_normal((len(tm), C))
+    fm_d = torch.from_numpy(fm.astype(np.complex64)).cuda()
+    out = plan.adjoint(fm_d).cpu().numpy()
+    assert np.array_equal(out, plan.adjoint(fm_d).cpu().numpy())
+    for s in range(3):
+        sl = slice(moff[s], moff[s + 1])
+        got = np.transpose(out[s], tuple(range(D - 1, -1, -1)) + (D,)).reshape(-1, C, order="F")
+        if not len(tms[s]):
+            assert not got.any()
+            continue
+        ref = oracle.interp_adj(fm[sl] * np.conj(ph[sl])[:, None], h, J, L, tms[s], K, order,
+                                impl=ref_impl())
+        assert rel_l2(got, ref) <= ADJ_TOL, s
+    plan.set_spread([min(8, k) for k in K])
+    assert plan.config()["spread_points"] == 0
+    assert rel_l2(plan.adjoint(fm_d).cpu().numpy(), out) <= 5e-6
+    plan.close()
