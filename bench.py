@@ -444,6 +444,8 @@ def run_gpu(args, w):
     rows, staged = tuned.get("spread_sweep_rows", 1), tuned.get("spread_staged", 0)
     if D == 3:
         sweep_kernel = "spread_sweep3_kernel"
+    elif tuned.get("spread_split", 0):
+        sweep_kernel = "spread_sweep2s_kernel + spread_points_kernel (dense tiles)"
     elif staged == 2:
         sweep_kernel = f"spread_sweep2s_kernel rows={rows} (caller-order samples)"
     elif staged == 1:

@@ -234,16 +234,19 @@ int mirt_interp_plan_adjoint(mirt_interp_plan *plan, const void *fm, void *ck, v
  * bitwise deterministic for any choice. */
 int mirt_interp_plan_autotune(mirt_interp_plan *plan, void *stream);
 
-/* Current launch configuration: up to 24 values
+/* Current launch configuration: up to 25 values
  * {T1, T2, T3, spread threads, spread heavy-first order, coil lanes,
  *  gather threads, (unused), gather CTAs, B1, B2, B3, split chunk,
  *  spread tasks, spare tile columns, partial-tile reductions,
  *  spread shared-tile atomics, ownership spread, row-sweep segments (0: off,
  *  -1: balanced team list), row-sweep rows per band, TMA gather,
- *  row-sweep dense-bin patches, staged row sweep mode, column lanes of the
- *  point spread (0: off)}.  The point spread is the default where the sweeps
- *  are not; mirt_interp_plan_set_sweep, _set_spread and _set_ownership turn
- *  it off. */
+ *  row-sweep dense-bin patches, staged row sweep mode, lane shape of the point
+ *  spread (0: off), split spread}.  The point spread is the default where the
+ *  sweeps are not, the split spread (the staged row sweep with the point spread
+ *  on dense tiles) in 2D from 25 columns; mirt_interp_plan_set_sweep,
+ *  _set_spread and _set_ownership turn them off, and where the row sweep is
+ *  selected beneath the split spread (32 columns and more) so do _set_dense and
+ *  _set_staged. */
 int mirt_interp_plan_config(mirt_interp_plan *plan, int32_t *out, int32_t n);
 
 /* Adjoint accumulation order.  deterministic = 1 (the default): every

@@ -256,12 +256,19 @@ int sweep_buffer(mirt_interp_plan *P) {
 // in all, in grid order (neighbouring bands read the same samples, so they
 // run together; heaviest-first order measured slower at full size).  Teams
 // write disjoint points, each summed in the same fixed order.
+// Columns from which the split spread is the default (2D, J = 6): its sweep's
+// lanes are 32 columns whatever their use, while the point spread's chunks fit
+// the columns (20 columns, 115,968 samples on 384^2: 151 against 139 us; 24
+// columns, 145,920 on 5 x 384^2: 203 and 200 us; 32 columns, 204,800 on 512^2:
+// 240 us against 313 us of the unstaged sweep with dense-bin patches).
+constexpr int kSplitColumns = 25;
 // bins with at least this many samples are summed into patches before a sweep
 constexpr int kDenseBin = 16;
 
 // Visits per bin column of every band of `rows` grid rows: vb[(s * nband +
 // band) * K1 + x] = samples in bin column x of the band's rows + 5 bin rows.
-int sweep_band_visits(mirt_interp_plan *P, int rows, cudaStream_t st, std::vector<float> &vb) {
+int sweep_band_visits(mirt_interp_plan *P, int rows, cudaStream_t st, std::vector<float> &vb,
+                      bool patches = true) {
   const InterpArgs &a = P->a;
   const Tiling &t = P->t;
   const int K1 = a.g.K[0], K2 = a.g.K[1], S = t.nslice, NQ = rows + 5;
@@ -282,7 +289,7 @@ int sweep_band_visits(mirt_interp_plan *P, int rows, cudaStream_t st, std::vecto
         for (int x = 0; x < K1; x++) {
           const int n = br[x + 1] - br[x];
           // a dense bin costs its patch rows, not its samples
-          v[x] += (float)(P->t.dense_of && n >= kDenseBin ? 6 : n);
+          v[x] += (float)(patches && P->t.dense_of && n >= kDenseBin ? 6 : n);
         }
       }
     }
@@ -290,6 +297,21 @@ int sweep_band_visits(mirt_interp_plan *P, int rows, cudaStream_t st, std::vecto
   return MIRT_OK;
 }
 
+// Split spread: a tile is dense when a brick of it takes more samples than one
+// warp's share of the whole cost (heaviest teams run first, so a team up to that
+// share ends with the rest), and a team takes about a third of a share.  Measured
+// on batches of 1, 4, 16 and 64 slices (K = 512^2, 32 columns): shares of 0.3, 0.6,
+// 1.0, 1.5 and 2.5 give 299, 240, 254, 250, 327 us (1), 484, 457, 443, 553, 572 us
+// (4) and 1372, 1346, 1393, 1573, 1535 us (16); teams of 1/2, 1/4, 1/8 share 4667,
+// 4532, 4545 us (64).
+constexpr double kSplitDense = 1.0, kSplitTeams = 3;
+// ... and in any case when a brick (a window of 81 bins, 36 of them a point's)
+// takes more than this many, so that no point of the sweep sums over about 450
+// samples one after another, as many as the bins below the dense-bin threshold
+// make there.  Error of the 64-slice batch's adjoint against FP64, and its time:
+// 1024: 1.6e-7, 4926 us; 2048: 2.8e-7, 4843 us; no limit 1.6e-6, 4530 us; the
+// unstaged sweep with dense-bin patches 2.1e-7, 9305 us.
+constexpr double kSplitMost = 1024;
 // cost of a team: its visits (five warm-up columns included) + 2 per column step
 constexpr double kSweepColumnCost = 2.0;
 
@@ -387,6 +409,13 @@ int build_sweep_teams(mirt_interp_plan *P, int rows, long long target, cudaStrea
   t.sweep = -1;
   t.sweep_rows = rows;
   return build_sweep_order(P, vb, st);
+}
+
+// The balanced team list of the row sweep's default (one-row bands, about 64k
+// teams), made when it is first needed.
+int sweep_teams_ready(mirt_interp_plan *P, cudaStream_t st) {
+  if (P->t.sweep >= 0 || P->t.sweep_team) return MIRT_OK;
+  return build_sweep_teams(P, P->t.sweep_rows, 65536, st);
 }
 
 // The sweeps' dense bins: bins with at least `minc` samples (0: none), their
@@ -515,35 +544,32 @@ int set_line_sweep3(mirt_interp_plan *P, int nseg, cudaStream_t st) {
   return MIRT_OK;
 }
 
-// Point spread: the split of every base tile from the sort's bins, and the task
-// list, most split tiles first.
-int build_points(mirt_interp_plan *P, cudaStream_t st) {
+// Point spread: its task list from the tiles' counts (the most samples that
+// reach a brick), tiles with at most `over` left out, most split tiles first.
+int build_point_tasks(mirt_interp_plan *P, int shape, const std::vector<int> &most, int over,
+                      cudaStream_t st) {
   const InterpArgs &a = P->a;
   Tiling &t = P->t;
-  const int shape = points_shape(a.C);
-  const long long n = points_tiles(a, shape, t.nslice);
-  if (n < 1 || n >= (1ll << 30)) return MIRT_OK;
-  DMem lgd;
-  CK(lgd.alloc(n));
-  CK(P->pt_hdr.alloc(std::max<long long>(a.Mtot, 1) * sizeof(int4)));
-  CK(launch_points_split(a, t, shape, t.nslice, P->bin_start.as<int>(), lgd.as<unsigned char>(),
-                         P->pt_hdr.as<int4>(), st));
-  std::vector<unsigned char> lg(n);
-  CK(cudaMemcpyAsync(lg.data(), lgd.p, n, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  long long cnt[32] = {0};
-  for (unsigned char l : lg) cnt[l] += 1ll << l;
-  long long at[32], total = 0;
+  const long long n = (long long)most.size();
+  long long ntile = 0;
+  for (int m : most) ntile += m > over;
+  std::vector<unsigned char> lg(n, 0);
+  long long cnt[32] = {0}, at[32], total = 0;
+  for (long long i = 0; i < n; i++)
+    if (most[i] > over) {
+      lg[i] = (unsigned char)points_split(a, shape, most[i], ntile);
+      cnt[lg[i]] += 1ll << lg[i];
+    }
   for (int l = 31; l >= 0; l--) {
     at[l] = total;
     total += cnt[l];
   }
-  if (total >= (1ll << 31)) return MIRT_OK;
+  if (total >= (1ll << 31)) return fail(MIRT_ERR_ARG, "too many spread tasks");
   const int lc = points_cta_log2(shape);
   std::vector<int4> task(total);
   long long slots = 0;
   for (long long i = 0; i < n; i++)
-    for (int k = 0; k < 1 << lg[i]; k++) {
+    for (int k = 0; most[i] > over && k < 1 << lg[i]; k++) {
       int4 e = make_int4((int)i, k | lg[i] << 16, 0, 0);
       if (lg[i] > lc) {  // the CTAs of a brick are consecutive
         e.z = (int)slots;
@@ -560,13 +586,129 @@ int build_points(mirt_interp_plan *P, cudaStream_t st) {
     CK(cudaMemcpyAsync(P->pt_task.p, task.data(), total * sizeof(int4), cudaMemcpyHostToDevice, st));
   if (slots) CK(cudaMemsetAsync(P->pt_count.p, 0, slots * nch * sizeof(int), st));
   CK(cudaStreamSynchronize(st));
+  t.points = shape;
   t.pt_task = P->pt_task.as<int4>();
   t.n_pt_task = (int)total;
   t.pt_slots = (int)slots;
   t.pt_scratch = P->pt_scratch.as<float2>();
   t.pt_count = P->pt_count.as<int>();
   t.pt_hdr = P->pt_hdr.as<int4>();
+  return MIRT_OK;
+}
+
+// The tiles' counts and the positions' headers; empty when the geometry does
+// not fit the point spread.
+int point_counts(mirt_interp_plan *P, int shape, cudaStream_t st, std::vector<int> &most) {
+  const long long n = points_tiles(P->a, shape, P->t.nslice);
+  most.clear();
+  if (n < 1 || n >= (1ll << 30)) return MIRT_OK;
+  DMem d;
+  CK(d.alloc(n * sizeof(int)));
+  CK(P->pt_hdr.alloc(std::max<long long>(P->a.Mtot, 1) * sizeof(int4)));
+  CK(launch_points_count(P->a, P->t, shape, P->t.nslice, P->bin_start.as<int>(), d.as<int>(),
+                         P->pt_hdr.as<int4>(), st));
+  most.resize(n);
+  CK(cudaMemcpyAsync(most.data(), d.p, n * sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  return MIRT_OK;
+}
+
+int build_points(mirt_interp_plan *P, cudaStream_t st) {
+  const int shape = points_shape(P->a.C);
+  std::vector<int> most;
+  int rc = point_counts(P, shape, st, most);
+  if (rc || most.empty()) return rc;
   P->points_shape = shape;
+  return build_point_tasks(P, shape, most, -1, st);
+}
+
+// The staged sweep's records (FFMA2 operand pairs of the taps).
+int build_sweep_records(mirt_interp_plan *P, cudaStream_t st) {
+  const long long M = P->a.Mtot;
+  CK(P->wsw.alloc(std::max<long long>(M, 1) * 9 * sizeof(float4)));
+  if (M > 0)
+    mirt_plan_kernels::sweep_records_kernel<<<(unsigned)((M + 255) / 256), 256, 0, st>>>(
+        P->a.W, M, P->wsw.as<float4>());
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(st));
+  P->t.wsw = P->wsw.as<float4>();
+  return MIRT_OK;
+}
+
+// Split spread: the plane's tiles that a band's segment could not share out
+// evenly go to the point spread, which splits them over groups and CTAs; the
+// bands of four rows between them are cut into segments of about a quarter of a
+// warp's share of the whole cost (at least eight columns).
+int build_split(mirt_interp_plan *P, cudaStream_t st) {
+  const InterpArgs &a = P->a;
+  Tiling &t = P->t;
+  constexpr int kRows = 4, kWarps = 148 * 16;
+  const int shape = points_shape(a.C), K1 = a.g.K[0], K2 = a.g.K[1];
+  int ext[3], nt[3];
+  points_tile_extent(a, shape, ext, nt);
+  if (ext[1] % kRows) return MIRT_OK;
+  std::vector<int> most;
+  int rc = point_counts(P, shape, st, most);
+  if (rc || most.empty()) return rc;
+  std::vector<float> vb;
+  rc = sweep_band_visits(P, kRows, st, vb, false);
+  if (rc) return rc;
+  const int nband = (K2 + kRows - 1) / kRows;
+  const double nch = (a.C + 31) / 32;
+  double total = 0;
+  for (float v : vb) total += v + kSweepColumnCost;
+  const double share = std::max(1.0, total * nch / kWarps);
+  const int dense = (int)std::min(kSplitMost, std::max(64.0, kSplitDense * share));
+  const double target = std::max(32.0, share / kSplitTeams);
+  std::vector<int4> tk;
+  std::vector<double> cost;
+  for (int s = 0; s < t.nslice; s++)
+    for (int bi = 0; bi < nband; bi++) {
+      const float *v = vb.data() + ((size_t)s * nband + bi) * K1;
+      const int *tile = most.data() + ((size_t)s * nt[1] + bi * kRows / ext[1]) * nt[0];
+      int x0 = 0;
+      while (x0 < K1) {
+        if (tile[x0 / ext[0]] > dense) {
+          x0 = (x0 / ext[0] + 1) * ext[0];
+          continue;
+        }
+        int xr = x0;  // the run of columns up to the next dense tile
+        while (xr < K1 && tile[xr / ext[0]] <= dense) xr = std::min(K1, (xr / ext[0] + 1) * ext[0]);
+        while (x0 < xr) {
+          double c = 5 * kSweepColumnCost;
+          for (int x = x0 - 5; x < x0; x++) c += v[(x + K1) % K1];
+          int x1 = x0;
+          while (x1 < xr) {
+            const double add = v[x1] + kSweepColumnCost;
+            if (x1 - x0 >= 8 && c + add > target) break;
+            c += add;
+            x1++;
+          }
+          if (xr - x1 < 8)
+            for (; x1 < xr; x1++) c += v[x1] + kSweepColumnCost;
+          tk.push_back(make_int4(s, bi * kRows, x0, x1));
+          cost.push_back(c);
+          x0 = x1;
+        }
+      }
+    }
+  std::vector<int> order(tk.size());
+  for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+  std::vector<int4> sorted(tk.size());
+  for (size_t i = 0; i < order.size(); i++) sorted[i] = tk[order[i]];
+  CK(P->split_teams.alloc(std::max<size_t>(sorted.size(), 1) * sizeof(int4)));
+  CK(P->split_next.alloc((size_t)nch * sizeof(int)));
+  if (!sorted.empty())
+    CK(cudaMemcpyAsync(P->split_teams.p, sorted.data(), sorted.size() * sizeof(int4),
+                       cudaMemcpyHostToDevice, st));
+  CK(cudaStreamSynchronize(st));
+  t.split_team = P->split_teams.as<int4>();
+  t.split_nteams = (int)sorted.size();
+  t.split_next = P->split_next.as<int>();
+  rc = build_point_tasks(P, shape, most, dense, st);
+  if (rc) return rc;
+  P->split_ok = 1;
   return MIRT_OK;
 }
 
@@ -651,6 +793,10 @@ void choose_config(mirt_interp_plan *P) {
   t.own = 0;
   t.sweep = 0;
   t.sweep_rows = 1;
+  t.split = 0;
+  t.split_team = nullptr;
+  t.split_nteams = 0;
+  t.split_next = nullptr;
   t.points = 0;
   t.pt_task = nullptr;
   t.n_pt_task = 0;
@@ -1099,16 +1245,18 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
   if (sweep_ok(a, P->t) && P->ls.cw == 32) {
     int rc3 = sweep_buffer(P);
     if (rc3) return rc3;
-    rc3 = build_sweep_teams(P, 1, 65536, st);
+    // (its team list is made when it is first needed: sweep_teams_ready)
+    P->t.sweep = -1;
+    P->t.sweep_rows = 1;
+    const size_t nq = (size_t)(a.C + 31) / 32;  // the queue counters of slice ranges
+    CK(P->team_next.alloc(nq * sizeof(int)));
+    P->t.team_next = P->team_next.as<int>();
+  }
+  if (sweep_ok(a, P->t) && a.C >= kSplitColumns) {
+    int rc3 = build_sweep_records(P, st);
+    if (!rc3) rc3 = build_split(P, st);
     if (rc3) return rc3;
-    // the staged sweep's records (FFMA2 operand pairs of the taps)
-    CK(P->wsw.alloc(std::max<long long>(Mtot, 1) * 9 * sizeof(float4)));
-    if (Mtot > 0)
-      mirt_plan_kernels::sweep_records_kernel<<<(unsigned)((Mtot + 255) / 256), 256, 0, st>>>(
-          a.W, Mtot, P->wsw.as<float4>());
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(st));
-    P->t.wsw = P->wsw.as<float4>();
+    P->t.split = P->split_ok;
   }
   // 3D, J = 6, coil chunks of 8, 16 or 32: the line sweep, two segments per line
   if (sweep3_ok(a, P->t, P->ls.cw)) {
@@ -1118,12 +1266,11 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     if (rc3) return rc3;
   }
   // everything else: the point spread
-  if (!P->t.sweep && a.C > 0) {
+  if (!P->t.sweep && !P->t.split && a.C > 0) {
     int rc3 = build_points(P, st);
     if (rc3) return rc3;
-    P->t.points = P->points_shape;
   }
-  return MIRT_OK;
+  return P->t.sweep < 0 && !P->t.split ? sweep_teams_ready(P, st) : MIRT_OK;
 }
 
 // Re-tile the spread (tiles of T[d] points, multiples of the sort bins) and
@@ -1149,7 +1296,8 @@ struct SpreadCand {
   int threads, padc, atomic, own, sweep, sweep_rows;
   int dense = 0;  // 2D row sweep with dense-bin patches (one-row bands)
   int staged = 0;  // 2D row sweep staged per column (1), reading the caller's samples (2)
-  int points = 0;  // point spread (its column lanes)
+  int points = 0;  // point spread (its lane shape)
+  int split = 0;   // split spread
 };
 
 // spare columns the J = 6 row update can use (0 elsewhere)
@@ -1219,6 +1367,13 @@ int validate_geometry(int D, const int *K, const int *J, const int *L, int order
 
 // The plan whose launches a setter tunes: a 4D plan's 3D plan, else the plan.
 static mirt_interp_plan *launch_plan(mirt_interp_plan *P) { return P->sub4 ? P->sub4 : P; }
+
+// A row-sweep setting was chosen: the row sweep itself, not the split spread.
+static int leave_split(mirt_interp_plan *P) {
+  if (!P->t.sweep || !P->t.split) return MIRT_OK;
+  P->t.points = P->t.split = 0;
+  return sweep_teams_ready(P, as_stream(nullptr));
+}
 
 extern "C" {
 
@@ -1410,6 +1565,12 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     c.points = P->points_shape;
     cands.push_back(c);
   }
+  if (P->split_ok) {
+    SpreadCand c{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, cw == 32 ? -1 : 0, 1};
+    c.points = points_shape(a.C);
+    c.split = 1;
+    cands.push_back(c);
+  }
   SpreadCand best{};
   float best_ms = 1e30f;
   int built_rows = 0;  // rows of the team list last built
@@ -1420,6 +1581,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     P->t.dense_on = c.dense;
     P->t.sweep_staged = c.staged;
     P->t.points = c.points;
+    P->t.split = c.split;
     if (c.sweep < 0 && built_rows != c.sweep_rows) {
       int rc = build_sweep_teams(P, c.sweep_rows, 65536, st);
       if (rc) return rc;
@@ -1444,9 +1606,9 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     if (autotune_log())
       std::fprintf(stderr,
                    "mirt autotune spread: tile %dx%dx%d threads %d padc %d atomic %d own %d "
-                   "sweep %d rows %d dense %d staged %d points %d: %.3f ms\n",
+                   "sweep %d rows %d dense %d staged %d points %d split %d: %.3f ms\n",
                    c.T[0], c.T[1], c.T[2], c.threads, c.padc, c.atomic, c.own, c.sweep,
-                   c.sweep_rows, c.dense, c.staged, c.points, ms);
+                   c.sweep_rows, c.dense, c.staged, c.points, c.split, ms);
     if (ms < best_ms) {
       best_ms = ms;
       best = c;
@@ -1459,6 +1621,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     P->t.dense_on = best.dense;
     P->t.sweep_staged = best.staged;
     P->t.points = best.points;
+    P->t.split = best.split;
     if (best.sweep < 0 && built_rows != best.sweep_rows) {
       int rc = build_sweep_teams(P, best.sweep_rows, 65536, st);
       if (rc) return rc;
@@ -1559,12 +1722,12 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
 int mirt_interp_plan_config(mirt_interp_plan *P, int32_t *out, int32_t n) {
   if (!P || !out) return fail(MIRT_ERR_ARG, "NULL argument");
   P = launch_plan(P);
-  const int32_t v[24] = {P->t.T[0], P->t.T[1], P->t.T[2], P->ls.threads, P->heavy_first, P->ls.cw,
+  const int32_t v[25] = {P->t.T[0], P->t.T[1], P->t.T[2], P->ls.threads, P->heavy_first, P->ls.cw,
                          P->lg.threads, P->lg.sb, P->lg.grid, P->t.B[0], P->t.B[1], P->t.B[2],
                          P->split_chunk, P->t.ntask, P->t.padc, P->t.nred, P->ls.atomic,
                          P->t.own, P->t.sweep, P->t.sweep_rows, P->gtma, P->t.dense_on,
-                         P->t.sweep_staged, P->t.points};
-  for (int i = 0; i < n && i < 24; i++) out[i] = v[i];
+                         P->t.sweep_staged, P->t.points, P->t.split};
+  for (int i = 0; i < n && i < 25; i++) out[i] = v[i];
   return MIRT_OK;
 }
 
@@ -1612,7 +1775,7 @@ int mirt_interp_plan_set_sweep(mirt_interp_plan *P, int32_t segments, int32_t ro
                                 "chunks of 8, 16 or 32");
     if (segments < 0 || segments > P->a.g.K[0])
       return fail(MIRT_ERR_ARG, "3D line-sweep segments must be in 1..K1 (0: off)");
-    P->t.points = 0;
+    P->t.points = P->t.split = 0;
     if (segments) {
       int rc = sweep_buffer(P);
       if (rc) return rc;
@@ -1627,7 +1790,7 @@ int mirt_interp_plan_set_sweep(mirt_interp_plan *P, int32_t segments, int32_t ro
     return fail(MIRT_ERR_ARG, "row-sweep segments must be in 1..K1 (0: off, -1: balanced)");
   if (segments && rows != 1 && rows != 2 && rows != 4)
     return fail(MIRT_ERR_ARG, "row-sweep rows per band must be 1, 2 or 4");
-  P->t.points = 0;
+  P->t.points = P->t.split = 0;
   if (segments) {
     int rc = sweep_buffer(P);
     if (rc) return rc;
@@ -1650,22 +1813,26 @@ int mirt_interp_plan_set_sweep(mirt_interp_plan *P, int32_t segments, int32_t ro
   return fail(MIRT_ERR_ALLOC, "out of host memory");
 }
 
-int mirt_interp_plan_set_dense(mirt_interp_plan *P, int32_t on) {
+int mirt_interp_plan_set_dense(mirt_interp_plan *P, int32_t on) try {
   if (!P) return fail(MIRT_ERR_ARG, "plan is NULL");
   P = launch_plan(P);
   if (on && !P->t.dense_of) return fail(MIRT_ERR_ARG, "the plan has no dense bins");
   P->t.dense_on = on ? 1 : 0;
-  return MIRT_OK;
+  return leave_split(P);
+} catch (const std::bad_alloc &) {
+  return fail(MIRT_ERR_ALLOC, "out of host memory");
 }
 
-int mirt_interp_plan_set_staged(mirt_interp_plan *P, int32_t mode) {
+int mirt_interp_plan_set_staged(mirt_interp_plan *P, int32_t mode) try {
   if (!P) return fail(MIRT_ERR_ARG, "plan is NULL");
   P = launch_plan(P);
   if (mode < 0 || mode > 2) return fail(MIRT_ERR_ARG, "staged mode must be 0, 1 or 2");
   if (mode && (P->ls.cw != 32 || !P->t.wsw))
     return fail(MIRT_ERR_ARG, "the staged row sweep needs 32-coil lanes (C >= 32)");
   P->t.sweep_staged = mode;
-  return MIRT_OK;
+  return leave_split(P);
+} catch (const std::bad_alloc &) {
+  return fail(MIRT_ERR_ALLOC, "out of host memory");
 }
 
 int mirt_interp_plan_set_ownership(mirt_interp_plan *P, int32_t own, void *stream) try {
@@ -1675,7 +1842,7 @@ int mirt_interp_plan_set_ownership(mirt_interp_plan *P, int32_t own, void *strea
     return fail(MIRT_ERR_ARG, "ownership spread needs 2D, J = 6, tiles of >= 5 points and an "
                               "even number of tiles (last one >= 5 points) per dimension");
   P->t.own = own ? 1 : 0;
-  P->t.points = 0;
+  P->t.points = P->t.split = 0;
   if (own) {
     P->ls.atomic = 0;
     P->t.sweep = 0;
@@ -1728,7 +1895,7 @@ int mirt_interp_plan_set_spread(mirt_interp_plan *P, const int32_t *T, int32_t t
   P->t.padc = padc;
   P->ls.threads = threads;
   P->t.sweep = 0;
-  P->t.points = 0;
+  P->t.points = P->t.split = 0;
   int rc = set_spread_tiles(P, Tn, st);
   if (rc) return rc;
   CK(cudaStreamSynchronize(st));
@@ -2947,6 +3114,7 @@ int nufft_adjoint_range(mirt_nufft *p, int s0, int s1, const float2 *X, float2 *
   const long long gi = p->gg.ngrid * C, xi = p->gg.npix * C;
   mirt_interp_plan *P = p->ip;
   Tiling t = P->t;
+  t.points = t.split = 0;
   if (t.sweep < 0) t.sweep = 2;  // a chunk: uniform halves of rows (same sums)
   t.team_order = nullptr;        // the chunk's teams in index order
   if (t.ndense > 0) {            // the chunk's dense bins and their sample chunks
@@ -3156,7 +3324,9 @@ int mirt_nufft_config(mirt_nufft *p, int32_t *out, int32_t n) {
   // gather: one launch (TMA-staged or plain)
   const int fwd = (p->own_fft ? p->gg.D : 2) + 1;
   int spread = 1;  // the point spread: one launch
-  if (t.points && !p->ip->ls.atomic) {
+  if (t.split) {
+    spread = (t.split_nteams > 0) + (t.n_pt_task > 0);
+  } else if (t.points && !p->ip->ls.atomic) {
   } else if (t.sweep != 0) {
     // ordering pass, dense-bin patches (chunk sums, per-bin sums), sweep (and a
     // memset of the queue counters)

@@ -227,8 +227,26 @@ cudaError_t launch_mark_dense(const int *dense_bin, int n, int *dense_of, cudaSt
 cudaError_t launch_spread(const InterpArgs &a, const Tiling &t, const Launch &l,
                           const int *bin_start, const float2 *fm, float2 *ck, cudaStream_t st) {
   if (a.C == 0) return cudaSuccess;
-  if (t.points && !l.atomic) return launch_spread_points(a, t, bin_start, fm, ck, st);
   Launch lc = l;
+  if (t.split && (t.sweep || !l.atomic)) {
+    if (t.split_nteams) {
+      Tiling ts = t;
+      ts.sweep = -1;
+      ts.sweep_rows = 4;
+      ts.sweep_staged = 2;
+      ts.dense_on = 0;
+      ts.sweep_team = t.split_team;
+      ts.nteams = t.split_nteams;
+      ts.team_order = nullptr;
+      ts.team_next = t.split_next;
+      lc.cw = 32;
+      detail::Req r{detail::SPREAD, &a, &ts, &lc, bin_start, fm, ck, st};
+      cudaError_t e = dispatch(r);
+      if (e != cudaSuccess) return e;
+    }
+    return launch_spread_points(a, t, bin_start, fm, ck, st);
+  }
+  if (t.points && !l.atomic) return launch_spread_points(a, t, bin_start, fm, ck, st);
   detail::Req r{detail::SPREAD, &a, &t, &lc, bin_start, fm, ck, st};
   return dispatch(r);
 }

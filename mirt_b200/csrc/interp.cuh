@@ -117,6 +117,13 @@ struct Tiling {
   float2 *pt_scratch;
   int *pt_count;
   const int4 *pt_hdr;    // per position: first tap k1, caller's sample index, phase (float bits)
+  // Split spread (2D, J = 6, many columns): the staged row sweep over the team
+  // list `split_team` (bands of four rows, segments of their columns, heaviest
+  // first), which leaves out the dense tiles; the point spread's tasks are those
+  int split;             // 0: off
+  const int4 *split_team;
+  int split_nteams;
+  int *split_next;       // its queue counters, one per chunk of 32 columns
   int color_beg[9];
   int red_beg[9];
   int padc;              // spread: spare columns on each side of a tile row in
@@ -216,19 +223,22 @@ cudaError_t query_gather_grid(const InterpArgs &a, Launch &l);
 cudaError_t launch_gather(const InterpArgs &a, const Launch &l, const float2 *ck,
                           float2 *fm, cudaStream_t st);
 
-// Point spread (spread_points.cu): the lane shape for C columns, the base tiles
-// of nslice slices (0: the geometry does not fit it), and the log2 split of each
-// of them (from the sort's bins) with the positions' headers.  A tile of split
-// 2^l is 2^l consecutive tasks; points_cta_log2: the l up to which a brick's
-// groups are one CTA's, beyond it 2^(l - points_cta_log2) CTAs share a brick
+// Point spread (spread_points.cu): the lane shape for C columns; the base tiles
+// of nslice slices (0: the geometry does not fit it), their extent in points and
+// their number per dimension; the most samples that reach a brick of each tile,
+// with the positions' headers; and the log2 split of a tile of `most` among the
+// ntile tiles that are launched.  A tile of split 2^l is 2^l consecutive tasks;
+// points_cta_log2: the l up to which a brick's groups are one CTA's, beyond it
+// 2^(l - points_cta_log2) CTAs share a brick.
+int points_shape(int C);
+long long points_tiles(const InterpArgs &a, int shape, int nslice);
+void points_tile_extent(const InterpArgs &a, int shape, int *ext, int *n);
 int points_cta_log2(int shape);
 size_t points_slot_bytes(int shape);
 int points_chunks(int shape, int C);
-int points_shape(int C);
-long long points_tiles(const InterpArgs &a, int shape, int nslice);
-cudaError_t launch_points_split(const InterpArgs &a, const Tiling &t, int shape, int nslice,
-                                const int *bin_start, unsigned char *lg, int4 *hdr,
-                                cudaStream_t st);
+cudaError_t launch_points_count(const InterpArgs &a, const Tiling &t, int shape, int nslice,
+                                const int *bin_start, int *most, int4 *hdr, cudaStream_t st);
+int points_split(const InterpArgs &a, int shape, int most, long long ntile);
 cudaError_t launch_spread_points(const InterpArgs &a, const Tiling &t, const int *bin_start,
                                  const float2 *fm, float2 *ck, cudaStream_t st);
 

@@ -75,6 +75,8 @@ struct mirt_interp_plan {
   std::vector<int4> team_host;  // the same list on the host
   mirt::DMem team_order, team_next;  // row-sweep work queue: heaviest-first order, counter
   mirt::DMem pt_task, pt_hdr, pt_scratch, pt_count;  // point spread (Tiling)
+  mirt::DMem split_teams, split_next;                // split spread (Tiling)
+  int split_ok = 0;                  // 1: the plan has the split spread's lists
   int points_shape = 0;              // its lane shape (0: the plan has none)
   mirt::DMem dense_of, dense_bin, patch;  // the sweeps' dense bins and their patches
   mirt::DMem dense_chunk, dense_part0, patch_part;  // chunks of the patch sums

@@ -110,7 +110,7 @@ inline PtSmem pt_smem(const Geom &g, const PtTile &t, int cw, int nc) {
   s.off_rec = (s.ne * 2 * 4 + 4 + 15) & ~15;
   s.off_f = s.off_rec + S * s.rs * 8;
   s.off_d = (s.off_f + S * cw * nc * 8 + 15) & ~15;
-  s.bytes = s.off_d + S * 16;
+  s.bytes = s.off_d + S * 24;
   return s;
 }
 
@@ -123,11 +123,10 @@ __global__ void point_header_kernel(InterpArgs a, int4 *__restrict__ hdr) {
                      __float_as_int(ph.y));
 }
 
-// split 2^lg of each base tile: the most samples that reach one of its bricks,
-// over vmax samples a group
-__global__ void point_split_kernel(InterpArgs a, Tiling t, PtTile pt, int ngrp, int lgmin, int vmax,
+// the most samples that reach one brick, of every base tile
+__global__ void point_count_kernel(InterpArgs a, Tiling t, PtTile pt, int ngrp,
                                    const int *__restrict__ bin_start, long long ntile,
-                                   unsigned char *__restrict__ lg) {
+                                   int *__restrict__ most) {
   const long long tile = blockIdx.x;
   if (tile >= ntile) return;
   const Geom &g = a.g;
@@ -159,10 +158,9 @@ __global__ void point_split_kernel(InterpArgs a, Tiling t, PtTile pt, int ngrp, 
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int m = 0, l = lgmin;
+    int m = 0;
     for (int b = 0; b < ngrp; b++) m = max(m, cnt[b]);
-    while ((1 << l) < ngrp << PT_SHARE && (m >> l) > vmax) l++;
-    lg[tile] = (unsigned char)l;
+    most[tile] = m;
   }
 }
 
@@ -187,6 +185,7 @@ __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
   float2 *rec = reinterpret_cast<float2 *>(gsm + sm.off_rec);
   float2 *sf = reinterpret_cast<float2 *>(gsm + sm.off_f);
   int4 *sd = reinterpret_cast<int4 *>(gsm + sm.off_d);
+  float2 *sph = reinterpret_cast<float2 *>(sd + S);  // phases (column chunks of 8 and more)
   // the task: part of base tile tk.x, split G = 2^lg: 1/G of its bricks with G
   // groups each, or (G > NGRP) one brick shared by G / NGRP CTAs
   const int4 tk = t.pt_task[blockIdx.x];
@@ -304,19 +303,28 @@ __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
             }
         }
         // first tap relative to the brick (after 4 pad entries), tap row and plane
-        if (sub == 0)
-          sd[ci] = make_int4(4 + X0 - h.x + (ps ? K1 : 0), e % nq2 | e / nq2 << 16, h.y, p);
+        if (sub == 0) {
+          sd[ci] = make_int4(4 + X0 - h.x + (ps ? K1 : 0), e % nq2 | e / nq2 << 16, h.y, 0);
+          if (CW * NC >= 8) sph[ci] = make_float2(__int_as_float(h.z), __int_as_float(h.w));
+        }
       }
       __syncwarp();
       if constexpr (CW * NC >= 8) {
-        // the chunk's columns, the group's lanes along them
-        for (int i = gl; i < n * (CW * NC); i += GL) {
-          const int j = i / (CW * NC), c = i % (CW * NC);
-          const int4 hj = sd[j];
-          float2 v2 =
-              c0 + c < C ? __ldg(fm + (long long)hj.z * C + c0 + c) : make_float2(0.f, 0.f);
-          if (a.phase) v2 = cmulc(__ldg(a.phase + hj.w), v2);
-          sf[i] = v2;
+        // the chunk's columns, the group's lanes along them, four loads in flight
+        constexpr int CN = CW * NC, U = 4;
+        for (int i0 = gl; i0 < n * CN; i0 += U * GL) {
+          float2 v2[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const int i = i0 + u * GL, j = i / CN, c = i % CN;
+            v2[u] = make_float2(0.f, 0.f);
+            if (i < n * CN && c0 + c < C) v2[u] = __ldg(fm + (long long)sd[j].z * C + c0 + c);
+          }
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const int i = i0 + u * GL;
+            if (i < n * CN) sf[i] = a.phase ? cmulc(sph[i / CN], v2[u]) : v2[u];
+          }
         }
         __syncwarp();
       }
@@ -486,21 +494,34 @@ int points_chunks(int shape, int C) {
   return (C + n - 1) / n;
 }
 
-cudaError_t launch_points_split(const InterpArgs &a, const Tiling &t, int shape, int nslice,
-                                const int *bin_start, unsigned char *lg, int4 *hdr,
-                                cudaStream_t st) {
-  const int cw = shape / 8, ngrp = PT_THREADS / (cw * pt_lb(cw));
-  const PtTile pt = pt_tile(a.g, cw);
+void points_tile_extent(const InterpArgs &a, int shape, int *ext, int *n) {
+  const PtTile t = pt_tile(a.g, shape / 8);
+  ext[0] = t.W * t.bx;
+  ext[1] = t.R2 * t.by;
+  ext[2] = t.R3 * t.bz;
+  n[0] = t.nt1;
+  n[1] = t.nt2;
+  n[2] = t.nt3;
+}
+
+cudaError_t launch_points_count(const InterpArgs &a, const Tiling &t, int shape, int nslice,
+                                const int *bin_start, int *most, int4 *hdr, cudaStream_t st) {
+  const PtTile pt = pt_tile(a.g, shape / 8);
+  const int ngrp = PT_THREADS / (shape / 8 * pt_lb(shape / 8));
   const long long n = points_tiles(a, shape, nslice);
-  const long long chunks = points_chunks(shape, a.C);
-  int lgmin = 0;
-  // few tiles: split them all until there are two CTAs per SM
-  while ((1 << lgmin) < ngrp && (n * chunks << lgmin) < 296) lgmin++;
-  point_split_kernel<<<(unsigned)n, 128, 0, st>>>(a, t, pt, ngrp, lgmin, pt_visits(a.g.D),
-                                                  bin_start, n, lg);
+  point_count_kernel<<<(unsigned)n, 128, 0, st>>>(a, t, pt, ngrp, bin_start, n, most);
   if (a.Mtot > 0)
     point_header_kernel<<<(unsigned)((a.Mtot + 255) / 256), 256, 0, st>>>(a, hdr);
   return cudaGetLastError();
+}
+
+int points_split(const InterpArgs &a, int shape, int most, long long ntile) {
+  const int lc = points_cta_log2(shape);
+  int l = 0;
+  // few tiles: split them all until there are two CTAs per SM
+  while (l < lc && (ntile * points_chunks(shape, a.C) << l) < 296) l++;
+  while (l < lc + PT_SHARE && (most >> l) > pt_visits(a.g.D)) l++;
+  return l;
 }
 
 cudaError_t launch_spread_points(const InterpArgs &a, const Tiling &t, const int *bin_start,

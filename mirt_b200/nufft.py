@@ -66,15 +66,15 @@ def minmax_kb_scale(N: int, J: int, K: int) -> np.ndarray:
 
 
 def _plan_config(lib, handle) -> dict:
-    v = (C.c_int32 * 24)()
-    check(lib.mirt_interp_plan_config(handle, v, 24))
+    v = (C.c_int32 * 25)()
+    check(lib.mirt_interp_plan_config(handle, v, 25))
     return {"spread_tile": [v[0], v[1], v[2]], "spread_threads": v[3], "spread_heavy_first": v[4],
             "coil_lanes": v[5], "gather_threads": v[6],
             "gather_ctas": v[8], "sort_bin": [v[9], v[10], v[11]], "split_chunk": v[12],
             "spread_tasks": v[13], "spread_padc": v[14], "spread_reductions": v[15],
             "spread_atomic": v[16], "spread_own": v[17], "spread_sweep": v[18],
             "spread_sweep_rows": v[19], "gather_tma": v[20], "spread_dense": v[21],
-            "spread_staged": v[22], "spread_points": v[23]}
+            "spread_staged": v[22], "spread_points": v[23], "spread_split": v[24]}
 
 
 class InterpPlan:

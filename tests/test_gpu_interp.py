@@ -915,3 +915,42 @@ def test_point_spread_matches_oracle(K, J, C, variant):
     assert plan.config()["spread_points"] == 0
     assert rel_l2(plan.adjoint(fm_d).cpu().numpy(), out) <= 5e-6
     plan.close()
+
+
+@pytest.mark.parametrize("K,C,order", [((64, 48), 25, 0), ((41, 50), 32, 1), ((96, 80), 33, 0),
+                                       ((6, 7), 64, 0)])
+def test_split_spread_matches_oracle(K, C, order):
+    """The split spread (the default from 25 columns in 2D, J = 6): a slice of
+    even density, an empty one and one with a dense centre, so that some tiles go
+    to the point spread and the bands between them to the row sweep; odd grids
+    (bands and tiles cut at the end), idle columns and several chunks; the
+    oracle's adjoint, bitwise reproducible, and the row sweep's result."""
+    import torch
+    rng = np.random.default_rng(C + K[0])
+    J, L = [6, 6], [256, 256]
+    h = ([mb.newfft_kb_table(6, 256)] * 2 if order else
+         [mb.minmax_kb_table(max(2, k // 2), 6, k, 256) for k in K])
+    tms = [rng.uniform(-60, 60, (900, 2)), np.zeros((0, 2)),
+           np.concatenate([rng.uniform(-2, 2, (6000, 2)), rng.uniform(-30, 30, (600, 2))])]
+    moff = np.concatenate([[0], np.cumsum([len(t) for t in tms])])
+    tm = np.concatenate(tms)
+    ph = np.exp(1j * rng.uniform(0, 6, len(tm)))
+    plan = mb.InterpPlan(K, J, L, h, tm, C, order=order, slice_moff=moff, phase=ph)
+    assert plan.config()["spread_split"] == 1
+    fm = rng.standard_normal((len(tm), C)) + 1j * rng.standard_normal((len(tm), C))
+    fm_d = torch.from_numpy(fm.astype(np.complex64)).cuda()
+    out = plan.adjoint(fm_d).cpu().numpy()
+    assert np.array_equal(out, plan.adjoint(fm_d).cpu().numpy())
+    for s in range(3):
+        sl = slice(moff[s], moff[s + 1])
+        got = np.transpose(out[s], (1, 0, 2)).reshape(-1, C, order="F")
+        if not len(tms[s]):
+            assert not got.any()
+            continue
+        ref = oracle.interp_adj(fm[sl] * np.conj(ph[sl])[:, None], h, J, L, tms[s], K, order,
+                                impl=ref_impl())
+        assert rel_l2(got, ref) <= ADJ_TOL, s
+    plan.set_sweep(1, 1)
+    assert plan.config()["spread_split"] == 0
+    assert rel_l2(plan.adjoint(fm_d).cpu().numpy(), out) <= 5e-6
+    plan.close()
