@@ -392,9 +392,11 @@ mirt_interp_plan *mirt_nufft_interp_plan(mirt_nufft *p);
 int mirt_nufft_autotune(mirt_nufft *p, void *stream);
 
 /* How the NUFFT runs: up to 3 values {1 if the oversampled FFT runs as the
- * library's fused passes over the interpolation grid (power-of-two K from
- * 64 to 1024 in every dimension), 0 if through cuFFT with coil-layout
- * transposes; library kernel launches of one forward; of one adjoint} (cuFFT's
+ * library's fused passes over the interpolation grid (K in every dimension a
+ * power of two from 64 to 1024, or 80, 96, 100, 112, 120, 144, 160, 192, 200,
+ * 224, 240, 280, 288, 320, 336, 360, 384, 400, 448, 480, 560, 576, 640, 672, 768
+ * or 896), 0 if through cuFFT (with coil-layout transposes where there are
+ * several columns); library kernel launches of one forward; of one adjoint} (cuFFT's
  * own launches not counted).  No reference counterpart. */
 int mirt_nufft_config(mirt_nufft *p, int32_t *out, int32_t n);
 

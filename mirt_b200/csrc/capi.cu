@@ -2439,13 +2439,38 @@ namespace {
       return fail(MIRT_ERR_FFT, std::string(#call) + " failed: " + std::to_string((int)r_)); \
   } while (0)
 
-// one batched C2C execution over every slice and coil of the coil-major grid:
-// forward out of place from the zero-padded input, inverse in place
-int nufft_fft(mirt_nufft *p, int dir, cudaStream_t st) {
-  CF(cufftSetStream(p->fft, st));
-  cufftComplex *g = reinterpret_cast<cufftComplex *>(p->grid_cm.as<float2>());
-  cufftComplex *src = dir == CUFFT_FORWARD ? reinterpret_cast<cufftComplex *>(p->pad.as<float2>()) : g;
-  CF(cufftExecC2C(p->fft, src, g, dir));
+// The cuFFT path over slices [s0, s1) with `fft` made for that many: the
+// zero-padded coil-major input, one batched C2C execution over its slices and
+// coils (forward out of place, inverse in place), and the transposes to and from
+// the interpolation's coil-innermost grid, which one column does without.
+int cufft_forward(mirt_nufft *p, int s0, int s1, const float2 *x, cufftHandle fft,
+                  cudaStream_t st) {
+  const int ns = s1 - s0;
+  const long long gi = p->gg.ngrid * p->C;
+  float2 *pad = p->pad.as<float2>() + s0 * gi, *grid = p->grid.as<float2>() + s0 * gi;
+  float2 *gcm = p->one_col ? grid : p->grid_cm.as<float2>() + s0 * gi;
+  CK(launch_deapod_image_cm(x + s0 * p->gg.npix * p->C, p->sn.as<float2>(), pad, p->gg, p->C, ns,
+                            st));
+  CF(cufftSetStream(fft, st));
+  CF(cufftExecC2C(fft, reinterpret_cast<cufftComplex *>(pad), reinterpret_cast<cufftComplex *>(gcm),
+                  CUFFT_FORWARD));
+  if (!p->one_col)
+    CK(launch_transpose_cols(gcm, grid, p->gg.ngrid, p->C, ns, 1, st, &p->gp));
+  return MIRT_OK;
+}
+
+int cufft_adjoint(mirt_nufft *p, int s0, int s1, float2 *x, cufftHandle fft, cudaStream_t st) {
+  const int ns = s1 - s0;
+  const long long gi = p->gg.ngrid * p->C;
+  float2 *grid = p->grid.as<float2>() + s0 * gi;
+  float2 *gcm = p->one_col ? grid : p->grid_cm.as<float2>() + s0 * gi;
+  if (!p->one_col)
+    CK(launch_transpose_cols(grid, gcm, p->gg.ngrid, p->C, ns, 0, st, &p->gp));
+  CF(cufftSetStream(fft, st));
+  CF(cufftExecC2C(fft, reinterpret_cast<cufftComplex *>(gcm), reinterpret_cast<cufftComplex *>(gcm),
+                  CUFFT_INVERSE));
+  CK(launch_crop_deapod_cm(gcm, p->sn.as<float2>(), x + s0 * p->gg.npix * p->C, p->gg, p->C, ns,
+                           st));
   return MIRT_OK;
 }
 
@@ -2608,7 +2633,7 @@ int nufft_finish(mirt_nufft *p, int D, const int32_t *Nd, const int32_t *Kd, con
     bool fold = any_mid;
     for (int d = 0; d < D && fold; d++) {
       const long long m4 = 4ll * (nmid ? nmid[d] : 0);
-      if (m4 % Kd[d] != 0) fold = false;
+      if (m4 % Kd[d] != 0 || !fft_fold_ok(Kd[d])) fold = false;
       else qm[d] = (int)(((m4 / Kd[d]) % 4 + 4) % 4);
     }
     std::vector<float2> tw;
@@ -2651,9 +2676,18 @@ int nufft_finish(mirt_nufft *p, int D, const int32_t *Nd, const int32_t *Kd, con
     p->nf.gp = &p->gp;
     return MIRT_OK;
   }
+  // a grid phase of whole periods is a shift of the padded image
+  bool whole = any_mid;
+  for (int d = 0; d < D && whole; d++)
+    whole = nmid[d] == std::floor(nmid[d]) && nmid[d] >= 0 && nmid[d] < Kd[d];
+  if (whole) {
+    for (int d = 0; d < D; d++) p->gg.shift[d] = (int)nmid[d];
+    for (int d = 0; d < 3; d++) p->gp.tab[d] = nullptr;
+  }
+  p->one_col = ncol == 1 && !p->gp.tab[0];
   {
     cudaError_t e = p->grid.alloc((size_t)nslice * p->gg.ngrid * ncol * sizeof(float2));
-    if (e == cudaSuccess) e = p->grid_cm.alloc((size_t)nslice * p->gg.ngrid * ncol * sizeof(float2));
+    if (e == cudaSuccess && !p->one_col) e = p->grid_cm.alloc((size_t)nslice * p->gg.ngrid * ncol * sizeof(float2));
     if (e == cudaSuccess) e = p->pad.alloc((size_t)nslice * p->gg.ngrid * ncol * sizeof(float2));
     if (e == cudaSuccess)
       e = cudaMemsetAsync(p->pad.p, 0, (size_t)nslice * p->gg.ngrid * ncol * sizeof(float2), st);
@@ -3047,12 +3081,8 @@ int mirt_nufft_forward(mirt_nufft *p, const void *x, void *X, void *stream) {
     CK(plan_gather(p->ip, p->grid.as<float2>(), static_cast<float2 *>(X), st));
     return MIRT_OK;
   }
-  CK(launch_deapod_image_cm(static_cast<const float2 *>(x), p->sn.as<float2>(),
-                            p->pad.as<float2>(), p->gg, p->C, p->nslice, st));
-  int rc = nufft_fft(p, CUFFT_FORWARD, st);
+  int rc = cufft_forward(p, 0, p->nslice, static_cast<const float2 *>(x), p->fft, st);
   if (rc) return rc;
-  CK(launch_transpose_cols(p->grid_cm.as<float2>(), p->grid.as<float2>(), p->gg.ngrid, p->C,
-                           p->nslice, 1, st, &p->gp));
   CK(plan_gather(p->ip, p->grid.as<float2>(), static_cast<float2 *>(X), st));
   return MIRT_OK;
 }
@@ -3068,13 +3098,7 @@ int mirt_nufft_adjoint(mirt_nufft *p, const void *X, void *x, void *stream) {
     CK(fft_nufft_adjoint(p->nf, p->grid.as<float2>(), static_cast<float2 *>(x), 0, p->nslice, st));
     return MIRT_OK;
   }
-  CK(launch_transpose_cols(p->grid.as<float2>(), p->grid_cm.as<float2>(), p->gg.ngrid, p->C,
-                           p->nslice, 0, st, &p->gp));
-  int rc = nufft_fft(p, CUFFT_INVERSE, st);
-  if (rc) return rc;
-  CK(launch_crop_deapod_cm(p->grid_cm.as<float2>(), p->sn.as<float2>(), static_cast<float2 *>(x),
-                           p->gg, p->C, p->nslice, st));
-  return MIRT_OK;
+  return cufft_adjoint(p, 0, p->nslice, static_cast<float2 *>(x), p->fft, st);
 }
 
 }  // extern "C"
@@ -3086,21 +3110,13 @@ namespace {
 // slices.
 int nufft_forward_range(mirt_nufft *p, int s0, int s1, const float2 *x, float2 *X,
                         cufftHandle fft, cudaStream_t st) {
-  const int ns = s1 - s0, C = p->C;
-  const long long gi = p->gg.ngrid * C, xi = p->gg.npix * C;
   if (p->own_fft) {
     CK(fft_nufft_forward(p->nf, x, p->grid.as<float2>(), s0, s1, st));
     CK(plan_gather(p->ip, p->grid.as<float2>(), X, st, s0, s1));
     return MIRT_OK;
   }
-  float2 *pad = p->pad.as<float2>() + s0 * gi;
-  float2 *gcm = p->grid_cm.as<float2>() + s0 * gi;
-  CK(launch_deapod_image_cm(x + s0 * xi, p->sn.as<float2>(), pad, p->gg, C, ns, st));
-  CF(cufftSetStream(fft, st));
-  CF(cufftExecC2C(fft, reinterpret_cast<cufftComplex *>(pad), reinterpret_cast<cufftComplex *>(gcm),
-                  CUFFT_FORWARD));
-  CK(launch_transpose_cols(gcm, p->grid.as<float2>() + s0 * gi, p->gg.ngrid, C, ns, 1, st,
-                           &p->gp));
+  int rc = cufft_forward(p, s0, s1, x, fft, st);
+  if (rc) return rc;
   // the gather over the chunk's slices (slice-major in the gather order)
   CK(plan_gather(p->ip, p->grid.as<float2>(), X, st, s0, s1));
   return MIRT_OK;
@@ -3110,8 +3126,6 @@ int nufft_forward_range(mirt_nufft *p, int s0, int s1, const float2 *x, float2 *
 // buffers.
 int nufft_adjoint_range(mirt_nufft *p, int s0, int s1, const float2 *X, float2 *x,
                         cufftHandle fft, cudaStream_t st) {
-  const int ns = s1 - s0, C = p->C;
-  const long long gi = p->gg.ngrid * C, xi = p->gg.npix * C;
   mirt_interp_plan *P = p->ip;
   Tiling t = P->t;
   t.points = t.split = 0;
@@ -3124,7 +3138,7 @@ int nufft_adjoint_range(mirt_nufft *p, int s0, int s1, const float2 *X, float2 *
     t.nchunks = P->dense_part0_host[t.dense0 + t.ndense] - t.chunk0;
   }
   t.slice0 = s0;
-  t.nslice = ns;
+  t.nslice = s1 - s0;
   t.pos0 = P->moff_host[s0];
   t.npos = P->moff_host[s1] - t.pos0;
   CK(launch_spread(P->a, t, P->ls, P->bin_start.as<int>(), X, p->grid.as<float2>(), st));
@@ -3132,14 +3146,7 @@ int nufft_adjoint_range(mirt_nufft *p, int s0, int s1, const float2 *X, float2 *
     CK(fft_nufft_adjoint(p->nf, p->grid.as<float2>(), x, s0, s1, st));
     return MIRT_OK;
   }
-  float2 *gcm = p->grid_cm.as<float2>() + s0 * gi;
-  CK(launch_transpose_cols(p->grid.as<float2>() + s0 * gi, gcm, p->gg.ngrid, C, ns, 0, st,
-                           &p->gp));
-  CF(cufftSetStream(fft, st));
-  CF(cufftExecC2C(fft, reinterpret_cast<cufftComplex *>(gcm), reinterpret_cast<cufftComplex *>(gcm),
-                  CUFFT_INVERSE));
-  CK(launch_crop_deapod_cm(gcm, p->sn.as<float2>(), x + s0 * xi, p->gg, C, ns, st));
-  return MIRT_OK;
+  return cufft_adjoint(p, s0, s1, x, fft, st);
 }
 
 // Chunks of a host-buffer call: up to 8, of ch slices (the last may be smaller).
@@ -3322,7 +3329,8 @@ int mirt_nufft_config(mirt_nufft *p, int32_t *out, int32_t n) {
   if (!p || !out) return fail(MIRT_ERR_ARG, "NULL argument");
   const Tiling &t = p->ip->t;
   // gather: one launch (TMA-staged or plain)
-  const int fwd = (p->own_fft ? p->gg.D : 2) + 1;
+  const int glue = p->own_fft ? p->gg.D : p->one_col ? 1 : 2;  // around the interpolation
+  const int fwd = glue + 1;
   int spread = 1;  // the point spread: one launch
   if (t.split) {
     spread = (t.split_nteams > 0) + (t.n_pt_task > 0);
@@ -3343,7 +3351,7 @@ int mirt_nufft_config(mirt_nufft *p, int32_t *out, int32_t n) {
   } else {
     spread = (t.ntask > 0) + (t.nred > 0);
   }
-  const int adj = spread + (p->own_fft ? p->gg.D : 2);
+  const int adj = spread + glue;
   const int32_t v[3] = {p->own_fft ? 1 : 0, fwd, adj};
   for (int i = 0; i < n && i < 3; i++) out[i] = v[i];
   return MIRT_OK;

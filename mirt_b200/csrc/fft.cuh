@@ -46,9 +46,16 @@ struct FftPass {
   const float2 *ph_out, *ph_in;
 };
 
-// Transform lengths the passes handle (powers of two from 64 to 1024), and
-// the two radices n = R1 R2 of a length.
+// Transform lengths the passes handle (the powers of two from 64 to 1024 and 26
+// products of two radices up to 32 between 80 and 896), the two radices n = R1 R2
+// of a length, and whether a quarter-turn grid phase folds into its twiddles
+// (both radices multiples of 4).
+// The fused passes against cuFFT with its transposes and glue, forward + adjoint,
+// us: 5 slices x 24 columns on 384^2 522 -> 173; 16 columns on 384^2 93 -> 31; one
+// column on 144 x 120 x 96 297 -> 29.  Bound by the latency of stage 1's loads, as
+// the powers of two.
 bool fft_len_ok(int n);
+bool fft_fold_ok(int n);
 void fft_radix(int n, int *r1, int *r2);
 
 cudaError_t launch_fft_pass(const FftPass &p, cudaStream_t st);

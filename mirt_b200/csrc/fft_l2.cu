@@ -1,0 +1,23 @@
+// fft_l2.cu -- DFT passes of lengths off the powers of two, part 2 (fft_impl.cuh).
+#include "fft_impl.cuh"
+
+namespace mirt {
+namespace fftk {
+
+cudaError_t launch_l2(const FftPass &p, cudaStream_t st) {
+  switch (p.n) {
+    case 240: return launch_r<12, 20, true>(p, st);
+    case 280: return launch_r<20, 14, true>(p, st);
+    case 288: return launch_r<12, 24, true>(p, st);
+    case 320: return launch_r<16, 20, true>(p, st);
+    case 336: return launch_r<24, 14, true>(p, st);
+    case 360: return launch_r<20, 18, true>(p, st);
+    case 384: return launch_r<16, 24, true>(p, st);
+    case 400: return launch_r<20, 20, true>(p, st);
+    case 448: return launch_r<16, 28, true>(p, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace fftk
+}  // namespace mirt

@@ -35,14 +35,7 @@ __device__ __forceinline__ ImageTile image_tile(const GlueGeom &g) {
   t.r = row - t.s * rows_per_slice;
   t.n1_0 = blockIdx.y * 32;
   t.c0 = blockIdx.z * 32;
-  long long kstr = 1, rem = t.r;
-  t.krow = 0;
-  for (int d = 1; d < g.D; d++) {
-    const long long nd = rem % g.N[d];
-    rem /= g.N[d];
-    t.krow += nd * kstr;
-    kstr *= g.K[d];
-  }
+  t.krow = image_krow(g, t.r);
   return t;
 }
 
@@ -72,7 +65,7 @@ __global__ void __launch_bounds__(256) deapod_image_cm_kernel(const float2 *__re
   for (int i = ty; i < 32; i += 8) {
     const int c = t.c0 + i;
     const int n1 = t.n1_0 + tx;
-    if (c < C && n1 < g.N[0]) pad[((t.s * C + c) * krows + t.krow) * g.K[0] + n1] = tile[tx][i];
+    if (c < C && n1 < g.N[0]) pad[((t.s * C + c) * krows + t.krow) * g.K[0] + image_k1(g, n1)] = tile[tx][i];
   }
 }
 
@@ -89,7 +82,7 @@ __global__ void __launch_bounds__(256) crop_deapod_cm_kernel(const float2 *__res
     const int c = t.c0 + i;
     const int n1 = t.n1_0 + tx;
     float2 v = make_float2(0.f, 0.f);
-    if (c < C && n1 < g.N[0]) v = grid[((t.s * C + c) * krows + t.krow) * g.K[0] + n1];
+    if (c < C && n1 < g.N[0]) v = grid[((t.s * C + c) * krows + t.krow) * g.K[0] + image_k1(g, n1)];
     tile[i][tx] = v;
   }
   __syncthreads();
@@ -103,6 +96,36 @@ __global__ void __launch_bounds__(256) crop_deapod_cm_kernel(const float2 *__res
       // a * conj(b)
       x[(t.s * g.npix + n) * C + c] = make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
     }
+  }
+}
+
+// One column: the same two kernels, a block per image row and its threads along
+// it (the tiles above would use one of their 32 coil lanes: 7 us each for 201 x
+// 175, and 22 us more for each transpose, which one column does without; the
+// forward and adjoint FFT of that image on 402 x 350 101 -> 33 us in all).
+__global__ void __launch_bounds__(256) deapod_image_1_kernel(const float2 *__restrict__ x,
+                                                             const float2 *__restrict__ sn,
+                                                             float2 *__restrict__ pad, GlueGeom g) {
+  const int rows = (int)(g.npix / g.N[0]);
+  const int s = blockIdx.x / rows, r = blockIdx.x - s * rows;
+  const float2 *xr = x + (s * (long long)rows + r) * g.N[0], *sr = sn + (long long)r * g.N[0];
+  float2 *o = pad + s * g.ngrid + image_krow(g, r) * g.K[0];
+  for (int n = threadIdx.x; n < g.N[0]; n += blockDim.x) {
+    const float2 a = xr[n], b = sr[n];
+    o[image_k1(g, n)] = make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  }
+}
+
+__global__ void __launch_bounds__(256) crop_deapod_1_kernel(const float2 *__restrict__ grid,
+                                                            const float2 *__restrict__ sn,
+                                                            float2 *__restrict__ x, GlueGeom g) {
+  const int rows = (int)(g.npix / g.N[0]);
+  const int s = blockIdx.x / rows, r = blockIdx.x - s * rows;
+  const float2 *gr = grid + s * g.ngrid + image_krow(g, r) * g.K[0], *sr = sn + (long long)r * g.N[0];
+  float2 *o = x + (s * (long long)rows + r) * g.N[0];
+  for (int n = threadIdx.x; n < g.N[0]; n += blockDim.x) {
+    const float2 a = gr[image_k1(g, n)], b = sr[n];
+    o[n] = make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
   }
 }
 
@@ -279,11 +302,21 @@ dim3 image_grid(const GlueGeom &g, int C, int nslice) {
   return dim3((unsigned)(g.npix / g.N[0] * nslice), (unsigned)((g.N[0] + 31) / 32),
               (unsigned)((C + 31) / 32));
 }
+
+int row_threads(const GlueGeom &g) {
+  const int t = (g.N[0] + 31) / 32 * 32;
+  return t > 256 ? 256 : t;
+}
 }  // namespace
 
 cudaError_t launch_deapod_image_cm(const float2 *x, const float2 *sn, float2 *pad,
                                    const GlueGeom &g, int C, int nslice, cudaStream_t st) {
   if (nslice == 0 || C == 0) return cudaSuccess;
+  if (C == 1) {
+    deapod_image_1_kernel<<<(unsigned)(g.npix / g.N[0] * nslice), row_threads(g), 0, st>>>(x, sn, pad,
+                                                                                          g);
+    return cudaGetLastError();
+  }
   deapod_image_cm_kernel<<<image_grid(g, C, nslice), dim3(32, 8), 0, st>>>(x, sn, pad, g, C);
   return cudaGetLastError();
 }
@@ -291,6 +324,11 @@ cudaError_t launch_deapod_image_cm(const float2 *x, const float2 *sn, float2 *pa
 cudaError_t launch_crop_deapod_cm(const float2 *grid, const float2 *sn, float2 *x,
                                   const GlueGeom &g, int C, int nslice, cudaStream_t st) {
   if (nslice == 0 || C == 0) return cudaSuccess;
+  if (C == 1) {
+    crop_deapod_1_kernel<<<(unsigned)(g.npix / g.N[0] * nslice), row_threads(g), 0, st>>>(grid, sn, x,
+                                                                                         g);
+    return cudaGetLastError();
+  }
   crop_deapod_cm_kernel<<<image_grid(g, C, nslice), dim3(32, 8), 0, st>>>(grid, sn, x, g, C);
   return cudaGetLastError();
 }

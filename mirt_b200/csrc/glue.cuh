@@ -20,7 +20,29 @@ struct GlueGeom {
   int K[3];            // oversampled grid size per dimension
   long long npix;      // prod(N)
   long long ngrid;     // prod(K)
+  // image pixel n sits at grid point (n - shift) mod K: a grid phase of whole
+  // periods, exp(2 pi i k shift / K), is this shift of the padded image (cuFFT
+  // path; 0 elsewhere)
+  int shift[3];
 };
+
+// grid row of image row r (the dimensions above the first), and the grid
+// position of image column n1
+__host__ __device__ inline long long image_krow(const GlueGeom &g, long long r) {
+  long long krow = 0, kstr = 1;
+  for (int d = 1; d < g.D; d++) {
+    long long nd = r % g.N[d] - g.shift[d];
+    r /= g.N[d];
+    if (nd < 0) nd += g.K[d];
+    krow += nd * kstr;
+    kstr *= g.K[d];
+  }
+  return krow;
+}
+__host__ __device__ inline int image_k1(const GlueGeom &g, int n1) {
+  const int k = n1 - g.shift[0];
+  return k < 0 ? k + g.K[0] : k;
+}
 
 // image x[s][n][c] .* sn -> the image region of the coil-major zero-padded grid
 // pad[s][c][k] (its padding is zero already and stays so)

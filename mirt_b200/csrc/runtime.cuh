@@ -120,9 +120,11 @@ struct mirt_nufft {
   mirt::GridPhase gp{};                  // tables into phtab (tab[0] null: no grid phase)
   cufftHandle fft = 0;
   bool fft_ok = false;
-  // power-of-two grids from 64 to 1024 points per dimension: the FFT runs as
-  // fused passes over `grid` itself (fft.cu) and grid_cm / pad / cuFFT are unused
+  // grids of lengths that fft_len_ok takes: the FFT runs as fused passes over
+  // `grid` itself (fft.cu) and grid_cm / pad / cuFFT are unused
   bool own_fft = false;
+  // cuFFT path, one column, no grid phase: the coil-major grid is `grid` itself
+  bool one_col = false;
   mirt::DMem twtab;                      // exp(-2 pi i k / K_d) per dimension, float2 [sum K_d]
   mirt::NufftFft nf{};
   // host-buffer calls, pipelined by slice chunks: copy streams, per-chunk

@@ -215,3 +215,30 @@ def test_argument_errors():
         mb.newfft(om, (16, 16), tables=[np.ones(6 * 512 + 1)] * 2)
     with pytest.raises(ValueError, match="J\\*L\\+1"):
         mb.newfft(om, (16, 16), tables=[np.ones(10)] * 2, sn=np.ones(256))
+
+
+@pytest.mark.parametrize("Nd,Kd,ncol", [((41, 50), (82, 100), 1), ((41, 50), (82, 100), 3),
+                                        ((13, 8, 9), (26, 22, 18), 1), ((25,), (54,), 2),
+                                        ((40, 51), (80, 112), 2), ((50, 45), (100, 120), 1)])
+def test_grid_phase_as_shift_and_tables(Nd, Kd, ncol):
+    """newfft's grid phase: a shift of the padded image where the FFT is cuFFT's
+    (odd and even Nmid, K off 2 N), per-dimension tables in the fused passes of
+    lengths whose radices do not fold it; two slices, the FP64 oracle."""
+    import torch
+    D = len(Nd)
+    rng = np.random.default_rng(sum(Nd) + ncol)
+    om = rng.uniform(-np.pi, np.pi, (150, D))
+    moff = [0, 70, 150]
+    ns = rng.uniform(0, 5, D)
+    st = mb.newfft(om, Nd, Kd=Kd, n_shift=ns, ncol=ncol, slice_moff=moff)
+    x = rng.standard_normal(st.image_shape) + 1j * rng.standard_normal(st.image_shape)
+    y = rng.standard_normal((150, ncol)) + 1j * rng.standard_normal((150, ncol))
+    X = st.forward(torch.from_numpy(x.astype(np.complex64)).cuda()).cpu().numpy()
+    z = st.adjoint(torch.from_numpy(y.astype(np.complex64)).cuda()).cpu().numpy()
+    for s in range(2):
+        sl = slice(moff[s], moff[s + 1])
+        so = nf.newfft_init(om[sl], Nd, Kd=Kd, n_shift=ns)
+        for c in range(ncol):
+            assert rel_l2(X[sl, c], nf.newfft_for(x[s, ..., c].T, so)) <= TOL
+            assert rel_l2(z[s, ..., c].T, nf.newfft_adj(y[sl, c], so)) <= TOL
+    st.close()

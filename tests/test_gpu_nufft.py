@@ -253,3 +253,58 @@ def test_nufft_init_kaiser_3d_table_test_setup():
     assert rel_l2(mb.nufft(x, st), X_o) <= 1e-5
     X = np.arange(1, len(om) + 1) + 1j
     assert rel_l2(mb.nufft_adj(X, st), nr.nufft_adj(X, so, ad)) <= 1e-5
+
+
+FFT_LENGTHS = [80, 96, 100, 112, 120, 144, 160, 192, 200, 224, 240, 280, 288, 320, 336, 360, 384, 400,
+               448, 480, 560, 576, 640, 672, 768, 896]
+
+
+@pytest.mark.parametrize("K", FFT_LENGTHS)
+def test_fft_lengths_off_the_powers_of_two(K):
+    """Every length of the fused passes that is no power of two, in 1D: half the
+    grid (the pruned passes: N = K/2), an odd N below it, and N > K/2 (unpruned),
+    with vectors of 1, 8 and 16 columns; the FP64 oracle."""
+    import torch
+    rng = np.random.default_rng(K)
+    om = rng.uniform(-np.pi, np.pi, (60, 1))
+    for N, C in ((K // 2, 1), (K // 2, 8), (K // 2, 16), (K // 2 - 3, 8), (K - 5, 16), (K // 2 + 1, 1)):
+        plan = mb.NufftPlan(om, (N,), (6,), (K,), n_shift=(N / 2,), Ld=512, ncol=C)
+        assert plan.fft_config()["fused_fft"] == 1
+        st_o = nr.nufft_init_table(om, (N,), (6,), (K,), (N / 2,), 512)
+        fw, ad = _oracle_pair(st_o)
+        x = rng.standard_normal((1, N, C)) + 1j * rng.standard_normal((1, N, C))
+        y = rng.standard_normal((60, C)) + 1j * rng.standard_normal((60, C))
+        X = plan.forward(torch.from_numpy(x.astype(np.complex64)).cuda()).cpu().numpy()
+        z = plan.adjoint(torch.from_numpy(y.astype(np.complex64)).cuda()).cpu().numpy()
+        for c in (0, C - 1):
+            assert rel_l2(X[:, c], nr.nufft(x[0, :, c], st_o, fw)) <= FWD_TOL, (N, C, c)
+            assert rel_l2(z[0, :, c], nr.nufft_adj(y[:, c], st_o, ad)) <= ADJ_TOL, (N, C, c)
+        plan.close()
+
+
+@pytest.mark.parametrize("N,K,C", [((50, 41), (100, 82), 1), ((50, 41), (100, 82), 3),
+                                   ((11, 9, 7), (22, 18, 14), 1), ((33,), (66,), 1)])
+def test_grids_through_cufft(N, K, C):
+    """Grids the fused passes do not take, one column (no transposes) and several,
+    two slices; nufft against the FP64 oracle."""
+    import torch
+    D = len(N)
+    rng = np.random.default_rng(C + sum(K))
+    om = rng.uniform(-np.pi, np.pi, (120, D))
+    moff = [0, 50, 120]
+    ns = tuple(n / 2 for n in N)
+    plan = mb.NufftPlan(om, N, (6,) * D, K, n_shift=ns, Ld=512, ncol=C, slice_moff=moff)
+    assert plan.fft_config()["fused_fft"] == 0
+    x = rng.standard_normal(plan.image_shape) + 1j * rng.standard_normal(plan.image_shape)
+    y = rng.standard_normal((120, C)) + 1j * rng.standard_normal((120, C))
+    X = plan.forward(torch.from_numpy(x.astype(np.complex64)).cuda()).cpu().numpy()
+    z = plan.adjoint(torch.from_numpy(y.astype(np.complex64)).cuda()).cpu().numpy()
+    a, b = plan.forward_host(x.astype(np.complex64)), plan.adjoint_host(y.astype(np.complex64))
+    assert rel_l2(a, X) <= 1e-6 and rel_l2(b, z) <= 1e-6
+    for s in range(2):
+        sl = slice(moff[s], moff[s + 1])
+        st_o = nr.nufft_init_table(om[sl], N, (6,) * D, K, ns, 512)
+        fw, ad = _oracle_pair(st_o)
+        assert rel_l2(X[sl, C - 1], nr.nufft(x[s, ..., C - 1].T, st_o, fw)) <= FWD_TOL
+        assert rel_l2(z[s, ..., C - 1].T, nr.nufft_adj(y[sl, C - 1], st_o, ad)) <= ADJ_TOL
+    plan.close()
