@@ -99,3 +99,27 @@ def test_nrmse_tracking_weighted_and_warm_start():
     A.cg(x0, y, 5, W=wn)
     nr2, _ = A.cg(x0, y, 60, xref=xref)
     assert np.all(nr2[-1] <= 1e-3), nr2[-1]
+
+
+@pytest.mark.parametrize("N,C,spokes", [(9, 3, [5, 4, 7]), (70, 9, [30, 21])])
+def test_block_sums_of_small_and_large_problems(N, C, spokes):
+    """The inner products over one block a problem (9 x 9 images, 7 columns in the
+    last lane group) and over many; FP64 iterates of weighted CG, twice the same
+    bits, and the tracked NRMSE of a zero start."""
+    import torch
+    A, refs, xt, ys, moff = _batch(7 + N, N, 2 * N, C, spokes)
+    rng = np.random.default_rng(N)
+    W = rng.uniform(0.5, 1.5, int(moff[-1])).astype(np.float32)
+    y = torch.from_numpy(np.concatenate(ys).astype(np.complex64)).cuda()
+    xr = torch.from_numpy(xt.astype(np.complex64)).cuda()
+    x = torch.zeros(A.image_shape, dtype=torch.complex64, device="cuda")
+    nr, _ = A.cg(x, y, 4, W=torch.from_numpy(W).cuda(), xref=xr)
+    x2 = torch.zeros_like(x)
+    A.cg(x2, y, 4, W=torch.from_numpy(W).cuda())
+    assert torch.equal(x, x2)
+    for s, R in enumerate(refs):
+        it = qpwls_pcg1(np.zeros_like(xt[s]), R, W[moff[s]:moff[s + 1]], ys[s], 4)
+        assert rel_l2(x[s].cpu().numpy(), it[4]) <= 1e-4
+        for k in range(5):
+            ref = np.linalg.norm(it[k] - xt[s]) / np.linalg.norm(xt[s])
+            assert abs(nr[k, s] - ref) <= 1e-4 * max(ref, 1)
