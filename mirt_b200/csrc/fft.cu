@@ -2,6 +2,8 @@
 // lengths and their dispatch, and the forward and adjoint pass sequences.
 #include "fft_impl.cuh"
 
+#include <cmath>
+
 namespace mirt {
 namespace {
 
@@ -80,6 +82,39 @@ cudaError_t launch_fft_pass(const FftPass &p, cudaStream_t st) {
   }
 }
 
+cudaError_t launch_circulant_pass(const CirculantPass &p, cudaStream_t st) {
+  const FftLen *l = find_len(p.n);
+  if (!l || p.vw < 1 || p.vw > 16 || (p.vw & (p.vw - 1)) || p.nvec < 1) return cudaErrorInvalidValue;
+  if ((long long)p.nslice * p.nvec >= (1ll << 31)) return cudaErrorInvalidValue;
+  switch (l->unit) {
+    case 1: return fftk::launch_c1(p, st);
+    case 2: return fftk::launch_c2(p, st);
+    case 3: return fftk::launch_c3(p, st);
+    default: break;
+  }
+  switch (p.n) {
+    case 64: return fftk::launch_c<8, 8>(p, st);
+    case 128: return fftk::launch_c<8, 16>(p, st);
+    case 256: return fftk::launch_c<16, 16>(p, st);
+    case 512: return fftk::launch_c<16, 32>(p, st);
+    case 1024: return fftk::launch_c<32, 32>(p, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+void fft_twiddles(int n, bool inverse, std::vector<float2> &tw) {
+  int r1 = 0, r2 = 0;
+  fft_radix(n, &r1, &r2);
+  tw.clear();
+  for (int q = 0; q < r2; q++)
+    for (int p1 = 0; p1 < r1; p1++) {
+      const double a = fftk::kTwoPi * (double)(((long long)p1 * q) % n) / n;
+      tw.push_back(make_float2((float)std::cos(a), (float)(inverse ? std::sin(a) : -std::sin(a))));
+    }
+}
+
+int fft_vec_width(long long v) { return vec_width(v); }
+
 void fft_radix(int n, int *r1, int *r2) {
   const FftLen *l = find_len(n);
   *r1 = l ? l->r1 : 0;
@@ -89,7 +124,7 @@ void fft_radix(int n, int *r1, int *r2) {
 int fft_nufft_passes(const NufftFft &f) { return f.g.D; }
 
 cudaError_t fft_nufft_forward(const NufftFft &f, const float2 *x, float2 *grid, int s0, int s1,
-                              cudaStream_t st) {
+                              cudaStream_t st, const float2 *img) {
   const GlueGeom &g = f.g;
   const long long C = f.C, xs = g.npix * C, gs = g.ngrid * C;
   if (s1 <= s0 || C == 0) return cudaSuccess;
@@ -114,7 +149,8 @@ cudaError_t fft_nufft_forward(const NufftFft &f, const float2 *x, float2 *grid, 
     p.nvec = (int)(C / p.vw);
     p.nin = N1;
     p.nout = K1;
-    p.sn_in = f.sn;
+    p.sn_in = img ? img + s0 * g.npix : f.sn;
+    p.sn_rows = img ? N2 * N3 : 0;
     cudaError_t e = launch_fft_pass(p, st);
     if (e != cudaSuccess || g.D == 1) return e;
   }

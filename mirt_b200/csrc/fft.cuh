@@ -18,6 +18,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "glue.cuh"
 
 namespace mirt {
@@ -39,9 +41,11 @@ struct FftPass {
   // phase folded in (FP64-built; see NufftFft)
   const float2 *tw;
   int tw_unit0;              // 1: the twiddle of p1 = 0 is 1 in every column (skipped)
-  // deapodisation: sn_in scales input k of line (r2, r1) by sn[(r2*nr1 + r1)*nin + k];
+  // deapodisation: sn_in scales input k of line (s, r2, r1) by
+  // sn[(s*sn_rows + r2*nr1 + r1)*nin + k] (sn_rows 0: one image for every slice);
   // sn_out scales output p by conj(sn[(r2*nr1 + r1)*nout + p])
   const float2 *sn_in, *sn_out;
+  int sn_rows;
   // grid phase of this dimension: ph_out[p] on outputs, conj(ph_in[k]) on inputs
   const float2 *ph_out, *ph_in;
 };
@@ -59,6 +63,28 @@ bool fft_fold_ok(int n);
 void fft_radix(int n, int *r1, int *r2);
 
 cudaError_t launch_fft_pass(const FftPass &p, cudaStream_t st);
+
+// The last forward pass of a zero-padded transform, the product with a spectrum
+// and the first pass of the inverse in one kernel, in place on the n/2 kept
+// elements of each line: io[k] <- scale IDFT(H . DFT(io zero-padded to n))[k],
+// k < n/2.  Lines as in FftPass with one slice stride; element e of a line's
+// vectors (e = w*vw + v) takes the spectrum of column e / C of the n1 columns,
+// H[(s*n + p)*n1 + e/C] (complex) or Hr (real).
+struct CirculantPass {
+  float2 *io;
+  int nslice, nvec, vw, n, C, n1;
+  long long slice, es;
+  const float2 *tw;          // stage-1 twiddles of the forward transform (FftPass)
+  const float2 *H;
+  const float *Hr;
+  float scale;
+};
+cudaError_t launch_circulant_pass(const CirculantPass &p, cudaStream_t st);
+
+// Stage-1 twiddles [q][p1] of a length, forward exp(-2 pi i p1 q / n) or inverse
+void fft_twiddles(int n, bool inverse, std::vector<float2> &tw);
+// widest vector (16 or less) that divides v elements
+int fft_vec_width(long long v);
 
 // Geometry of the NUFFT's FFT: image N, grid K, C columns, per-dimension
 // stage-1 twiddle tables of the forward and the adjoint passes (device,
@@ -79,9 +105,10 @@ struct NufftFft {
   int phase_folded;
 };
 
-// fftn(x .* sn, K) of slices [s0, s1): x [s][n][c] -> grid [s][k][c]
+// fftn(x .* sn, K) of slices [s0, s1): x [s][n][c] -> grid [s][k][c].  With img
+// [s][n]: of x .* img instead (x: maps times sn, an image common to all columns)
 cudaError_t fft_nufft_forward(const NufftFft &f, const float2 *x, float2 *grid, int s0, int s1,
-                              cudaStream_t st);
+                              cudaStream_t st, const float2 *img = nullptr);
 // prod(K) ifftn(grid), cropped, .* conj(sn), slices [s0, s1): grid is overwritten
 cudaError_t fft_nufft_adjoint(const NufftFft &f, float2 *grid, float2 *x, int s0, int s1,
                               cudaStream_t st);

@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
       const int s = o / P.nr2;
       bi = s * P.is[0] + r2 * P.is[1] + r1 * P.is[2] + (long long)w * vw;
       bo = s * P.os[0] + r2 * P.os[1] + r1 * P.os[2] + (long long)w * vw;
-      row = r2 * P.nr1 + r1;
+      row = s * P.sn_rows + r2 * P.nr1 + r1;
     }
     base_in[threadIdx.x] = bi;
     base_out[threadIdx.x] = bo;
@@ -351,32 +351,169 @@ __global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
   }
 }
 
+// ---- forward, spectrum, inverse ------------------------------------------------
+// Stage 1 and stage 2 of the forward transform as in fft_pass_kernel (inputs
+// pruned to n/2), so that thread (line, p1) holds X[p1 + R1 p2] for all p2; times
+// the spectrum; then the inverse with k = p1 + R1 p2 and m = m2 + R2 m1,
+//   x[m] = sum_p1 W_R1^{m1 p1} W_n^{m2 p1} sum_p2 W_R2^{m2 p2} Y[p1 + R1 p2],
+// whose first radix-R2 stage stays in that thread's registers and goes back to
+// the same row of shared memory, and whose radix-R1 stage forms the first half of
+// its outputs (m < n/2).
+template <int R1, int R2, int VW>
+__global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
+    circulant_pass_kernel(CirculantPass P, int lpb, int pitch_rt) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int vw = VW ? VW : P.vw;
+  const int lvw = VW ? (VW == 16 ? 4 : 3) : __ffs(vw) - 1;
+  const int pitch = VW ? R2 * VW + (VW < 16 ? VW : 0) : pitch_rt;
+  const int nlines = P.nslice * P.nvec;
+  const int g0 = blockIdx.x * lpb;
+  auto line = [&](int g, int v) -> float2 * {
+    const int gl = g0 + g;
+    if (gl >= nlines) return nullptr;
+    const int s = gl / P.nvec, w = gl - s * P.nvec;
+    return P.io + s * P.slice + ((long long)w << lvw) + v;
+  };
+  // stage 1
+  const int n1 = (lpb * R2) << lvw;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n1; i += blockDim.x) {
+    const int v = i & (vw - 1), q = (i >> lvw) % R2, g = (i >> lvw) / R2;
+    const float2 *sp = line(g, v);
+    if (!sp) continue;
+    float2 x[R1];
+    sp += (long long)q * P.es;
+    const long long st = (long long)R2 * P.es;
+#pragma unroll
+    for (int k1 = 0; k1 < R1; k1++) {
+      x[k1] = make_float2(0.f, 0.f);
+      if (k1 < R1 / 2) {
+        x[k1] = *sp;
+        sp += st;
+      }
+    }
+    dft_half_in<R1, false>(x);
+    const float4 *tw4 = reinterpret_cast<const float4 *>(P.tw) + q * (R1 / 2);
+#pragma unroll
+    for (int j = 0; j < R1 / 2; j++) {
+      const float4 t = __ldg(tw4 + j);
+      if (j > 0) x[2 * j] = cmul(x[2 * j], make_float2(t.x, t.y));
+      x[2 * j + 1] = cmul(x[2 * j + 1], make_float2(t.z, t.w));
+    }
+    float2 *d = sm + (size_t)(g * R1) * pitch + (q << lvw) + v;
+#pragma unroll
+    for (int p1 = 0; p1 < R1; p1++) d[p1 * pitch] = x[p1];
+  }
+  __syncthreads();
+  // stage 2, spectrum, inverse stage 1
+  const int n2 = (lpb * R1) << lvw;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+    const int v = i & (vw - 1), p1 = (i >> lvw) % R1, g = (i >> lvw) / R1;
+    const int gl = g0 + g;
+    if (gl >= nlines) continue;
+    float2 y[R2];
+    float2 *s = sm + (size_t)(g * R1 + p1) * pitch + v;
+#pragma unroll
+    for (int k = 0; k < R2; k++) y[k] = s[k << lvw];
+    Dft<R2, false>::run(y);
+    const int sl = gl / P.nvec, w = gl - sl * P.nvec;
+    const long long h0 = ((long long)sl * P.n + p1) * P.n1 + ((w << lvw) + v) / P.C;
+    const long long hs = (long long)R1 * P.n1;
+    if (P.Hr) {
+      const float *h = P.Hr + h0;
+#pragma unroll
+      for (int k = 0; k < R2; k++) {
+        const float a = P.scale * __ldg(h);
+        h += hs;
+        y[k] = make_float2(a * y[k].x, a * y[k].y);
+      }
+    } else {
+      const float2 *h = P.H + h0;
+#pragma unroll
+      for (int k = 0; k < R2; k++) {
+        const float2 a = __ldg(h);
+        h += hs;
+        y[k] = cmul(y[k], make_float2(P.scale * a.x, P.scale * a.y));
+      }
+    }
+    Dft<R2, true>::run(y);
+    const float2 *tw = P.tw + p1;  // conj(W_n^{m2 p1})
+#pragma unroll
+    for (int k = 0; k < R2; k++) s[k << lvw] = k ? cmulc(__ldg(tw + k * R1), y[k]) : y[k];
+  }
+  __syncthreads();
+  // inverse stage 2: outputs m = m2 + R2 m1, m1 < R1 / 2
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n1; i += blockDim.x) {
+    const int v = i & (vw - 1), q = (i >> lvw) % R2, g = (i >> lvw) / R2;
+    float2 *dp = line(g, v);
+    if (!dp) continue;
+    float2 x[R1];
+    const float2 *d = sm + (size_t)(g * R1) * pitch + (q << lvw) + v;
+#pragma unroll
+    for (int p1 = 0; p1 < R1; p1++) x[p1] = d[p1 * pitch];
+    dft_half_out<R1, true>(x);
+    dp += (long long)q * P.es;
+    const long long st = (long long)R2 * P.es;
+#pragma unroll
+    for (int m1 = 0; m1 < R1 / 2; m1++) {
+      *dp = x[m1];
+      dp += st;
+    }
+  }
+}
+
+// lines per block and the block size whose sweeps over the stages' items (lpb R2
+// vw twice or once, lpb R1 vw) idle least
+template <int R1, int R2>
+void block_shape(int vw, int stages_r2, int *lpb, unsigned *threads) {
+  *lpb = kThreads / ((R1 < R2 ? R1 : R2) * vw);
+  if (*lpb < 1) *lpb = 1;
+  if (*lpb > kMaxLpb) *lpb = kMaxLpb;
+  const unsigned n1 = *lpb * R2 * vw, n2 = *lpb * R1 * vw;
+  unsigned best = ~0u;
+  for (unsigned t = kThreads; t >= 96; t -= 32) {
+    const unsigned work = (stages_r2 * ((n1 + t - 1) / t) + (n2 + t - 1) / t) * t;
+    if (work < best) {
+      best = work;
+      *threads = t;
+    }
+  }
+}
+
+template <int R1, int R2>
+cudaError_t launch_c(const CirculantPass &P, cudaStream_t st) {
+  int lpb = 1;
+  unsigned threads = kThreads;
+  block_shape<R1, R2>(P.vw, 2, &lpb, &threads);
+  const int pitch = R2 * P.vw + (P.vw < 16 ? P.vw : 0);
+  const size_t smem = (size_t)lpb * R1 * pitch * sizeof(float2);
+  const long long nlines = (long long)P.nslice * P.nvec;
+  if (nlines <= 0) return cudaSuccess;
+  const unsigned grid = (unsigned)((nlines + lpb - 1) / lpb);
+  auto kern = P.vw == 16 ? circulant_pass_kernel<R1, R2, 16> : circulant_pass_kernel<R1, R2, 0>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  kern<<<grid, threads, smem, st>>>(P, lpb, pitch);
+  return cudaGetLastError();
+}
+
 // EXTRA: a length off the powers of two; the exact forms only where pruned
 // (K >= 2 N, the usual oversampling), the general form elsewhere
 template <int R1, int R2, bool EXTRA = false>
 cudaError_t launch_r(const FftPass &P, cudaStream_t st) {
   const int vw = P.vw;
-  int lpb = kThreads / ((R1 < R2 ? R1 : R2) * vw);
-  if (lpb < 1) lpb = 1;
-  if (lpb > kMaxLpb) lpb = kMaxLpb;
+  int lpb = 1;
+  unsigned threads = kThreads;
+  block_shape<R1, R2>(vw, 1, &lpb, &threads);
+  if (!EXTRA) threads = kThreads;
   const int pitch = R2 * vw + (vw < 16 ? vw : 0);
   const size_t smem = (size_t)lpb * R1 * pitch * sizeof(float2);
   const long long nlines = (long long)P.nslice * P.nr2 * P.nr1 * P.nvec;
   if (nlines <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((nlines + lpb - 1) / lpb);
-  // the block size whose last sweep over the two stages' items idles least
-  unsigned threads = kThreads;
-  if (EXTRA) {
-    const unsigned n1 = lpb * R2 * vw, n2 = lpb * R1 * vw;
-    unsigned best = ~0u;
-    for (unsigned t = kThreads; t >= 96; t -= 32) {
-      const unsigned work = ((n1 + t - 1) / t + (n2 + t - 1) / t) * t;
-      if (work < best) {
-        best = work;
-        threads = t;
-      }
-    }
-  }
   const bool prune = P.inverse ? (2 * P.nout <= P.n) : (2 * P.nin <= P.n);
   auto pick = [&](auto kern) -> cudaError_t {
     cudaError_t e =
@@ -412,6 +549,9 @@ cudaError_t launch_r(const FftPass &P, cudaStream_t st) {
 cudaError_t launch_l1(const FftPass &p, cudaStream_t st);
 cudaError_t launch_l2(const FftPass &p, cudaStream_t st);
 cudaError_t launch_l3(const FftPass &p, cudaStream_t st);
+cudaError_t launch_c1(const CirculantPass &p, cudaStream_t st);
+cudaError_t launch_c2(const CirculantPass &p, cudaStream_t st);
+cudaError_t launch_c3(const CirculantPass &p, cudaStream_t st);
 
 }  // namespace fftk
 }  // namespace mirt

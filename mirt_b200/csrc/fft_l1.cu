@@ -20,5 +20,21 @@ cudaError_t launch_l1(const FftPass &p, cudaStream_t st) {
   }
 }
 
+cudaError_t launch_c1(const CirculantPass &p, cudaStream_t st) {
+  switch (p.n) {
+    case 80: return launch_c<8, 10>(p, st);
+    case 96: return launch_c<8, 12>(p, st);
+    case 100: return launch_c<10, 10>(p, st);
+    case 112: return launch_c<8, 14>(p, st);
+    case 120: return launch_c<12, 10>(p, st);
+    case 144: return launch_c<12, 12>(p, st);
+    case 160: return launch_c<8, 20>(p, st);
+    case 192: return launch_c<12, 16>(p, st);
+    case 200: return launch_c<20, 10>(p, st);
+    case 224: return launch_c<16, 14>(p, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 }  // namespace fftk
 }  // namespace mirt

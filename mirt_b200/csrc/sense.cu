@@ -159,6 +159,14 @@ __global__ void __launch_bounds__(256) k_combine(const float2 *__restrict__ z,
     finish_dot(dot, acc, [&](double v) { new_product(sc + blockIdx.y * SC_N, v, first); });
 }
 
+// out[s][p][c] = sens[s][p][c] sn[p]
+__global__ void k_maps_sn(const float2 *__restrict__ sens, const float2 *__restrict__ sn,
+                          float2 *__restrict__ out, long long n, long long np, int C) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
+       e += (long long)gridDim.x * blockDim.x)
+    out[e] = cmul(sens[e], sn[e / C % np]);
+}
+
 // r = W (y - Ax), W per sample (all coils) or 1
 __global__ void k_resid(const float2 *__restrict__ y, const float2 *__restrict__ Ax,
                         const float *__restrict__ W, float2 *__restrict__ r, long long n, int C) {
@@ -361,20 +369,6 @@ __global__ void __launch_bounds__(256) k_errnorm(const float2 *__restrict__ x,
   finish_dot(dot, acc, [&](double w) { out[blockIdx.y] = w; });
 }
 
-}  // namespace
-
-struct mirt_sense {
-  mirt_nufft *G = nullptr;
-  int S = 0, C = 0, N1 = 0, N2 = 0;
-  long long np = 0, M = 0;
-  DMem sens, beta, z, ioff, soff;
-  std::vector<double> beta_host;
-  mirt_toeplitz *T = nullptr;  // Gram operator and preconditioner (mirt_sense_toeplitz)
-  ~mirt_sense() { delete T; }
-};
-
-namespace {
-
 // Blocks per problem of a kernel over n elements a problem: about kBlocks in all
 // (16 blocks of 256 threads per SM: two waves), at least 512 elements each.
 constexpr int kBlocks = 148 * 16;
@@ -382,6 +376,32 @@ unsigned problem_blocks(long long n, int S) {
   const long long p = std::min((kBlocks + S - 1ll) / S, (n + 511) / 512);
   return (unsigned)std::max(1ll, p);
 }
+
+}  // namespace
+
+namespace mirt {
+cudaError_t launch_coil_combine(const float2 *z, const float2 *sens, float2 *out, long long np, int C,
+                                int S, cudaStream_t st) {
+  k_combine<false><<<dim3(problem_blocks(np * 8, S), S), 256, 0, st>>>(z, sens, nullptr, out, np, C,
+                                                                      DotBuf{}, nullptr, 0);
+  return cudaGetLastError();
+}
+}  // namespace mirt
+
+struct mirt_sense {
+  mirt_nufft *G = nullptr;
+  int S = 0, C = 0, N1 = 0, N2 = 0;
+  long long np = 0, M = 0;
+  DMem sens, beta, z, ioff, soff;
+  // sens .* sn where the NUFFT's FFT runs as fused passes: A's first pass reads it
+  // times the image, so that the coil images are never written
+  DMem sens_sn;
+  std::vector<double> beta_host;
+  mirt_toeplitz *T = nullptr;  // Gram operator and preconditioner (mirt_sense_toeplitz)
+  ~mirt_sense() { delete T; }
+};
+
+namespace {
 
 // the inner products' buffers of one call
 struct DotMem {
@@ -397,6 +417,11 @@ struct DotMem {
 };
 
 int sense_A(mirt_sense *op, const float2 *x, float2 *y, cudaStream_t st) {
+  mirt_nufft *G = op->G;
+  if (op->sens_sn.p) {
+    SCK(fft_nufft_forward(G->nf, op->sens_sn.as<float2>(), G->grid.as<float2>(), 0, op->S, st, x));
+    return mirt_interp_plan_forward(G->ip, G->grid.p, y, st);
+  }
   const long long n = (long long)op->S * op->np * op->C;
   k_expand<<<nblocks(n), 256, 0, st>>>(x, op->sens.as<float2>(), op->z.as<float2>(), n, op->C);
   SCK(cudaGetLastError());
@@ -474,6 +499,14 @@ int mirt_sense_create(mirt_sense **out, mirt_nufft *G, const void *sens, const d
                               cudaMemcpyHostToDevice, st);
   if (!e) e = cudaMemcpyAsync(op->soff.p, so.data(), so.size() * sizeof(long long),
                               cudaMemcpyHostToDevice, st);
+  if (!e && G->own_fft && op->S > 0 && op->C > 0) {
+    const long long n = (long long)nimg * op->C;
+    if (op->sens_sn.alloc(n * sizeof(float2)))
+      return bail(api_fail(MIRT_ERR_ALLOC, "CG-SENSE buffers"));
+    k_maps_sn<<<nblocks(n), 256, 0, st>>>(op->sens.as<float2>(), G->sn.as<float2>(),
+                                          op->sens_sn.as<float2>(), n, op->np, op->C);
+    e = cudaGetLastError();
+  }
   if (!e) e = cudaStreamSynchronize(st);
   if (e) return bail(api_fail(MIRT_ERR_CUDA, cudaGetErrorString(e)));
   *out = op;

@@ -238,6 +238,66 @@ __global__ void k_dcf_blend(const float2 *__restrict__ Hw, const float *__restri
   }
 }
 
+// crop(IFFT(H FFT(pad(in)))) / (4 N1 N2) of nc columns as three fused passes: along
+// dimension 1 into the image rows of the work grid (times img, one image for all
+// columns, when given), along dimension 2 forward, times the spectrum and back in
+// one kernel, and along dimension 1 back to the N1 kept columns.  H complex or Hr
+// real.  (6 problems of 16 columns, N = 256: 526 us through cuFFT with its pad,
+// product and crop passes, 178 us; bound by the latency of the passes' loads.)
+cudaError_t own_circulant(mirt_toeplitz *T, int nc, const float2 *in, const float2 *img,
+                          const float2 *H, const float *Hr, float2 *out, cudaStream_t st) {
+  const long long N1 = T->N1, N2 = T->N2, row = 2 * N1 * nc;
+  float2 *work = T->work.as<float2>();
+  FftPass a{};
+  a.in = in;
+  a.out = work;
+  a.nslice = T->S;
+  a.nr2 = 1;
+  a.nr1 = (int)N2;
+  a.vw = fft_vec_width(nc);
+  a.nvec = nc / a.vw;
+  a.is[0] = N1 * N2 * nc;
+  a.is[2] = N1 * nc;
+  a.os[0] = N2 * row;
+  a.os[2] = row;
+  a.es_in = a.es_out = nc;
+  a.n = (int)(2 * N1);
+  a.nin = (int)N1;
+  a.nout = (int)(2 * N1);
+  a.tw = T->tw1f;
+  a.tw_unit0 = 1;
+  a.sn_in = img;
+  a.sn_rows = (int)N2;
+  cudaError_t e = launch_fft_pass(a, st);
+  if (e != cudaSuccess) return e;
+  CirculantPass c{};
+  c.io = work;
+  c.nslice = T->S;
+  c.vw = fft_vec_width(row);
+  c.nvec = (int)(row / c.vw);
+  c.n = (int)(2 * N2);
+  c.C = nc;
+  c.n1 = (int)(2 * N1);
+  c.slice = N2 * row;
+  c.es = row;
+  c.tw = T->tw2f;
+  c.H = H;
+  c.Hr = Hr;
+  c.scale = 1.f / (float)(4 * N1 * N2);
+  e = launch_circulant_pass(c, st);
+  if (e != cudaSuccess) return e;
+  std::swap(a.is[0], a.os[0]);
+  std::swap(a.is[2], a.os[2]);
+  a.in = work;
+  a.out = out;
+  a.nin = (int)(2 * N1);
+  a.nout = (int)N1;
+  a.inverse = 1;
+  a.tw = T->tw1a;
+  a.sn_in = nullptr;
+  return launch_fft_pass(a, st);
+}
+
 int make_plan(cufftHandle *h, int N1, int N2, int batch) {
   int n[2] = {2 * N2, 2 * N1};
   const int P = 4 * N1 * N2;
@@ -291,11 +351,30 @@ int toep_create(mirt_toeplitz **out, const double *om, long long M, const long l
     if (code) delete T;
     return code;
   };
+  T->own = fft_len_ok(2 * T->N1) && fft_len_ok(2 * T->N2);
   if (f.alloc(std::max<long long>(M, 1) * sizeof(float2)) ||
       b1.alloc(nslice * np * sizeof(float2)) || b2.alloc(nslice * np * sizeof(float2)) ||
       T->H.alloc(nslice * P * sizeof(float2)) ||
-      T->pad.alloc((size_t)nslice * ncol * P * sizeof(float2)))
+      (T->own ? T->work.alloc((size_t)nslice * ncol * (P / 2) * sizeof(float2)) ||
+                    T->z.alloc((size_t)nslice * ncol * (P / 4) * sizeof(float2))
+              : T->pad.alloc((size_t)nslice * ncol * P * sizeof(float2))))
     return fin(api_fail(MIRT_ERR_ALLOC, "Toeplitz buffers"));
+  if (T->own) {
+    std::vector<float2> tw, t;
+    size_t at[3];
+    for (int k = 0; k < 3; k++) {
+      fft_twiddles(2 * (k < 2 ? T->N1 : T->N2), k == 1, t);
+      at[k] = tw.size();
+      tw.insert(tw.end(), t.begin(), t.end());
+    }
+    if (T->tw.alloc(tw.size() * sizeof(float2)) ||
+        cudaMemcpyAsync(T->tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, st) ||
+        cudaStreamSynchronize(st))
+      return fin(api_fail(MIRT_ERR_ALLOC, "Toeplitz twiddles"));
+    T->tw1f = T->tw.as<float2>() + at[0];
+    T->tw1a = T->tw.as<float2>() + at[1];
+    T->tw2f = T->tw.as<float2>() + at[2];
+  }
   k_w_to_c64<<<nblk(M), 256, 0, st>>>(w, M, f.as<float2>());
   rc = mirt_nufft_adjoint(g1, f.p, b1.p, st);
   if (!rc) rc = mirt_nufft_adjoint(g2, f.p, b2.p, st);
@@ -306,7 +385,7 @@ int toep_create(mirt_toeplitz **out, const double *om, long long M, const long l
   rc = make_plan(&T->fft_1, T->N1, T->N2, nslice);
   if (rc) return fin(rc);
   T->ok_1 = true;
-  if (ncol > 1) {
+  if (ncol > 1 && !T->own) {
     rc = make_plan(&T->fft_n, T->N1, T->N2, nslice * ncol);
     if (rc) return fin(rc);
     T->ok_n = true;
@@ -324,6 +403,11 @@ int toep_gram_sense(mirt_toeplitz *T, const float2 *x, const float2 *sens, float
                     cudaStream_t st) {
   const int S = T->S, nc = T->ncol;
   const long long P = 4ll * T->N1 * T->N2;
+  if (T->own) {
+    TCK(own_circulant(T, nc, sens, x, T->H.as<float2>(), nullptr, T->z.as<float2>(), st));
+    TCK(launch_coil_combine(T->z.as<float2>(), sens, out, P / 4, nc, S, st));
+    return MIRT_OK;
+  }
   cufftHandle h = nc > 1 ? T->fft_n : T->fft_1;
   float2 *u = T->pad.as<float2>();
   k_pad<<<nblk(S * nc * P), 256, 0, st>>>(x, sens, u, S, nc, T->N1, T->N2, 1);
@@ -384,6 +468,10 @@ int toep_precon_dcf(mirt_toeplitz *T, const mirt_toeplitz *Tw, double blend, cud
 int toep_precon_apply(mirt_toeplitz *T, const float2 *x, float2 *out, cudaStream_t st) {
   const int S = T->S;
   const long long P = 4ll * T->N1 * T->N2;
+  if (T->own) {
+    TCK(own_circulant(T, 1, x, nullptr, nullptr, T->Hp.as<float>(), out, st));
+    return MIRT_OK;
+  }
   float2 *u = T->pad.as<float2>();  // the first S planes of the work grid
   k_pad<<<nblk(S * P), 256, 0, st>>>(x, nullptr, u, S, 1, T->N1, T->N2, 1);
   int rc = fft(T->fft_1, u, CUFFT_FORWARD, st);
@@ -416,6 +504,11 @@ int mirt_toeplitz_apply(mirt_toeplitz *T, const void *x, void *y, void *stream) 
   cudaStream_t st = as_stream(stream);
   const int S = T->S, nc = T->ncol;
   const long long P = 4ll * T->N1 * T->N2;
+  if (T->own) {
+    TCK(own_circulant(T, nc, static_cast<const float2 *>(x), nullptr, T->H.as<float2>(), nullptr,
+                      static_cast<float2 *>(y), st));
+    return MIRT_OK;
+  }
   cufftHandle h = nc > 1 ? T->fft_n : T->fft_1;
   float2 *u = T->pad.as<float2>();
   k_pad<<<nblk(S * nc * P), 256, 0, st>>>(static_cast<const float2 *>(x), nullptr, u, S, nc, T->N1,

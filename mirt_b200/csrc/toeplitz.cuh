@@ -14,6 +14,13 @@ struct mirt_toeplitz {
   mirt::DMem H;    // complex64 [S][2N2][2N1]: FFT of the circulant kernel
   mirt::DMem Hp;   // float [S][2N2][2N1]: circulant preconditioner spectrum (or empty)
   mirt::DMem Hp1;  // float [S][2N2][2N1]: the unweighted spectrum, kept when Hp is blended
+  // Sizes 2N that fft_len_ok takes: the padded transforms run as fused passes on
+  // `work`, the N2 image rows of a coil-innermost grid [S][N2][2N1][ncol] (the rows
+  // of padding exist only inside the pass along dimension 2), with `z` the coil
+  // images of the SENSE form.  Others: cuFFT on the coil-major `pad`.
+  bool own = false;
+  mirt::DMem work, z, tw;  // tw: stage-1 twiddles of 2N1 forward, 2N1 inverse, 2N2 forward
+  const float2 *tw1f = nullptr, *tw1a = nullptr, *tw2f = nullptr;
   mirt::DMem pad;  // complex64 [S * ncol][2N2][2N1]: work grid
   cufftHandle fft_n = 0, fft_1 = 0;  // batches S * ncol and S
   bool ok_n = false, ok_1 = false;
@@ -32,6 +39,10 @@ int toep_create(mirt_toeplitz **out, const double *om, long long M, const long l
 // out[s][p] = sum_c conj(sens[s][p][c]) (T_s (sens_c x_s))[p]   (ncol = C)
 int toep_gram_sense(mirt_toeplitz *T, const float2 *x, const float2 *sens, float2 *out,
                     cudaStream_t st);
+
+// out[s][p] = sum_c conj(sens[s][p][c]) z[s][p][c] (sense.cu)
+cudaError_t launch_coil_combine(const float2 *z, const float2 *sens, float2 *out, long long np, int C,
+                                int S, cudaStream_t st);
 
 // Circulant preconditioner spectrum 1 / max(lam_s Re H_s + r_s, floor_s),
 // r_s the spectrum of the quadratic first-order penalty with weight beta_s

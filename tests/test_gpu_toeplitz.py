@@ -42,6 +42,28 @@ def test_gram_apply_matches_oracle():
     T.close()
 
 
+@pytest.mark.parametrize("N,ncol", [((32, 64), 16), ((40, 50), 8), ((256, 168), 5), ((60, 140), 2),
+                                    ((33, 32), 3), ((64, 37), 4)])
+def test_gram_apply_fused_and_library_transforms(N, ncol):
+    """Padded sizes of the fused passes (powers of two and others, vectors of 16,
+    8, 2 and 1 columns, one wide and one narrow dimension) and sizes that stay on
+    the FFT library."""
+    import torch
+    rng = np.random.default_rng(N[0])
+    K = (2 * N[0], 2 * N[1])
+    oms = [wl.vd_random(900, rng), wl.vd_random(350, rng)]
+    moff = np.concatenate([[0], np.cumsum([len(o) for o in oms])])
+    G = mb.NufftPlan(np.concatenate(oms), N, (6, 6), K, Ld=1024, ncol=1, slice_moff=moff)
+    T = ms.Gram(G, ncol=ncol)
+    x = rng.standard_normal((2, N[1], N[0], ncol)) + 1j * rng.standard_normal((2, N[1], N[0], ncol))
+    y = T.apply(torch.from_numpy(x.astype(np.complex64)).cuda()).cpu().numpy()
+    for s, o in enumerate(oms):
+        H = tr.gram_kernel(o, N, K)
+        for c in range(ncol):
+            assert rel_l2(y[s, :, :, c], tr.gram_apply(H, x[s, :, :, c].T).T) <= 1e-5, (s, c)
+    T.close()
+
+
 def _sense_batch(seed, N=32, K=64, C=4, spokes=(22, 16)):
     import torch
     rng = np.random.default_rng(seed)
