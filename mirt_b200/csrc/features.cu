@@ -57,56 +57,113 @@ __global__ void feat_keys_kernel(const double *__restrict__ om, long long M,
   keys[m] = (uint32_t)((long long)s * g.ncells + c);
 }
 
-__global__ void feat_gather_kernel(const double2 *__restrict__ t, const int *__restrict__ perm,
-                                   long long M, double2 *__restrict__ ts) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p < M) ts[p] = t[perm[p]];
-}
-
-// one thread per sorted position
-__global__ void feat_hist_kernel(const double *__restrict__ om, const double2 *__restrict__ ts,
-                                 const int *__restrict__ perm, const int *__restrict__ bin_start,
-                                 const int *__restrict__ slice_of, long long M, FeatGeom g,
-                                 float *__restrict__ feat) {
+// what the histogram needs of each sorted position: coordinates, {first bin of its
+// slice, hash cell, sample} and the two polar features
+__global__ void feat_gather_kernel(const double *__restrict__ om, const double2 *__restrict__ t,
+                                   const int *__restrict__ perm, const int *__restrict__ slice_of,
+                                   long long M, FeatGeom g, double2 *__restrict__ ts,
+                                   int4 *__restrict__ info, float2 *__restrict__ polar) {
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= M) return;
   const int m = perm[p];
-  const double2 tp = ts[p];
-  const int s = slice_of ? slice_of[m] : 0;
-  const int c0 = cell_of(tp.x, g.K[0], g.nc[0]);
-  const int c1 = cell_of(tp.y, g.K[1], g.nc[1]);
-  int h[16];
+  const double2 tp = t[m];
+  const double w0 = om[m], w1 = om[M + m];
+  ts[p] = tp;
+  info[p] = make_int4((slice_of ? slice_of[m] : 0) * g.ncells, cell_of(tp.x, g.K[0], g.nc[0]),
+                      cell_of(tp.y, g.K[1], g.nc[1]), m);
+  polar[p] = make_float2((float)(sqrt(w0 * w0 + w1 * w1) / M_PI), (float)(atan2(w1, w0) / M_PI));
+}
+
+// Eight lanes per sorted position over the candidates of its 3 x 3 hash cells (three
+// runs of the sort order, walked as one), four positions a warp with their histograms
+// in shared memory; the warp writes their rows.  The bin of a distance is its FP32
+// square root, put right by FP64 comparisons with the exact edges (b / 8)^2, so the
+// counts stay those of the FP64 comparisons.  Bound by the chain of dependent loads
+// and FP64 operations of the short walks (27 candidates on average, 600 at the
+// trajectory's centre; 8 slices of 101 spokes x 512): 204 us with one thread a sample
+// and 15 comparisons a candidate, 87 us so.
+// floor(8 sqrt(d2)) or one off it, 0 <= d2 < 4: the double's bits cut to FP32 (below
+// 2^-126 to zero), an approximate root and a rounding by a large constant, as the
+// conversions between FP64, FP32 and integers run at a fraction of the rate
+__device__ __forceinline__ int bin_guess(double d2) {
+  const int hi = max(__double2hiint(d2) - 0x38000000, 0);
+  const float f = __uint_as_float(__funnelshift_l(__double2loint(d2), hi, 3));
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(f));
+  const int b = __float_as_int(fmaf(8.f, r, 8388607.5f)) & 31;
+  return b > 15 ? (b > 16 ? 0 : 15) : b;
+}
+
+constexpr int kFeatLanes = 8, kFeatBlock = 256, kFeatPos = 32 / kFeatLanes;
+
+__global__ void __launch_bounds__(kFeatBlock)
+    feat_hist_kernel(const double2 *__restrict__ ts, const int4 *__restrict__ info,
+                     const float2 *__restrict__ polar, const int *__restrict__ bin_start,
+                     long long M, FeatGeom g, float *__restrict__ feat) {
+  __shared__ int hist[kFeatBlock / 32][16 * kFeatPos];
+  __shared__ double edge[17];  // exact squared bin edges
+  const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  const int pos = ln / kFeatLanes, lane = ln % kFeatLanes;
+  int *h = hist[warp];
+  if (threadIdx.x < 17) edge[threadIdx.x] = (threadIdx.x * 0.125) * (threadIdx.x * 0.125);
+  h[ln] = 0;
+  h[32 + ln] = 0;
+  __syncthreads();
+  const long long p0 = ((long long)blockIdx.x * (kFeatBlock / 32) + warp) * kFeatPos;
+  if (p0 >= M) return;
+  const int np = (int)min((long long)kFeatPos, M - p0);
+  const long long p = p0 + pos;
+  int m = 0;
+  if (pos < np) {
+    const int4 in = info[p];
+    const double2 tp = ts[p];
+    m = in.w;
+    const int *bs = bin_start + in.x;
+    const int ca = max(in.y - 1, 0), cb = min(in.y + 1, g.nc[0] - 1);
+    int first[3], n[3];
 #pragma unroll
-  for (int b = 0; b < 16; b++) h[b] = 0;
-  const long long sbase = (long long)s * g.ncells;
-  for (int d1 = -1; d1 <= 1; d1++) {
-    const int cc1 = c1 + d1;
-    if (cc1 < 0 || cc1 >= g.nc[1]) continue;
-    // the three cells of this row are contiguous in the sort order
-    const int ca = max(c0 - 1, 0), cb = min(c0 + 1, g.nc[0] - 1);
-    const long long q0 = bin_start[sbase + (long long)cc1 * g.nc[0] + ca];
-    const long long q1 = bin_start[sbase + (long long)cc1 * g.nc[0] + cb + 1];
-    for (long long q = q0; q < q1; q++) {
-      if (q == p) continue;
+    for (int r = 0; r < 3; r++) {
+      // the three cells of a row are contiguous in the sort order
+      const int cc1 = in.z + r - 1;
+      const bool ok = cc1 >= 0 && cc1 < g.nc[1];
+      const int *b = bs + (ok ? (long long)cc1 * g.nc[0] : 0);
+      first[r] = ok ? b[ca] : 0;
+      n[r] = ok ? b[cb + 1] - first[r] : 0;
+    }
+    const int n01 = n[0] + n[1], total = n01 + n[2];
+    const int a1 = first[1] - n[0], a2 = first[2] - n01;
+    for (int i = lane; i < total; i += kFeatLanes) {
+      const int q = i + (i < n[0] ? first[0] : i < n01 ? a1 : a2);
       const double2 tq = ts[q];
       const double dx = __dsub_rn(tq.x, tp.x), dy = __dsub_rn(tq.y, tp.y);
       const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-      if (d2 < 4.0) {
+      if (d2 < 4.0 && q != p) {
         // bin b: (b/8)^2 <= d2 < ((b+1)/8)^2, edges exact in binary
-        int b = 0;
-#pragma unroll
-        for (int e = 1; e < 16; e++) b += d2 >= (e * 0.125) * (e * 0.125) ? 1 : 0;
-#pragma unroll
-        for (int e = 0; e < 16; e++) h[e] += (e == b) ? 1 : 0;
+        int b = bin_guess(d2);
+        b += (d2 >= edge[b + 1]) - (d2 < edge[b]);
+        atomicAdd(h + b * kFeatPos + pos, 1);
       }
     }
   }
-  const double w0 = om[m], w1 = om[M + m];
-  float *f = feat + (long long)m * MIRT_DCF_NFEAT;
-  f[0] = (float)(sqrt(w0 * w0 + w1 * w1) / M_PI);
-  f[1] = (float)(atan2(w1, w0) / M_PI);
+  __syncwarp();
 #pragma unroll
-  for (int b = 0; b < 16; b++) f[2 + b] = log1pf((float)h[b]);
+  for (int e = 0; e < 16 * kFeatPos; e += 32)
+    h[e + ln] = __float_as_int(log1pf((float)h[e + ln]));
+  __syncwarp();
+  for (int e = ln; e < ((np * MIRT_DCF_NFEAT + 31) & ~31); e += 32) {
+    const int r = e / MIRT_DCF_NFEAT, j = e - r * MIRT_DCF_NFEAT;
+    const int mr = __shfl_sync(0xffffffffu, m, (r < np ? r : 0) * kFeatLanes);
+    if (r < np) {
+      float v;
+      if (j < 2) {
+        const float2 pl = polar[p0 + r];
+        v = j ? pl.y : pl.x;
+      } else {
+        v = __int_as_float(h[(j - 2) * kFeatPos + r]);
+      }
+      feat[(long long)mr * MIRT_DCF_NFEAT + j] = v;
+    }
+  }
 }
 
 }  // namespace
@@ -138,7 +195,7 @@ extern "C" int mirt_dcf_features(const double *om, int64_t M, const int64_t *sli
   }
   if (M == 0) return MIRT_OK;
   cudaStream_t st = as_stream(stream);
-  DMem dmoff, slice, t, ts, keys, perm, bstart, tmp;
+  DMem dmoff, slice, t, ts, keys, perm, bstart, tmp, info, polar;
   const int *slice_of = nullptr;
   if (nslice > 1) {
     FCK(dmoff.alloc((nslice + 1) * sizeof(long long)));
@@ -150,6 +207,8 @@ extern "C" int mirt_dcf_features(const double *om, int64_t M, const int64_t *sli
   }
   FCK(t.alloc(M * sizeof(double2)));
   FCK(ts.alloc(M * sizeof(double2)));
+  FCK(info.alloc(M * sizeof(int4)));
+  FCK(polar.alloc(M * sizeof(float2)));
   FCK(keys.alloc(M * sizeof(uint32_t)));
   FCK(perm.alloc(M * sizeof(int)));
   FCK(bstart.alloc((nbins + 1) * sizeof(int)));
@@ -159,10 +218,12 @@ extern "C" int mirt_dcf_features(const double *om, int64_t M, const int64_t *sli
   FCK(cudaGetLastError());
   FCK(radix_sort_bins(keys.as<uint32_t>(), M, (int)nbins, tmp.p, perm.as<int>(), bstart.as<int>(),
                       st));
-  feat_gather_kernel<<<blk, 256, 0, st>>>(t.as<double2>(), perm.as<int>(), M, ts.as<double2>());
+  feat_gather_kernel<<<blk, 256, 0, st>>>(om, t.as<double2>(), perm.as<int>(), slice_of, M, g,
+                                          ts.as<double2>(), info.as<int4>(), polar.as<float2>());
   FCK(cudaGetLastError());
-  feat_hist_kernel<<<blk, 256, 0, st>>>(om, ts.as<double2>(), perm.as<int>(), bstart.as<int>(),
-                                        slice_of, M, g, feat);
+  const long long per = kFeatBlock / 32 * kFeatPos;
+  feat_hist_kernel<<<(unsigned)((M + per - 1) / per), kFeatBlock, 0, st>>>(
+      ts.as<double2>(), info.as<int4>(), polar.as<float2>(), bstart.as<int>(), M, g, feat);
   FCK(cudaGetLastError());
   FCK(cudaStreamSynchronize(st));
   return MIRT_OK;

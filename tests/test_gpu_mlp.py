@@ -41,6 +41,24 @@ def test_features_match_oracle():
     assert np.max(np.abs(f[:, 2:] - ref[:, 2:])) <= 2e-6
 
 
+@pytest.mark.parametrize("n0,n1,K", [(1, 0, (2, 2)), (2, 3, (3, 64)), (33, 31, (16, 7)),
+                                     (1024, 1, (64, 64)), (700, 1349, (9, 300))])
+def test_features_at_bin_edges_and_chunk_edges(n0, n1, K):
+    """Points on a lattice of 1/8 cell (distances at the bin edges, duplicates, cells
+    at the rim) plus points next to it, around warps and sort chunks: exact counts."""
+    rng = np.random.default_rng(n0)
+    n = n0 + n1
+    half = [min(k / 2, 3.0) for k in K]
+    t = np.stack([rng.integers(-int(8 * h), int(8 * h) + 1, n) / 8.0 for h in half], 1)
+    t[::3] += rng.uniform(-1e-15, 1e-15, t[::3].shape)
+    om = t * (2 * np.pi / np.array(K))
+    moff = np.array([0, n0, n])
+    f = mb.dcf_features(_dev(om), K, moff).cpu().numpy()
+    ref, hist = mlp_ref.features(om, K, moff)
+    assert np.array_equal(np.rint(np.expm1(f[:, 2:].astype(np.float64))), hist)
+    assert np.max(np.abs(f - ref)) <= 2e-6
+
+
 def test_forward_and_gradient_match_oracle():
     import torch
     rng = np.random.default_rng(5)
