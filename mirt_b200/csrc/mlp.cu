@@ -9,17 +9,17 @@
 // The forward and backward passes use the BF16 rounding (nearest even) of the
 // master weights, refreshed after every Adam update.
 //
-// Kernel layout.  A CTA of 256 threads takes 64 samples: the weights (as FP32)
-// and the 64 samples' activations and back-propagated errors live in shared
-// memory (rows padded to 65 floats, so a warp's 32 neurons hit 32 banks while
-// a sample row is a broadcast).  Thread t owns neuron i = t mod 64 of samples
-// t / 64 + 4k, k < 16, in every layer; for the weight gradients it owns entries
-// (i, t / 64 + 4k).  Each CTA writes its partial gradient; one reduction
-// kernel sums the partials in CTA order (deterministic) and applies Adam.
+// Gradient: mlp_grad_kernel, persistent over the batch in register tiles on the FP32
+// pipes; a reduction kernel sums the partial gradients in a fixed order
+// (deterministic) and applies Adam.  FP32 inference (mlp_infer_kernel): a CTA of 256
+// threads takes 64 samples with the weights (as FP32) and the activations in shared
+// memory (rows padded to 65 floats); thread t owns neuron t mod 64 of samples
+// t / 64 + 4k, k < 16, in every layer.
 #include "../../include/mirt_b200.h"
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <new>
@@ -66,10 +66,6 @@ struct Acts {
   float X[NS][LDI];
   float H1[NS][LD], H2[NS][LD], H3[NS][LD];
   float out[NS], dout[NS];
-};
-
-struct Errs {
-  float D1[NS][LD], D2[NS][LD], D3[NS][LD];
 };
 
 __device__ void load_weights(Weights &w, const __nv_bfloat16 *__restrict__ p) {
@@ -132,162 +128,414 @@ struct GradArgs {
   const float *x;        // [n][NIN]
   const float *y;        // [n]
   long long n;
-  const long long *idx;  // explicit sample list [batch] (or null: hashed draw)
   int batch;
   unsigned long long seed;
-  const int *step;       // device step counter (hashed draw)
+  const int *step;       // device step counter of the hashed draw (null: samples 0, 1, ...)
   const __nv_bfloat16 *wb;
-  float *part;           // [nblk][NPARAM]
-  float *loss_part;      // [nblk]
+  float *part;           // [nunit][NPARAM]
+  float *loss_part;      // [nunit]
 };
 
-// one CTA: forward + backward of up to 64 samples, partial gradient of the
-// mean squared error over the whole batch
-__global__ void __launch_bounds__(NT) mlp_grad_kernel(GradArgs g) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  Weights &w = *reinterpret_cast<Weights *>(smem);
-  Acts &a = *reinterpret_cast<Acts *>(smem + sizeof(Weights));
-  Errs &d = *reinterpret_cast<Errs *>(smem + sizeof(Weights) + sizeof(Acts));
-  load_weights(w, g.wb);
-  const int b0 = blockIdx.x * NS;
-  const int cnt = min(NS, g.batch - b0);
-  const int st = g.step ? *g.step : 0;
-  __shared__ long long src[NS];
-  __shared__ float yv[NS];
-  if (threadIdx.x < NS) {
-    long long m = 0;
-    if (threadIdx.x < cnt) {
-      const long long r = b0 + threadIdx.x;
-      m = g.idx ? g.idx[r]
-                : (long long)(mix64(g.seed ^ ((unsigned long long)st << 32) ^ (unsigned long long)r) %
-                              (unsigned long long)g.n);
+// ---- gradient -------------------------------------------------------------------
+// Forward and backward of the mean squared error.  A CTA is two units of 128
+// threads; a unit takes 64 samples at a time, and the weight gradients of all its
+// samples stay in its registers.  Activations lie in shared memory as
+// [neuron][sample], so that
+//  * a layer is, per input neuron k, 8 samples of row k (two 16-byte loads) times 4
+//    weights of row k (one load): a tile of 8 x 4 outputs a thread;
+//  * a weight gradient is, per 4 samples, 8 rows of errors times 4 rows of inputs:
+//    12 loads and 128 products, again 8 x 4 outputs a thread;
+// both in packed FP32 pairs of samples.  The weights are there in both orders.
+// Bound by the FP32 pipes and their operand loads (1.8e9 multiply-adds at 65,536
+// samples, 49 us at the pipes' rate; 8 warps an SM): 101 us, against 302 us with one weight and one
+// broadcast activation loaded for every product.
+constexpr int GU = 128;      // threads of a unit
+constexpr int GP = NS + 4;   // row pitch (floats): 8 rows' 16-byte loads hit all banks
+constexpr int kGradSMs = 148;
+
+typedef unsigned long long f32x2;  // two packed FP32
+
+__device__ __forceinline__ void fma2(f32x2 &d, f32x2 a, f32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+struct GradUnit {  // shared memory of a unit
+  float X[NIN][GP];
+  float H1[HID][GP], H2[HID][GP], D[HID][GP];
+  float red[4][NS];  // output unit: partial sums of the four warps
+  float y[NS];
+};
+struct GradSmem {
+  float W1t[NIN][HID];             // [input][output]
+  float W2t[HID][GP], W3t[HID][GP];
+  float W2[HID][GP], W3[HID][GP];  // [output][input]
+  float b1[HID], b2[HID], b3[HID], W4[HID];
+  float b4, pad[3];
+  GradUnit u[2];
+};
+
+__device__ __forceinline__ void unit_sync(int unit) {
+  asm volatile("bar.sync %0, %1;" ::"r"(unit + 1), "r"(GU) : "memory");
+}
+
+// acc[c][q] += sum_k W[k][i0 + c] A[k][samples of q]; q: pairs at s0, s0 + 2, s0 + 32, s0 + 34
+template <int K>
+__device__ __forceinline__ void tile_layer(const float *W, int ldw, const float *A, int i0, int s0,
+                                           f32x2 (&acc)[4][4]) {
+#pragma unroll 8
+  for (int k = 0; k < K; k++) {
+    const float4 w = *reinterpret_cast<const float4 *>(W + k * ldw + i0);
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(A + k * GP + s0);
+    const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(A + k * GP + s0 + 32);
+    const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const f32x2 ww = pack2(wv[c], wv[c]);
+      fma2(acc[c][0], ww, a0.x);
+      fma2(acc[c][1], ww, a0.y);
+      fma2(acc[c][2], ww, a1.x);
+      fma2(acc[c][3], ww, a1.y);
     }
-    src[threadIdx.x] = m;
-    yv[threadIdx.x] = threadIdx.x < cnt ? g.y[m] : 0.f;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < NS * NIN; e += NT) {
-    const int s = e / NIN, j = e % NIN;
-    a.X[s][j] = s < cnt ? g.x[src[s] * NIN + j] : 0.f;
-  }
-  __syncthreads();
-  forward(w, a);
-  const float inv_b = 1.f / (float)g.batch;
-  if (threadIdx.x < NS) {
-    const float r = threadIdx.x < cnt ? a.out[threadIdx.x] - yv[threadIdx.x] : 0.f;
-    a.dout[threadIdx.x] = 2.f * r * inv_b;
-    a.out[threadIdx.x] = r * r;  // squared residual, summed below
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float l = 0.f;
-    for (int s = 0; s < NS; s++) l += a.out[s];
-    g.loss_part[blockIdx.x] = l * inv_b;
-  }
-  const int i = threadIdx.x & (HID - 1), s0 = threadIdx.x >> 6;
-  // back-propagated errors
-#pragma unroll
-  for (int k = 0; k < KS; k++) {
-    const int s = s0 + 4 * k;
-    d.D3[s][i] = a.H3[s][i] > 0.f ? w.W4[i] * a.dout[s] : 0.f;
-  }
-  __syncthreads();
-  {
-    float acc[KS];
-#pragma unroll
-    for (int k = 0; k < KS; k++) acc[k] = 0.f;
-    for (int kk = 0; kk < HID; kk++) {
-      const float wk = w.W3[kk][i];
-#pragma unroll
-      for (int k = 0; k < KS; k++) acc[k] = fmaf(wk, d.D3[s0 + 4 * k][kk], acc[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < KS; k++) {
-      const int s = s0 + 4 * k;
-      d.D2[s][i] = a.H2[s][i] > 0.f ? acc[k] : 0.f;
-    }
-  }
-  __syncthreads();
-  {
-    float acc[KS];
-#pragma unroll
-    for (int k = 0; k < KS; k++) acc[k] = 0.f;
-    for (int kk = 0; kk < HID; kk++) {
-      const float wk = w.W2[kk][i];
-#pragma unroll
-      for (int k = 0; k < KS; k++) acc[k] = fmaf(wk, d.D2[s0 + 4 * k][kk], acc[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < KS; k++) {
-      const int s = s0 + 4 * k;
-      d.D1[s][i] = a.H1[s][i] > 0.f ? acc[k] : 0.f;
-    }
-  }
-  __syncthreads();
-  // partial weight gradients: entry (i, j) with j = s0 + 4k
-  float *part = g.part + (size_t)blockIdx.x * NPARAM;
-  auto outer = [&](const float (*Dl)[LD], const float *Hp, int ldh, int nj, int pw) {
-    float acc[KS];
-#pragma unroll
-    for (int k = 0; k < KS; k++) acc[k] = 0.f;
-    for (int s = 0; s < NS; s++) {
-      const float dv = Dl[s][i];
-      const float *hrow = Hp + s * ldh;
-#pragma unroll
-      for (int k = 0; k < KS; k++) {
-        const int j = s0 + 4 * k;
-        if (j < nj) acc[k] = fmaf(dv, hrow[j], acc[k]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < KS; k++) {
-      const int j = s0 + 4 * k;
-      if (j < nj) part[pw + i * nj + j] = acc[k];
-    }
-  };
-  outer(d.D3, &a.H2[0][0], LD, HID, P_W3);
-  outer(d.D2, &a.H1[0][0], LD, HID, P_W2);
-  outer(d.D1, &a.X[0][0], LDI, NIN, P_W1);
-  if (threadIdx.x < HID) {
-    float gb1 = 0.f, gb2 = 0.f, gb3 = 0.f, gw4 = 0.f;
-    for (int s = 0; s < NS; s++) {
-      gb1 += d.D1[s][i];
-      gb2 += d.D2[s][i];
-      gb3 += d.D3[s][i];
-      gw4 += a.dout[s] * a.H3[s][i];
-    }
-    part[P_B1 + i] = gb1;
-    part[P_B2 + i] = gb2;
-    part[P_B3 + i] = gb3;
-    part[P_W4 + i] = gw4;
-  }
-  if (threadIdx.x == 0) {
-    float gb4 = 0.f;
-    for (int s = 0; s < NS; s++) gb4 += a.dout[s];
-    part[P_B4] = gb4;
   }
 }
+
+// the tile's 4 x 8 values, row c = neuron i0 + c, v[c][0..3] at s0, v[c][4..7] at s0 + 32
+__device__ __forceinline__ void tile_values(const f32x2 (&acc)[4][4], float (&v)[4][8]) {
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float2 f = unpack2(acc[c][q]);
+      v[c][2 * q] = f.x;
+      v[c][2 * q + 1] = f.y;
+    }
+}
+
+__device__ __forceinline__ void tile_store(float *H, int i0, int s0, const float (&v)[4][8]) {
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    float *r = H + (i0 + c) * GP + s0;
+    *reinterpret_cast<float4 *>(r) = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
+    *reinterpret_cast<float4 *>(r + 32) = make_float4(v[c][4], v[c][5], v[c][6], v[c][7]);
+  }
+}
+
+// H = relu(b + W A) of the unit's 64 samples; v keeps the thread's tile
+template <int K>
+__device__ __forceinline__ void tile_relu(const float *W, int ldw, const float *b, const float *A,
+                                          int i0, int s0, float (&v)[4][8]) {
+  f32x2 acc[4][4];
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc[c][q] = pack2(b[i0 + c], b[i0 + c]);
+  tile_layer<K>(W, ldw, A, i0, s0, acc);
+  tile_values(acc, v);
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int e = 0; e < 8; e++) v[c][e] = fmaxf(v[c][e], 0.f);
+}
+
+// errors of the layer below: v = (H > 0) W^T D, and their sums over the tile's samples
+__device__ __forceinline__ void tile_back(const float *W, const float *D, const float *H, int i0,
+                                          int s0, float (&v)[4][8], float (&gb)[4]) {
+  f32x2 acc[4][4];
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc[c][q] = 0ull;
+  tile_layer<HID>(W, GP, D, i0, s0, acc);
+  tile_values(acc, v);
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const float *r = H + (i0 + c) * GP + s0;
+    const float4 h0 = *reinterpret_cast<const float4 *>(r);
+    const float4 h1 = *reinterpret_cast<const float4 *>(r + 32);
+    const float h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    float sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      v[c][e] = h[e] > 0.f ? v[c][e] : 0.f;
+      sum += v[c][e];
+    }
+    gb[c] += sum;
+  }
+}
+
+// g[r][c] += sum_s D[ig + 8r][s] H[jg + 16c][s] over the unit's 64 samples
+template <int NC>
+__device__ __forceinline__ void tile_outer(const float *D, const float *H, int ig, int jg,
+                                           float (&g)[8][NC]) {
+  f32x2 acc[8][NC];
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c < NC; c++) acc[r][c] = 0ull;
+#pragma unroll 2
+  for (int s = 0; s < NS; s += 4) {
+    ulonglong2 h[NC];
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+      h[c] = *reinterpret_cast<const ulonglong2 *>(H + (jg + 16 * c) * GP + s);
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      const ulonglong2 d = *reinterpret_cast<const ulonglong2 *>(D + (ig + 8 * r) * GP + s);
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        fma2(acc[r][c], d.x, h[c].x);
+        fma2(acc[r][c], d.y, h[c].y);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      const float2 f = unpack2(acc[r][c]);
+      g[r][c] += f.x + f.y;
+    }
+}
+
+// unit u (of 2 gridDim.x) takes samples 64 u .. 64 u + 63, then 128 gridDim.x further
+__global__ void __launch_bounds__(2 * GU, 1) mlp_grad_kernel(GradArgs g) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  GradSmem &S = *reinterpret_cast<GradSmem *>(smem);
+  for (int e = threadIdx.x; e < HID * NIN; e += 2 * GU)
+    S.W1t[e % NIN][e / NIN] = __bfloat162float(g.wb[P_W1 + e]);
+  for (int e = threadIdx.x; e < HID * HID; e += 2 * GU) {
+    const float w2 = __bfloat162float(g.wb[P_W2 + e]), w3 = __bfloat162float(g.wb[P_W3 + e]);
+    S.W2[e / HID][e % HID] = w2;
+    S.W2t[e % HID][e / HID] = w2;
+    S.W3[e / HID][e % HID] = w3;
+    S.W3t[e % HID][e / HID] = w3;
+  }
+  if (threadIdx.x < HID) {
+    const int e = threadIdx.x;
+    S.b1[e] = __bfloat162float(g.wb[P_B1 + e]);
+    S.b2[e] = __bfloat162float(g.wb[P_B2 + e]);
+    S.b3[e] = __bfloat162float(g.wb[P_B3 + e]);
+    S.W4[e] = __bfloat162float(g.wb[P_W4 + e]);
+    if (e == 0) S.b4 = __bfloat162float(g.wb[P_B4]);
+  }
+  __syncthreads();
+  const int half = threadIdx.x / GU, t = threadIdx.x % GU;
+  const int warp = t >> 5, lane = t & 31;
+  const int unit = half * gridDim.x + blockIdx.x;
+  const int nset = (g.batch + NS - 1) / NS;
+  if (unit >= nset) return;  // no barrier of the whole CTA from here on
+  GradUnit &U = S.u[half];
+  const int lo = lane & 7, hi = (lane >> 3) + 4 * warp;  // 8 x 16 threads of a unit
+  const int s0 = 4 * lo, i0 = 4 * hi;                    // layers: 8 samples, 4 neurons
+  const int st = g.step ? *g.step : 0;
+  const float inv_b = 1.f / (float)g.batch;
+  float gw3[8][4], gw2[8][4], gw1[8][1], gw1b = 0.f;  // entries (lo + 8r, hi + 16c)
+  float gb1[4], gb2[4], gb3[4], gw4[4], gb4 = 0.f, loss = 0.f;
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+    gw1[r][0] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; c++) gw3[r][c] = gw2[r][c] = 0.f;
+  }
+#pragma unroll
+  for (int c = 0; c < 4; c++) gb1[c] = gb2[c] = gb3[c] = gw4[c] = 0.f;
+
+  // this set's inputs, loaded ahead: thread t takes elements t + 128 k of [sample][input]
+  constexpr int NX = NS * NIN / GU;
+  static_assert(NX * GU == NS * NIN, "inputs of a set");
+  float xv[NX], yv = 0.f;
+  auto fetch = [&](int set) {
+    const int b0 = set * NS, cnt = min(NS, g.batch - b0);
+    auto row = [&](int s) -> long long {
+      const long long r = b0 + s;
+      return g.step ? (long long)(mix64(g.seed ^ ((unsigned long long)st << 32) ^
+                                        (unsigned long long)r) % (unsigned long long)g.n)
+                    : r;
+    };
+#pragma unroll
+    for (int k = 0; k < NX; k++) {
+      const int e = t + k * GU, s = e / NIN, j = e - s * NIN;
+      xv[k] = s < cnt ? g.x[row(s) * NIN + j] : 0.f;
+    }
+    if (t < cnt) yv = g.y[row(t)];
+  };
+  fetch(unit);
+#pragma unroll 1
+  for (int set = unit; set < nset; set += 2 * gridDim.x) {
+    const int cnt = min(NS, g.batch - set * NS);
+#pragma unroll
+    for (int k = 0; k < NX; k++) {
+      const int e = t + k * GU, s = e / NIN, j = e - s * NIN;
+      U.X[j][s] = xv[k];
+    }
+    if (t < NS) U.y[t] = yv;
+    unit_sync(half);
+    float v[4][8];
+    tile_relu<NIN>(&S.W1t[0][0], HID, S.b1, &U.X[0][0], i0, s0, v);
+    tile_store(&U.H1[0][0], i0, s0, v);
+    unit_sync(half);
+    tile_relu<HID>(&S.W2t[0][0], GP, S.b2, &U.H1[0][0], i0, s0, v);
+    tile_store(&U.H2[0][0], i0, s0, v);
+    unit_sync(half);
+    tile_relu<HID>(&S.W3t[0][0], GP, S.b3, &U.H2[0][0], i0, s0, v);
+    // output unit: the tile's 4 neurons, the warp's 16, then the four warps'
+    {
+      float o[8];
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        o[e] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) o[e] = fmaf(S.W4[i0 + c], v[c][e], o[e]);
+        o[e] += __shfl_xor_sync(0xffffffffu, o[e], 8);
+        o[e] += __shfl_xor_sync(0xffffffffu, o[e], 16);
+      }
+      if (lane < 8) {
+        *reinterpret_cast<float4 *>(&U.red[warp][s0]) = make_float4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<float4 *>(&U.red[warp][s0 + 32]) = make_float4(o[4], o[5], o[6], o[7]);
+      }
+    }
+    unit_sync(half);
+    {
+      float dout[8];
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        const int s = s0 + (e & 3) + (e >> 2) * 32;
+        const float o = S.b4 + ((U.red[0][s] + U.red[1][s]) + (U.red[2][s] + U.red[3][s]));
+        const float r = s < cnt ? o - U.y[s] : 0.f;
+        dout[e] = 2.f * r * inv_b;
+        if (hi == 0) {
+          loss = fmaf(r, r, loss);
+          gb4 += dout[e];
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const float w4 = S.W4[i0 + c];
+        float a = 0.f, b = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+          a = fmaf(dout[e], v[c][e], a);
+          v[c][e] = v[c][e] > 0.f ? w4 * dout[e] : 0.f;
+          b += v[c][e];
+        }
+        gw4[c] += a;
+        gb3[c] += b;
+      }
+    }
+    tile_store(&U.D[0][0], i0, s0, v);
+    unit_sync(half);
+    if (set + 2 * gridDim.x < nset) fetch(set + 2 * gridDim.x);
+    tile_outer(&U.D[0][0], &U.H2[0][0], lo, hi, gw3);
+    tile_back(&S.W3[0][0], &U.D[0][0], &U.H2[0][0], i0, s0, v, gb2);
+    unit_sync(half);
+    tile_store(&U.H2[0][0], i0, s0, v);  // the errors of layer 2 in place of its outputs
+    unit_sync(half);
+    tile_outer(&U.H2[0][0], &U.H1[0][0], lo, hi, gw2);
+    tile_back(&S.W2[0][0], &U.H2[0][0], &U.H1[0][0], i0, s0, v, gb1);
+    tile_store(&U.D[0][0], i0, s0, v);
+    unit_sync(half);
+    // first layer: inputs 0..15 as above, the last two one entry a thread
+    tile_outer(&U.D[0][0], &U.X[0][0], lo, hi, gw1);
+    {
+      const float *d = U.D[t % HID], *x = U.X[16 + t / HID];
+      float a = 0.f;
+#pragma unroll 4
+      for (int s = 0; s < NS; s += 4) {
+        const float4 dv = *reinterpret_cast<const float4 *>(d + s);
+        const float4 xv = *reinterpret_cast<const float4 *>(x + s);
+        a = fmaf(dv.x, xv.x, fmaf(dv.y, xv.y, fmaf(dv.z, xv.z, fmaf(dv.w, xv.w, a))));
+      }
+      gw1b += a;
+    }
+    unit_sync(half);
+  }
+  static_assert(NIN == 18 && GU == 2 * HID, "first layer's gradient tile");
+  float *part = g.part + (size_t)unit * NPARAM;
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+    const int i = lo + 8 * r;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      part[P_W3 + i * HID + hi + 16 * c] = gw3[r][c];
+      part[P_W2 + i * HID + hi + 16 * c] = gw2[r][c];
+    }
+    part[P_W1 + i * NIN + hi] = gw1[r][0];
+  }
+  part[P_W1 + (t % HID) * NIN + 16 + t / HID] = gw1b;
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      gb1[c] += __shfl_xor_sync(0xffffffffu, gb1[c], h);
+      gb2[c] += __shfl_xor_sync(0xffffffffu, gb2[c], h);
+      gb3[c] += __shfl_xor_sync(0xffffffffu, gb3[c], h);
+      gw4[c] += __shfl_xor_sync(0xffffffffu, gw4[c], h);
+    }
+    gb4 += __shfl_xor_sync(0xffffffffu, gb4, h);
+    loss += __shfl_xor_sync(0xffffffffu, loss, h);
+  }
+  if (lo == 0) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      part[P_B1 + i0 + c] = gb1[c];
+      part[P_B2 + i0 + c] = gb2[c];
+      part[P_B3 + i0 + c] = gb3[c];
+      part[P_W4 + i0 + c] = gw4[c];
+    }
+  }
+  if (t == 0) {
+    part[P_B4] = gb4;
+    g.loss_part[unit] = loss * inv_b;
+  }
+}
+
+// CTAs of a batch, and the units that write a partial gradient
+int grad_grid(int batch) { return std::min((batch + NS - 1) / NS, kGradSMs); }
+int grad_units(int batch) { return std::min((batch + NS - 1) / NS, 2 * kGradSMs); }
 
 struct AdamArgs {
   const float *part;
   const float *loss_part;
-  int nblk;
+  int nunit;
   float *master, *m, *v;
   __nv_bfloat16 *wb;
   float *grad_out;  // optional: the summed gradient
   float *loss_hist;
-  int *step;
+  const int *step;  // null: step 0
   float lr, beta1, beta2, eps;
   int apply;        // 0: only sum the gradient (and loss)
 };
 
-// sum the partial gradients in CTA order; Adam on the FP32 master weights
-__global__ void mlp_adam_kernel(AdamArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = *a.step + 1;
+// Sum the partial gradients in a fixed order, 32 parameters a block and every eighth
+// partial a thread, all loads coalesced (one thread a parameter over 1,024 partials:
+// 41 us, bound by the latency of its loads; 5.8 us over 296); Adam on the FP32 master
+// weights.
+constexpr int kAdamP = 32, kAdamK = 8;
+__global__ void __launch_bounds__(kAdamP *kAdamK) mlp_adam_kernel(AdamArgs a) {
+  __shared__ float sum[kAdamK][kAdamP];
+  const int c = threadIdx.x % kAdamP, k = threadIdx.x / kAdamP;
+  const int p = blockIdx.x * kAdamP + c;
+  const int t = (a.step ? *a.step : 0) + 1;
+  float part = 0.f;
   if (p < NPARAM) {
+#pragma unroll 8
+    for (int b = k; b < a.nunit; b += kAdamK) part += a.part[(size_t)b * NPARAM + p];
+  }
+  sum[k][c] = part;
+  __syncthreads();
+  if (k == 0 && p < NPARAM) {
     float g = 0.f;
-    for (int b = 0; b < a.nblk; b++) g += a.part[(size_t)b * NPARAM + p];
+    for (int i = 0; i < kAdamK; i++) g += sum[i][c];
     if (a.grad_out) a.grad_out[p] = g;
     if (a.apply) {
       const float m = a.beta1 * a.m[p] + (1.f - a.beta1) * g;
@@ -301,12 +549,14 @@ __global__ void mlp_adam_kernel(AdamArgs a) {
       a.wb[p] = __float2bfloat16_rn(th);
     }
   }
-  if (p == 0) {
+  if (blockIdx.x == 0 && k == 1) {
     float l = 0.f;
-    for (int b = 0; b < a.nblk; b++) l += a.loss_part[b];
-    if (a.loss_hist) a.loss_hist[t - 1] = l;
+    for (int b = c; b < a.nunit; b += 32) l += a.loss_part[b];
+    for (int h = 16; h > 0; h >>= 1) l += __shfl_xor_sync(0xffffffffu, l, h);
+    if (c == 0 && a.loss_hist) a.loss_hist[t - 1] = l;
   }
 }
+constexpr unsigned kAdamGrid = (NPARAM + kAdamP - 1) / kAdamP;
 
 __global__ void mlp_step_kernel(int *step) { *step += 1; }
 
@@ -523,14 +773,15 @@ __global__ void __launch_bounds__(NT, 2) mlp_infer_mma_kernel(const float *__res
   }
 }
 
-constexpr size_t kGradSmem = sizeof(Weights) + sizeof(Acts) + sizeof(Errs);
+constexpr size_t kGradSmem = sizeof(GradSmem);
+static_assert(kGradSmem <= 227 * 1024, "one CTA an SM");
 constexpr size_t kInferSmem = sizeof(Weights) + sizeof(Acts);
 
 }  // namespace
 
 struct mirt_mlp {
-  DMem master, m, v, wb, part, loss_part, step, grad, losses, idx;
-  int nblk_cap = 0;
+  DMem master, m, v, wb, part, loss_part, step, grad, losses;
+  int nunit_cap = 0;
   int tensor_cores = 1;  // inference on mma.sync (1) or on the FP32 pipes (0)
   float lr = 1e-3f, beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
 };
@@ -538,11 +789,11 @@ struct mirt_mlp {
 namespace {
 
 int ensure_batch(mirt_mlp *q, int batch) {
-  const int nblk = (batch + NS - 1) / NS;
-  if (nblk > q->nblk_cap) {
-    MCK(q->part.alloc((size_t)nblk * NPARAM * sizeof(float)));
-    MCK(q->loss_part.alloc((size_t)nblk * sizeof(float)));
-    q->nblk_cap = nblk;
+  const int nunit = grad_units(batch);
+  if (nunit > q->nunit_cap) {
+    MCK(q->part.alloc((size_t)nunit * NPARAM * sizeof(float)));
+    MCK(q->loss_part.alloc((size_t)nunit * sizeof(float)));
+    q->nunit_cap = nunit;
   }
   return MIRT_OK;
 }
@@ -558,34 +809,34 @@ int set_attrs() {
   return MIRT_OK;
 }
 
-GradArgs grad_args(mirt_mlp *q, const float *x, const float *y, long long n, const long long *idx,
-                   int batch, unsigned long long seed) {
+GradArgs grad_args(mirt_mlp *q, const float *x, const float *y, long long n, int batch,
+                   unsigned long long seed, const int *step) {
   GradArgs g{};
   g.x = x;
   g.y = y;
   g.n = n;
-  g.idx = idx;
   g.batch = batch;
   g.seed = seed;
-  g.step = q->step.as<int>();
+  g.step = step;
   g.wb = q->wb.as<__nv_bfloat16>();
   g.part = q->part.as<float>();
   g.loss_part = q->loss_part.as<float>();
   return g;
 }
 
-AdamArgs adam_args(mirt_mlp *q, int nblk, int apply, float *grad_out, float *loss_hist) {
+AdamArgs adam_args(mirt_mlp *q, int nunit, int apply, float *grad_out, float *loss_hist,
+                   const int *step) {
   AdamArgs a{};
   a.part = q->part.as<float>();
   a.loss_part = q->loss_part.as<float>();
-  a.nblk = nblk;
+  a.nunit = nunit;
   a.master = q->master.as<float>();
   a.m = q->m.as<float>();
   a.v = q->v.as<float>();
   a.wb = q->wb.as<__nv_bfloat16>();
   a.grad_out = grad_out;
   a.loss_hist = loss_hist;
-  a.step = q->step.as<int>();
+  a.step = step;
   a.lr = q->lr;
   a.beta1 = q->beta1;
   a.beta2 = q->beta2;
@@ -610,7 +861,7 @@ int mirt_mlp_create(mirt_mlp **out, const float *params) {
   };
   if (q->master.alloc(NPARAM * sizeof(float)) || q->m.alloc(NPARAM * sizeof(float)) ||
       q->v.alloc(NPARAM * sizeof(float)) || q->wb.alloc(NPARAM * sizeof(__nv_bfloat16)) ||
-      q->step.alloc(sizeof(int)) || q->grad.alloc(NPARAM * sizeof(float)))
+      q->step.alloc(sizeof(int)) || q->grad.alloc((NPARAM + 1) * sizeof(float)))
     return bail(api_fail(MIRT_ERR_ALLOC, "MLP parameter buffers"));
   cudaError_t e = cudaMemcpy(q->master.p, params, NPARAM * sizeof(float), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(q->m.p, 0, NPARAM * sizeof(float));
@@ -640,29 +891,19 @@ int mirt_mlp_grad(mirt_mlp *q, const float *x, const float *y, int64_t n, float 
   cudaStream_t st = as_stream(stream);
   int rc = ensure_batch(q, (int)n);
   if (rc) return rc;
-  DMem idx, lh;
-  std::vector<long long> hidx(n);
-  for (long long i = 0; i < n; i++) hidx[i] = i;
-  MCK(idx.alloc(n * sizeof(long long)));
-  MCK(lh.alloc(sizeof(float)));
-  MCK(cudaMemcpyAsync(idx.p, hidx.data(), n * sizeof(long long), cudaMemcpyHostToDevice, st));
-  const int nblk = (int)((n + NS - 1) / NS);
-  // a fixed-list gradient must not advance the step counter: use a scratch one
-  DMem st0;
-  MCK(st0.alloc(sizeof(int)));
-  MCK(cudaMemsetAsync(st0.p, 0, sizeof(int), st));
-  GradArgs g = grad_args(q, x, y, n, idx.as<long long>(), (int)n, 0);
-  g.step = st0.as<int>();
-  mlp_grad_kernel<<<nblk, NT, kGradSmem, st>>>(g);
+  // the loss behind the gradient, so that one copy brings both
+  std::vector<float> host(NPARAM + 1);
+  float *dg = q->grad.as<float>();
+  mlp_grad_kernel<<<grad_grid((int)n), 2 * GU, kGradSmem, st>>>(
+      grad_args(q, x, y, n, (int)n, 0, nullptr));
   MCK(cudaGetLastError());
-  AdamArgs a = adam_args(q, nblk, 0, q->grad.as<float>(), lh.as<float>());
-  a.step = st0.as<int>();
-  mlp_adam_kernel<<<(NPARAM + 255) / 256, 256, 0, st>>>(a);
+  mlp_adam_kernel<<<kAdamGrid, kAdamP * kAdamK, 0, st>>>(
+      adam_args(q, grad_units((int)n), 0, dg, dg + NPARAM, nullptr));
   MCK(cudaGetLastError());
-  MCK(cudaMemcpyAsync(grad, q->grad.p, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, st));
-  float l = 0.f;
-  MCK(cudaMemcpyAsync(&l, lh.p, sizeof(float), cudaMemcpyDeviceToHost, st));
+  MCK(cudaMemcpyAsync(host.data(), dg, host.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
   MCK(cudaStreamSynchronize(st));
+  std::copy(host.begin(), host.end() - 1, grad);
+  const float l = host[NPARAM];
   if (loss) *loss = l;
   return MIRT_OK;
 } catch (const std::bad_alloc &) {
@@ -682,9 +923,10 @@ int mirt_mlp_train(mirt_mlp *q, const float *x, const float *y, int64_t n, int32
   MCK(cudaMemcpyAsync(&step0, q->step.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   MCK(cudaStreamSynchronize(st));
   MCK(q->losses.alloc((size_t)(step0 + steps + 1) * sizeof(float)));
-  const int nblk = (batch + NS - 1) / NS;
-  GradArgs g = grad_args(q, x, y, n, nullptr, batch, seed);
-  AdamArgs a = adam_args(q, nblk, 1, nullptr, q->losses.as<float>());
+  const int *step = q->step.as<int>();
+  const GradArgs g = grad_args(q, x, y, n, batch, seed, step);
+  const AdamArgs a = adam_args(q, grad_units(batch), 1, nullptr, q->losses.as<float>(), step);
+  const unsigned grid = (unsigned)grad_grid(batch);
   // one training step = three launches; capture a block of steps in a CUDA
   // graph and replay it (the step counter lives on the device)
   const int chunk = steps < 64 ? steps : 64;
@@ -695,8 +937,8 @@ int mirt_mlp_train(mirt_mlp *q, const float *x, const float *y, int64_t n, int32
     cudaGraph_t graph;
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     for (int i = 0; i < chunk && e == cudaSuccess; i++) {
-      mlp_grad_kernel<<<nblk, NT, kGradSmem, cs>>>(g);
-      mlp_adam_kernel<<<(NPARAM + 255) / 256, 256, 0, cs>>>(a);
+      mlp_grad_kernel<<<grid, 2 * GU, kGradSmem, cs>>>(g);
+      mlp_adam_kernel<<<kAdamGrid, kAdamP * kAdamK, 0, cs>>>(a);
       mlp_step_kernel<<<1, 1, 0, cs>>>(q->step.as<int>());
     }
     cudaError_t e2 = cudaStreamEndCapture(cs, &graph);
@@ -713,8 +955,8 @@ int mirt_mlp_train(mirt_mlp *q, const float *x, const float *y, int64_t n, int32
     done += chunk;
   }
   for (; e == cudaSuccess && done < steps; done++) {
-    mlp_grad_kernel<<<nblk, NT, kGradSmem, st>>>(g);
-    mlp_adam_kernel<<<(NPARAM + 255) / 256, 256, 0, st>>>(a);
+    mlp_grad_kernel<<<grid, 2 * GU, kGradSmem, st>>>(g);
+    mlp_adam_kernel<<<kAdamGrid, kAdamP * kAdamK, 0, st>>>(a);
     mlp_step_kernel<<<1, 1, 0, st>>>(q->step.as<int>());
     e = cudaGetLastError();
   }

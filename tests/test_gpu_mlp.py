@@ -132,3 +132,19 @@ def test_learned_dcf_small_end_to_end():
         jack.append(ld.nrmse(wj, h["w"]))
     assert w_err < np.median(jack), (w_err, np.median(jack))
     assert np.median([e["recon_nrmse"] for e in ev]) < 0.2
+
+
+@pytest.mark.parametrize("n", [1, 63, 65, 148 * 64 + 1, 2 * 148 * 64 + 5])
+def test_gradient_at_set_and_unit_edges(n):
+    """Part-filled sets of 64, the second unit of a CTA, a unit's second set; twice
+    the same bits."""
+    rng = np.random.default_rng(n)
+    p = mlp_ref.init_params(rng)
+    x = rng.standard_normal((n, mlp_ref.NFEAT)).astype(np.float32)
+    y = rng.standard_normal(n).astype(np.float32)
+    net = mb.DcfMLP(p)
+    loss, g = net.grad(_dev(x), _dev(y))
+    _, g2 = net.grad(_dev(x), _dev(y))
+    ref_l, ref_g = mlp_ref.grad(p, x, y)
+    assert np.array_equal(g, g2)
+    assert rel_l2(g, ref_g) <= 1e-4 and abs(loss - ref_l) <= 1e-5 * ref_l
