@@ -728,7 +728,8 @@ cudaError_t plan_gather(mirt_interp_plan *P, const float2 *ck, float2 *fm, cudaS
                         int s0 = 0, int s1 = -1) {
   const int S = P->t.nslice;
   if (s1 < 0) s1 = S;
-  if (P->gtma) {
+  // (fewer than 32 columns have always taken grids at any address)
+  if (P->gtma && (P->a.C >= 32 || P->a.g.D == 3 || ((uintptr_t)ck & 15) == 0)) {
     const long long i0 = P->gitem_slice[s0], i1 = P->gitem_slice[s1];
     return launch_gather_tma(P->ag, P->gbk, S, i0, i1 - i0, ck, fm, P->gfault.as<int>(), st,
                              P->gfault_test, P->gtma == 2 ? 16 : 32);
@@ -1168,9 +1169,9 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
   P->ag = a;
   P->gtma = 0;
   if (a.g.D > 1 && Mtot > 0) {
-    // 8-point blocks where the gather runs on TMA-staged tiles (2D, J = 6,
-    // 32-coil chunks), 4-point blocks otherwise
-    const int gbs = (gather_tma_ok(a) && P->lg.cw == 32) ? gather_tma_block() : 4;
+    // 8-point blocks where the gather runs on TMA-staged tiles (2D, J = 6, an even
+    // C >= 16), 4-point blocks otherwise
+    const int gbs = gather_tma_ok(a) ? gather_tma_block() : 4;
     Tiling t4 = P->t;
     t4.nbins = 1;
     for (int d = 0; d < MIRT_DMAX; d++) {
@@ -1210,26 +1211,28 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
       CK(cudaMemcpy(hb.data(), bs4.p, (nb4 + 1) * sizeof(int), cudaMemcpyDeviceToHost));
       const int rc_n = tma3 ? gather_tma3_item() : gather_tma_item();
       const long long per = (long long)t4.nbins;
-      std::vector<int2> items;
+      std::vector<int4> items;
       P->gitem_slice.assign(nslice + 1, 0);
       for (long long bk = 0; bk < nb4; bk++) {
         if (bk % per == 0) P->gitem_slice[bk / per] = (long long)items.size();
-        for (int p0 = hb[bk]; p0 < hb[bk + 1]; p0 += rc_n) items.push_back(make_int2((int)bk, p0));
+        for (int p0 = hb[bk]; p0 < hb[bk + 1]; p0 += rc_n)
+          items.push_back(make_int4((int)bk, p0, std::min(rc_n, hb[bk + 1] - p0), 0));
       }
       P->gitem_slice[nslice] = (long long)items.size();
-      CK(P->gitem.alloc(std::max<size_t>(items.size(), 1) * sizeof(int2)));
+      CK(P->gitem.alloc(std::max<size_t>(items.size(), 1) * sizeof(int4)));
       if (!items.empty())
-        CK(cudaMemcpy(P->gitem.p, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(P->gitem.p, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
       CK(P->orec_g.alloc(Mtot * sizeof(int4)));
       mirt_plan_kernels::out_records_kernel<<<(unsigned)((Mtot + 255) / 256), 256, 0, st>>>(
           Mtot, P->ag.perm, P->ag.phase, P->orec_g.as<int4>());
       CK(cudaGetLastError());
       CK(cudaStreamSynchronize(st));
-      P->gbk = GatherBlocks{P->gblk.as<int>(), P->gitem.as<int2>(), P->orec_g.as<int4>(), gbs,
+      P->gbk = GatherBlocks{P->gitem.as<int4>(), P->orec_g.as<int4>(), gbs,
                             t4.nbin[0], t4.nbin[1], t4.nbin[2]};
       CK(P->gfault.alloc(sizeof(int)));
       CK(cudaMemset(P->gfault.p, 0, sizeof(int)));
-      P->gtma = 1;  // the default where it applies; the autotuner times both
+      // the default where it applies; the autotuner times the forms
+      P->gtma = a.g.D == 2 && a.C < 32 ? 2 : 1;
     }
   }
   int rc2 = build_tasks(P, st);
@@ -1696,7 +1699,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
   }
   if (had_tma)
     for (int mode : {1, 2}) {  // tiles of 32 or 16 coils (3D: of 8 coils, mode 1 only)
-      if (mode == 2 && a.g.D == 3) continue;
+      if (mode == (a.g.D == 3 ? 2 : a.C < 32 ? 1 : 0)) continue;
       P->gtma = mode;
       float ms = 0;
       int rc = time_launch([&]() {
@@ -1735,7 +1738,7 @@ int mirt_interp_plan_set_gather(mirt_interp_plan *P, int32_t tma) {
   if (!P) return fail(MIRT_ERR_ARG, "plan is NULL");
   P = launch_plan(P);
   if (tma < 0 || tma > 2) return fail(MIRT_ERR_ARG, "gather mode must be 0, 1 or 2");
-  if (tma && !P->gbk.item)
+  if (tma && (!P->gbk.item || (P->a.g.D == 2 && P->a.C < 32)))
     return fail(MIRT_ERR_ARG, "TMA gather needs J = 6 and, in 2D, an even C >= 32 and K >= 13, "
                               "in 3D an even C >= 8 and K >= 9");
   if (tma == 2 && P->a.g.D == 3)

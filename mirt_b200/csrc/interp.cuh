@@ -181,8 +181,7 @@ struct Launch {
 // orec[pos] = (caller's sample index, 0, phase as float bits), staged with the
 // tap records.
 struct GatherBlocks {
-  const int *start;
-  const int2 *item;
+  const int4 *item;  // block (slice-major), first position, samples
   const int4 *orec;
   int gb, nbx, nby, nbz;
 };

@@ -83,11 +83,11 @@ struct mirt_interp_plan {
   std::vector<int> dense_slice;           // first dense bin of each slice (+ total)
   std::vector<int> dense_part0_host;      // first chunk of each dense bin (+ total)
   // TMA gather: first position of each block of the gather order, work items
-  // (block, first position), the first item of each slice, fault flag
+  // (block, first position, samples), the first item of each slice, fault flag
   mirt::DMem gblk, gitem, gfault;
   std::vector<long long> gitem_slice;
   mirt::GatherBlocks gbk{};
-  int gtma = 0;            // 1: the gather runs on TMA-staged tiles
+  int gtma = 0;            // the gather's TMA-staged tiles: 1 of 32 coils (3D: 8), 2 of 16
   int gfault_test = 0;     // 1: test of the TMA gather's bounded waits (no copies)
   int split_chunk = 1024;  // sample visits per spread task before a tile is split
   int heavy_first = 1;     // spread task order: 1 heaviest first, 0 grid order

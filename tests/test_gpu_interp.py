@@ -667,6 +667,39 @@ def test_tma_gather_matches_plain_gather_and_oracle(C, K):
     plan.close()
 
 
+@pytest.mark.parametrize("C,K", [(16, (64, 48)), (18, (13, 30)), (24, (40, 33)), (30, (17, 96))])
+def test_tma_gather_of_16_to_31_columns(C, K):
+    """Tiles of 16 columns below 32 (one full chunk, a chunk of 2, of 8, of 14;
+    wrapped blocks as rows or point by point): the plain gather's bits, in its
+    arithmetic, from a grid at an odd multiple of 8 bytes too; the forms of 32
+    columns stay refused."""
+    import torch
+    rng = np.random.default_rng(C)
+    h = [mb.minmax_kb_table(max(k // 2, 6), 6, k, 256) for k in K]
+    tms = [rng.uniform(-20, 20, (900, 2)), rng.uniform(-2, 2, (1500, 2)), rng.uniform(-90, 90, (77, 2))]
+    moff = np.concatenate([[0], np.cumsum([len(t) for t in tms])])
+    plan = mb.InterpPlan(K, [6, 6], [256, 256], h, np.concatenate(tms), C, slice_moff=moff)
+    assert plan.config()["gather_tma"] == 2
+    ck = rng.standard_normal((3, K[1], K[0], C)) + 1j * rng.standard_normal((3, K[1], K[0], C))
+    buf = torch.zeros(ck.size + 1, dtype=torch.complex64, device="cuda")
+    odd = buf[1:].view(ck.shape)
+    odd.copy_(torch.from_numpy(ck.astype(np.complex64)))
+    even = odd.clone()
+    a = plan.forward(even).cpu().numpy()
+    assert np.array_equal(plan.forward(odd).cpu().numpy(), a)
+    for mode in (1, 2):
+        with pytest.raises(mb.MirtError, match="TMA gather"):
+            plan.set_gather(mode)
+    plan.set_gather(False)
+    assert np.array_equal(plan.forward(even).cpu().numpy(), a)
+    for s in range(3):
+        ref = oracle.interp_for(np.transpose(ck[s], (1, 0, 2)).reshape(-1, C, order="F"), h, [6, 6],
+                                [256, 256], tms[s], K, 0, impl=ref_impl())
+        assert rel_l2(a[moff[s]:moff[s + 1]], ref) <= FWD_TOL, s
+    assert plan.fault() == 0
+    plan.close()
+
+
 @pytest.mark.parametrize("C,K", [(8, (32, 24, 20)), (10, (12, 9, 16))])
 def test_tma_gather_3d_matches_plain_gather_and_oracle(C, K):
     """3D gather over TMA-staged 9 x 9 x 9 tiles of 8 coils (4 x 4 x 4 blocks
