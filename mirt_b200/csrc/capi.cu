@@ -231,7 +231,7 @@ int sweep_ok(const InterpArgs &a, const Tiling &t) {
 }
 
 // The 3D line sweep needs: 3D, J = 6, one-point bins, K >= 6 per dimension,
-// and coil chunks of 8, 16 or 32 lanes (blocks of 2 x 2, 2 x 1 or 1 lines).
+// and coil chunks of 8, 16 or 32 lanes (blocks of 4 x 2, 4 x 1 or 2 x 1 lines).
 int sweep3_ok(const InterpArgs &a, const Tiling &t, int cw) {
   if (a.g.D != 3 || (cw != 8 && cw != 16 && cw != 32)) return 0;
   for (int d = 0; d < 3; d++)
@@ -489,56 +489,107 @@ int build_dense(mirt_interp_plan *P, int minc, cudaStream_t st) {
   return MIRT_OK;
 }
 
-// 3D line sweep with nseg uniform segments per line block: the work queue of
-// its teams, heaviest first (cost: the samples of the block's bin lines in
-// the segment and its warm-up columns + 2 per column step).
+// 3D line sweep: the visit lists of its blocks, their parts and the work queue of
+// these, heaviest first (cost: visits + 2 per column step), made once per plan.
 int set_line_sweep3(mirt_interp_plan *P, int nseg, cudaStream_t st) {
   const InterpArgs &a = P->a;
   Tiling &t = P->t;
   const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2], S = t.nslice;
-  const int nl = 32 / P->ls.cw, B2 = nl >= 2 ? 2 : 1, B3 = nl / B2;
-  const int nby = (K2 + B2 - 1) / B2, nbz = (K3 + B3 - 1) / B3;
-  const long long nb = (long long)t.nbins * S;
-  std::vector<int> bs(nb + 1);
-  CK(cudaMemcpyAsync(bs.data(), P->bin_start.p, (nb + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  const int sw = (K1 + nseg - 1) / nseg;
-  const long long nteam = (long long)S * nbz * nby * nseg;
-  std::vector<double> cost(nteam, 0.0);
-  for (long long team = 0; team < nteam; team++) {
-    const int seg = (int)(team % nseg);
-    long long rest = team / nseg;
-    const int by = (int)(rest % nby);
-    rest /= nby;
-    const int bz = (int)(rest % nbz);
-    const int s = (int)(rest / nbz);
-    const int x0 = seg * sw, x1 = std::min(K1, x0 + sw);
-    if (x0 >= x1) continue;
-    double c = kSweepColumnCost * (x1 - x0 + 5);
-    for (int q3 = 0; q3 < B3 + 5; q3++)
-      for (int q2 = 0; q2 < B2 + 5; q2++) {
-        const int r = ((by * B2 - 5 + q2) % K2 + K2) % K2;
-        const int z = ((bz * B3 - 5 + q3) % K3 + K3) % K3;
-        const int *br = bs.data() + (size_t)s * t.nbins + ((size_t)z * K2 + r) * K1;
-        const int xs = x0 - 5;
-        if (xs < 0) c += br[K1] - br[xs + K1];
-        c += br[x1] - br[std::max(xs, 0)];
+  if (!t.s3_off) {
+    // the kernel's blocks of lines (Sweep3): 4 x 2 for 8 coils, 4 x 1 for 16, 2 x 1 for 32
+    const int cw = P->ls.cw, nl = 32 / cw, g2 = nl >= 2 ? 2 : 1, B2 = 2 * g2, B3 = nl / g2;
+    const long long per = (long long)((K2 + B2 - 1) / B2) * ((K3 + B3 - 1) / B3);
+    const long long nblock = per * S;
+    const size_t nchunk = (size_t)std::max(1, (a.C + cw - 1) / cw);
+    // visits per block and column
+    std::vector<int> n((size_t)nblock * K1);
+    {
+      DMem cnt;
+      CK(cnt.alloc(n.size() * sizeof(int)));
+      CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, nullptr, cnt.as<int>(),
+                            nullptr, nullptr, st));
+      CK(cudaMemcpyAsync(n.data(), cnt.p, n.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
+    }
+    long long total = 0;
+    for (int v : n) total += v;
+    // parts: runs of columns of a block with about `most` visits, an eighth of a
+    // warp's share at full occupancy (so that the heaviest one ends with the others)
+    const long long most = std::min<long long>(std::max<long long>(total / (148 * 24 * 8), 64), 1024);
+    std::vector<int4> part, fix;
+    std::vector<long long> off(1, 0), boff(nblock);
+    P->s3_slice_part.assign(S + 1, 0);
+    P->s3_slice_fix.assign(S + 1, 0);
+    int slots = 0;
+    long long at = 0;
+    for (long long b = 0; b < nblock; b++) {
+      if (b % per == 0) {
+        P->s3_slice_part[b / per] = (int)part.size();
+        P->s3_slice_fix[b / per] = (int)fix.size();
       }
-    cost[team] = c;
+      boff[b] = at;
+      const size_t first = part.size();
+      const int *v = n.data() + (size_t)b * K1;
+      long long run = 0;
+      int x0 = 0;
+      for (int x = 0; x < K1; x++) {
+        run += v[x];
+        at += v[x];
+        if (x + 1 == K1 || run + v[x + 1] > most) {
+          part.push_back(make_int4((int)b, x0, x + 1, -1));
+          off.push_back(at);
+          x0 = x + 1;
+          run = 0;
+        }
+      }
+      if (part.size() - first > 1) {
+        fix.push_back(make_int4((int)b, (int)first, (int)(part.size() - first), slots));
+        for (size_t i = first; i < part.size(); i++) part[i].w = slots++;
+      }
+    }
+    P->s3_slice_part[S] = (int)part.size();
+    P->s3_slice_fix[S] = (int)fix.size();
+    const long long np = (long long)part.size();
+    std::vector<int> order(np);
+    for (long long i = 0; i < np; i++) order[i] = (int)i;
+    auto cost = [&](int i) {
+      return (double)(off[i + 1] - off[i]) + kSweepColumnCost * (part[i].z - part[i].y);
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
+    DMem d_boff;
+    CK(d_boff.alloc(std::max<long long>(nblock, 1) * sizeof(long long)));
+    CK(P->s3_off.alloc(off.size() * sizeof(long long)));
+    CK(P->s3_pos.alloc(std::max<long long>(total, 1) * sizeof(int)));
+    CK(P->s3_line.alloc(std::max<long long>(total, 1)));
+    CK(P->s3_part.alloc(std::max<long long>(np, 1) * sizeof(int4)));
+    CK(P->s3_fix.alloc(std::max<size_t>(fix.size(), 1) * sizeof(int4)));
+    CK(P->s3_tail.alloc(std::max<size_t>(slots * nchunk * kSweep3Tail, 1) * sizeof(float2)));
+    CK(P->team_order.alloc(std::max<long long>(np, 1) * sizeof(int)));
+    CK(P->team_next.alloc(nchunk * sizeof(int)));
+    auto up = [&](DMem &d, const void *p, size_t bytes) {
+      return bytes ? cudaMemcpyAsync(d.p, p, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
+    };
+    CK(up(d_boff, boff.data(), boff.size() * sizeof(long long)));
+    CK(up(P->s3_off, off.data(), off.size() * sizeof(long long)));
+    CK(up(P->s3_part, part.data(), part.size() * sizeof(int4)));
+    CK(up(P->s3_fix, fix.data(), fix.size() * sizeof(int4)));
+    CK(up(P->team_order, order.data(), order.size() * sizeof(int)));
+    CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, d_boff.as<long long>(),
+                          nullptr, P->s3_pos.as<int>(), P->s3_line.as<unsigned char>(), st));
+    CK(cudaStreamSynchronize(st));
+    t.s3_pos = P->s3_pos.as<int>();
+    t.s3_line = P->s3_line.as<unsigned char>();
+    t.s3_part = P->s3_part.as<int4>();
+    t.s3_fix = P->s3_fix.as<int4>();
+    t.s3_tail = P->s3_tail.as<float2>();
+    t.s3_part0 = t.s3_fix0 = 0;
+    t.s3_nparts = (int)np;
+    t.s3_nfix = (int)fix.size();
+    t.team_order = P->team_order.as<int>();
+    t.team_next = P->team_next.as<int>();
+    t.s3_off = P->s3_off.as<long long>();
   }
-  std::vector<int> order(nteam);
-  for (long long i = 0; i < nteam; i++) order[i] = (int)i;
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-  if (P->team_order.bytes < std::max<size_t>(order.size(), 1) * sizeof(int))
-    CK(P->team_order.alloc(std::max<size_t>(order.size(), 1) * sizeof(int)));
-  if (!order.empty())
-    CK(cudaMemcpyAsync(P->team_order.p, order.data(), order.size() * sizeof(int),
-                       cudaMemcpyHostToDevice, st));
-  const size_t nq = (size_t)std::max(1, (a.C + P->ls.cw - 1) / std::max(P->ls.cw, 1));
-  if (P->team_next.bytes < nq * sizeof(int)) CK(P->team_next.alloc(nq * sizeof(int)));
-  CK(cudaStreamSynchronize(st));
-  t.team_order = P->team_order.as<int>();
-  t.team_next = P->team_next.as<int>();
+  // (the parts follow the visits, not the segments)
   t.sweep = nseg;
   t.sweep_rows = 1;
   return MIRT_OK;
@@ -813,6 +864,13 @@ void choose_config(mirt_interp_plan *P) {
   t.nteams = 0;
   t.team_order = nullptr;
   t.team_next = nullptr;
+  t.s3_off = nullptr;
+  t.s3_pos = nullptr;
+  t.s3_line = nullptr;
+  t.s3_part = nullptr;
+  t.s3_fix = nullptr;
+  t.s3_tail = nullptr;
+  t.s3_part0 = t.s3_nparts = t.s3_fix0 = t.s3_nfix = 0;
   t.dense_of = nullptr;
   t.dense_bin = nullptr;
   t.patch = nullptr;
@@ -1266,7 +1324,8 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     int rc3 = sweep_buffer(P);
     if (rc3) return rc3;
     rc3 = set_line_sweep3(P, 2, st);
-    if (rc3) return rc3;
+    if (rc3 && rc3 != MIRT_ERR_ALLOC) return rc3;
+    if (rc3) cudaGetLastError();  // no room for the visit lists: the point spread
   }
   // everything else: the point spread
   if (!P->t.sweep && !P->t.split && a.C > 0) {
@@ -1558,11 +1617,9 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
               if (!staged || (cw == 32 && !dense && P->t.wsw))
                 cands.push_back(SpreadCand{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0,
                                            0, 0, nseg, rows, dense, staged});
-  // 3D line sweep: 1, 2, 4 or 8 segments per line block
+  // 3D line sweep
   if (sweep3_ok(a, P->t, cw) && sweep_buffer(P) == MIRT_OK)
-    for (int nseg : {1, 2, 4, 8})
-      cands.push_back(SpreadCand{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0,
-                                 nseg, 1});
+    cands.push_back(SpreadCand{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, 2, 1});
   if (P->points_shape) {
     SpreadCand c{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, 0, 1};
     c.points = P->points_shape;
@@ -3139,6 +3196,12 @@ int nufft_adjoint_range(mirt_nufft *p, int s0, int s1, const float2 *X, float2 *
     t.ndense = P->dense_slice[s1] - t.dense0;
     t.chunk0 = P->dense_part0_host[t.dense0];
     t.nchunks = P->dense_part0_host[t.dense0 + t.ndense] - t.chunk0;
+  }
+  if (t.s3_off) {                // and its parts of the line sweep
+    t.s3_part0 = P->s3_slice_part[s0];
+    t.s3_nparts = P->s3_slice_part[s1] - t.s3_part0;
+    t.s3_fix0 = P->s3_slice_fix[s0];
+    t.s3_nfix = P->s3_slice_fix[s1] - t.s3_fix0;
   }
   t.slice0 = s0;
   t.nslice = s1 - s0;

@@ -196,6 +196,80 @@ cudaError_t radix_sort_bins(const uint32_t *keys, long long n, int nbins, void *
 }
 
 // ------------------------------------------------------------------------
+// visit lists of the 3D line sweep
+// ------------------------------------------------------------------------
+namespace {
+// One warp a block: per bin column, the samples of the bin lines around the block
+// (lane l keeps lines l and l + 32) in line and sort order, then the column's dense
+// bins in line order.
+__global__ void sweep3_list_kernel(InterpArgs a, Tiling t, const int *__restrict__ bin_start, int B2,
+                                   int B3, long long nblock, const long long *__restrict__ off,
+                                   int *__restrict__ count, int *__restrict__ pos,
+                                   unsigned char *__restrict__ line) {
+  const long long block = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  if (block >= nblock) return;
+  const int lane = threadIdx.x & 31;
+  const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2];
+  const int Q2 = B2 + 5, nl = Q2 * (B3 + 5);
+  const int nby = (K2 + B2 - 1) / B2, nbz = (K3 + B3 - 1) / B3;
+  const int y0 = (int)(block % nby) * B2;
+  const int z0 = (int)(block / nby % nbz) * B3;
+  const long long slice = block / ((long long)nby * nbz);
+  const int *bs = bin_start + slice * t.nbins;
+  const int *dof = t.dense_of ? t.dense_of + slice * t.nbins : nullptr;
+  const int dmin = t.dense_of ? t.dense_min : 0x7fffffff;
+  long long base[2];
+  for (int h = 0; h < 2; h++) {
+    const int l = lane + 32 * h;
+    int r = (y0 - 5 + l % Q2) % K2, z = (z0 - 5 + l / Q2) % K3;
+    if (r < 0) r += K2;
+    if (z < 0) z += K3;
+    base[h] = l < nl ? ((long long)z * K2 + r) * K1 : -1;
+  }
+  long long at = off ? off[block] : 0;
+  for (int x = 0; x < K1; x++) {
+    const long long at0 = at;
+    for (int h = 0; h < 2; h++) {
+      const int b0 = base[h] >= 0 ? bs[base[h] + x] : 0;
+      const int n = base[h] >= 0 ? bs[base[h] + x + 1] - b0 : 0;
+      const int s = n >= dmin ? 0 : n;
+      int inc = s;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(FULL, inc, o);
+        if (lane >= o) inc += u;
+      }
+      if (pos)
+        for (int k = 0; k < s; k++) {
+          pos[at + inc - s + k] = b0 + k;
+          line[at + inc - s + k] = (unsigned char)(lane + 32 * h);
+        }
+      at += __shfl_sync(FULL, inc, 31);
+    }
+    for (int h = 0; h < 2 && dof; h++) {
+      const int n = base[h] >= 0 ? bs[base[h] + x + 1] - bs[base[h] + x] : 0;
+      const unsigned m = __ballot_sync(FULL, n >= dmin && n > 0);
+      if (pos && n >= dmin && n > 0) {
+        const long long i = at + __popc(m & ((1u << lane) - 1u));
+        pos[i] = ~dof[base[h] + x];
+        line[i] = (unsigned char)(lane + 32 * h);
+      }
+      at += __popc(m);
+    }
+    if (count && lane == 0) count[block * K1 + x] = (int)(at - at0);
+  }
+}
+}  // namespace
+
+cudaError_t launch_sweep3_list(const InterpArgs &a, const Tiling &t, const int *bin_start, int B2,
+                               int B3, long long nblock, const long long *off, int *count, int *pos,
+                               unsigned char *line, cudaStream_t st) {
+  if (nblock <= 0) return cudaSuccess;
+  sweep3_list_kernel<<<(unsigned)((nblock + 7) / 8), 256, 0, st>>>(a, t, bin_start, B2, B3, nblock,
+                                                                  off, count, pos, line);
+  return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------------
 // per-position tap data
 // ------------------------------------------------------------------------
 cudaError_t launch_prep_taps(const InterpArgs &a, float2 *W, int4 *K0, cudaStream_t st) {

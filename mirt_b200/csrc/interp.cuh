@@ -77,6 +77,19 @@ struct Tiling {
   // chunk], which are cleared before every launch.
   const int *team_order;
   int *team_next;
+  // 3D line sweep: part i covers bin columns [s3_part[i].y, .z) of line block .x (slice-
+  // major, then planes, rows) and meets visits s3_off[i] .. s3_off[i + 1) in order:
+  // s3_pos = the sample's position, or ~d for dense bin d; s3_line = its bin line
+  // around the block.  .w: the part's slot of s3_tail (the five columns past its
+  // last), -1 where it covers its block alone; s3_fix: the blocks of several parts,
+  // (block, first part, parts, first slot).  A launch covers parts [s3_part0,
+  // s3_part0 + s3_nparts) and fix records [s3_fix0, s3_fix0 + s3_nfix).
+  const int4 *s3_part, *s3_fix;
+  float2 *s3_tail;
+  int s3_part0, s3_nparts, s3_fix0, s3_nfix;
+  const long long *s3_off;
+  const int *s3_pos;
+  const unsigned char *s3_line;
   // Dense bins (the sweeps): bins holding at least a threshold of samples.
   // Before a sweep, dense_part/reduce_kernel sum each dense bin's samples into its
   // patch of J^D taps x C (patch[d][tap][c], tap = (j3 J + j2) J + j1), and
@@ -185,6 +198,13 @@ struct GatherBlocks {
   const int4 *orec;
   int gb, nbx, nby, nbz;
 };
+// float2 of a part's tail slot: 5 columns x 2 lines a lane x 32 lanes
+constexpr int kSweep3Tail = 5 * 2 * 32;
+// The 3D line sweep's visit lists for blocks of B2 x B3 lines: counts per block and
+// column (off null), or the lists from the blocks' offsets.
+cudaError_t launch_sweep3_list(const InterpArgs &a, const Tiling &t, const int *bin_start, int B2,
+                               int B3, long long nblock, const long long *off, int *count, int *pos,
+                               unsigned char *line, cudaStream_t st);
 bool gather_tma_ok(const InterpArgs &a);
 int gather_tma_block();
 int gather_tma_item();

@@ -968,218 +968,267 @@ __device__ __forceinline__ void cp_async_wait_group1() {
   asm volatile("cp.async.wait_group 1;" ::: "memory");
 }
 
-constexpr int SW3_CAP = 32;  // visits staged per batch and warp
+// Shape of a warp's block of lines by its coil lanes: lanes = CW coils x NL line
+// groups (G2 along k2, the rest along k3), two neighbouring k2 lines a lane.
 template <int CW>
-constexpr int sweep3_warp_bytes() {
-  return 2 * SW3_CAP * 4 + SW3_CAP * 18 * 8 + SW3_CAP * CW * 8;
-}
+struct Sweep3 {
+  static constexpr int NL = 32 / CW, G2 = NL >= 2 ? 2 : 1;
+  static constexpr int B2 = 2 * G2, B3 = NL / G2;
+  static constexpr int Q2 = B2 + 5, Q3 = B3 + 5;  // bin lines with taps in the block
+  static constexpr int CAP = CW == 8 ? 16 : 8;    // visits staged at a time
+  static_assert(Q2 * Q3 <= 64, "bin line numbers are 6 bits");
+  float2 rec[2][CAP][18];
+  float2 f[2][CAP][CW];
+  int4 k0[2][CAP];
+  float4 w1[CAP][6];  // first-dimension taps as FFMA2 operand pairs (wr, wr, wi, -wi)
+  int4 meta[CAP];     // column, 5 - k2 bin line, 5 - k3 bin line, dense bin or -1
+};
 
-// A warp owns a block of B2 x B3 grid lines along k1 (rows y0 .. y0 + B2 - 1
-// of planes z0 .. z0 + B3 - 1; lanes = CW coils x the block's 32 / CW lines:
-// 2 x 2 lines for 8 coils, 2 x 1 for 16, one line for 32) and a segment
-// [x0, x1) of their columns.  The samples with taps in the block are those
-// binned in the Q2 x Q3 = (B2 + 5) x (B3 + 5) bin lines around it; lane l
-// keeps the bin pointers of bin lines l and l + 32, and loads those of the
-// next column while the current one is summed.  Per bin column the warp
-// lists the column's samples (bin lines in index order, samples in sort
-// order), copies their tap records and sample rows into its shared-memory
-// stage with cp.async (all in flight at once), and then every lane adds each
-// sample's six k1 taps into the six-column window of its own line (when the
-// line is within the sample's 6 x 6 tap rows), with the same FP32 operation
-// order per tap as the tiled spread (conj(w3) f, then conj(w2), then
-// conj(w1)).  Dense bins (at least dense_min samples) add their patches after
-// the column's samples, in bin-line order.  After bin column x, grid column x
-// of every line is complete and is stored once.  The summation order per
-// grid point is fixed and independent of the segments: bitwise reproducible.
+// a lane's coil and its two lines of a block (block: slice-major, then planes, rows)
+template <int CW>
+struct Sweep3Lane {
+  int c0, cl, dy, dz;
+  bool on;
+  __device__ __forceinline__ Sweep3Lane(const InterpArgs &a, int chunk0) {
+    const int lane = threadIdx.x & 31, li = lane / CW;
+    c0 = chunk0;
+    cl = lane % CW;
+    dy = 2 * (li % Sweep3<CW>::G2);
+    dz = li / Sweep3<CW>::G2;
+    on = c0 + cl < a.C;
+  }
+  __device__ __forceinline__ void lines(const InterpArgs &a, int block, float2 *ck,
+                                        float2 *(&out)[2], bool (&ok)[2]) const {
+    const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2];
+    const int nby = (K2 + Sweep3<CW>::B2 - 1) / Sweep3<CW>::B2;
+    const int nbz = (K3 + Sweep3<CW>::B3 - 1) / Sweep3<CW>::B3;
+    const int by = block % nby, bz = block / nby % nbz, slice = block / nby / nbz;
+    const int y = by * Sweep3<CW>::B2 + dy, z = bz * Sweep3<CW>::B3 + dz;
+    const long long rstr = (long long)K1 * a.C;
+    out[0] = ck + (long long)slice * a.grid_elems + ((long long)z * K2 + y) * rstr + c0 + cl;
+    out[1] = out[0] + rstr;
+    ok[0] = on && y < K2 && z < K3;
+    ok[1] = on && y + 1 < K2 && z < K3;
+  }
+};
+
+// A warp owns a block of B2 x B3 grid lines along k1 (4 x 2 lines for 8 coils, 4 x 1
+// for 16, 2 x 1 for 32) and a part of their bin columns.  The samples with taps in the
+// block are those binned in the Q2 x Q3 bin lines around it; the plan lists them per
+// block by column, bin line and sort order, then the column's dense bins
+// (sweep3_list_kernel), and cuts a block's columns into parts of about equal visits
+// (set_line_sweep3), so that the lines through the k-space centre do not set the time.
+// The warp streams its part's list, CAP visits at a time: the next batch's tap records
+// and sample rows on their way (cp.async) and the list of the one after loaded while a
+// batch is summed, every lane adding each sample's six k1 taps into the six-column
+// windows of its lines within the sample's reach, with the FP32 operation order per
+// tap of the tiled spread (conj(w3) f, then conj(w2), then conj(w1)).  When the
+// visits move past column x, grid column x of every line has the part's sum and is
+// stored once; what reaches past the part's last column, five columns, is added after
+// the sweep (sweep3_fix_kernel), or by the warp itself where one part covers the
+// block.  Parts depend on the plan's samples alone and the summation order per grid
+// point is fixed: bitwise reproducible.
+//
+// Bound by instruction issue.  4.19 M samples of 8 coils, 256^3: 5270 us with one line
+// a lane, two fixed segments and the visits found per column from the bin pointers
+// (1127 instructions a sample; the lines through the centre ended last), 4450 us so
+// (7.9 visits a sample in place of 12.3, 802 instructions; without the parts 7800).
 template <int CW, bool REAL>
 __device__ __forceinline__ void sweep3_team(const InterpArgs &a, const Tiling &t,
-                                            const int *__restrict__ bin_start,
                                             const float2 *__restrict__ fs,
-                                            float2 *__restrict__ ck, long long team,
-                                            unsigned char *wsm) {
-  constexpr unsigned FULLM = 0xffffffffu;
-  constexpr int NL = 32 / CW;             // lines per warp
-  constexpr int B2 = NL >= 2 ? 2 : 1;
-  constexpr int B3 = NL / B2;
-  constexpr int Q2 = B2 + 5, Q3 = B3 + 5, NBL = Q2 * Q3;  // bin lines, at most 49
-  static_assert(NBL <= 64, "bin lines must fit two per lane");
-  int *spos = reinterpret_cast<int *>(wsm);
-  int *slin = spos + SW3_CAP;
-  float2 *srec = reinterpret_cast<float2 *>(wsm + 2 * SW3_CAP * 4);
-  float2 *sf = srec + SW3_CAP * 18;
+                                            float2 *__restrict__ ck, int part_id,
+                                            Sweep3<CW> &S) {
+  using Sh = Sweep3<CW>;
+  constexpr int CAP = Sh::CAP, PARTS = 32 / CAP;
   const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2];
-  const int nseg = t.sweep;
-  const int nby = (K2 + B2 - 1) / B2, nbz = (K3 + B3 - 1) / B3;
-  const int seg = (int)(team % nseg);
-  long long rest = team / nseg;
-  const int by = (int)(rest % nby);
-  rest /= nby;
-  const int bz = (int)(rest % nbz);
-  const int slice = t.slice0 + (int)(rest / nbz);
-  const int y0 = by * B2, z0 = bz * B3;
-  const int sw = (K1 + nseg - 1) / nseg;
-  const int x0 = seg * sw, x1 = min(K1, x0 + sw);
-  if (x0 >= x1) return;
-  const int lane = threadIdx.x & 31;
-  const int li = lane / CW, cl = lane % CW;
-  const int dy = li % B2, dz = li / B2;
   const int C = a.C;
-  const int c0 = blockIdx.y * CW;
-  const bool on = c0 + cl < C;
-  const int *bs = bin_start + (long long)slice * t.nbins;
-  const int *dof = t.dense_of ? t.dense_of + (long long)slice * t.nbins : nullptr;
-  const int dmin = t.dense_of ? t.dense_min : 0x7fffffff;
-  auto line_base = [&](int l) -> long long {
-    int r = (y0 - 5 + l % Q2) % K2;
-    if (r < 0) r += K2;
-    int z = (z0 - 5 + l / Q2) % K3;
-    if (z < 0) z += K3;
-    return ((long long)z * K2 + r) * K1;
+  const Sweep3Lane<CW> L(a, (unsigned)blockIdx.y * CW);
+  const int c0 = L.c0, cl = L.cl, dy = L.dy, dz = L.dz;
+  const bool on = L.on;
+  const int4 pt = __ldg(t.s3_part + part_id);
+  float2 *out[2];
+  bool ok[2];
+  L.lines(a, pt.x, ck, out, ok);
+  const int x1 = pt.z;
+  const long long i0 = __ldg(t.s3_off + part_id);
+  const int n = (int)(__ldg(t.s3_off + part_id + 1) - i0);
+  const int lane = threadIdx.x & 31;
+  const int *lp = t.s3_pos + i0;
+  const unsigned char *lq = t.s3_line + i0;
+  const int cb = min(CW, C - c0) * 8;  // bytes of a sample row's chunk
+  const bool even = ((C | c0) & 1) == 0;
+  const int v = lane % CAP, part = lane / CAP;
+  constexpr int NONE = (int)0x80000000;
+  auto fetch = [&](int b, int &e, int &q) {
+    const int i = b * CAP + v;
+    e = i < n ? __ldg(lp + i) : NONE;
+    q = i < n ? __ldg(lq + i) : 0;
   };
-  const long long base0 = lane < NBL ? line_base(lane) : -1;
-  const long long base1 = lane + 32 < NBL ? line_base(lane + 32) : -1;
-  const int xs = x0 - 5;
-  auto wrapx = [&](int x) { return x < 0 ? x + K1 : x; };
-  int beg0 = base0 >= 0 ? __ldg(bs + base0 + wrapx(xs)) : 0;
-  int beg1 = base1 >= 0 ? __ldg(bs + base1 + wrapx(xs)) : 0;
-  // end of each bin line's samples
-  const int rend0 = base0 >= 0 ? __ldg(bs + base0 + K1) : 0;
-  const int rend1 = base1 >= 0 ? __ldg(bs + base1 + K1) : 0;
-  // end pointers of the next column (and the row starts where the sweep wraps)
-  int e0n = base0 >= 0 ? __ldg(bs + base0 + wrapx(xs) + 1) : beg0;
-  int e1n = base1 >= 0 ? __ldg(bs + base1 + wrapx(xs) + 1) : beg1;
-  int r0n = 0, r1n = 0;
-  float2 acc[6];
+  auto issue = [&](int buf, int e) {
+    if (e >= 0) {
+      const float2 *w = a.W + (long long)e * 18;
 #pragma unroll
-  for (int j = 0; j < 6; j++) acc[j] = make_float2(0.f, 0.f);
-  const bool out_ok = on && y0 + dy < K2 && z0 + dz < K3;
-  float2 *out = ck + (long long)slice * a.grid_elems +
-                ((long long)(z0 + dz) * K2 + (y0 + dy)) * K1 * C + c0 + cl;
-  for (int xb = xs; xb < x1; xb++) {
-    const int end0 = e0n, end1 = e1n;
-    if (xb == 0 && xs < 0) {
-      beg0 = r0n;
-      beg1 = r1n;
-    }
-    if (xb + 1 < x1) {
-      const int xn = wrapx(xb + 1);
-      if (base0 >= 0) e0n = __ldg(bs + base0 + xn + 1);
-      if (base1 >= 0) e1n = __ldg(bs + base1 + xn + 1);
-      if (xb + 1 == 0) {
-        if (base0 >= 0) r0n = __ldg(bs + base0);
-        if (base1 >= 0) r1n = __ldg(bs + base1);
+      for (int k = 0; k < (9 + PARTS - 1) / PARTS; k++) {
+        const int ch = k * PARTS + part;
+        if (ch < 9) cp_async16(&S.rec[buf][v][2 * ch], w + 2 * ch);
       }
-    }
-    const int n0 = end0 - beg0, n1 = end1 - beg1;
-    const int s0 = n0 >= dmin ? 0 : n0, s1 = n1 >= dmin ? 0 : n1;
-    // the column's sparse samples: line 0 .. 31, then 32 .. 48, in lane order
-    int i0 = s0, i1 = s1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u0 = __shfl_up_sync(FULLM, i0, o), u1 = __shfl_up_sync(FULLM, i1, o);
-      if (lane >= o) {
-        i0 += u0;
-        i1 += u1;
-      }
-    }
-    const int tot0 = __shfl_sync(FULLM, i0, 31);
-    const int V = tot0 + __shfl_sync(FULLM, i1, 31);
-    const int ex0 = i0 - s0, ex1 = tot0 + i1 - s1;
-    for (int vb = 0; vb < V; vb += SW3_CAP) {
-      const int nb = min(SW3_CAP, V - vb);
-      for (int k = max(0, vb - ex0); k < s0 && ex0 + k < vb + SW3_CAP; k++) {
-        spos[ex0 + k - vb] = beg0 + k;
-        slin[ex0 + k - vb] = lane;
-      }
-      for (int k = max(0, vb - ex1); k < s1 && ex1 + k < vb + SW3_CAP; k++) {
-        spos[ex1 + k - vb] = beg1 + k;
-        slin[ex1 + k - vb] = lane + 32;
-      }
-      __syncwarp();
-      for (int ch = lane; ch < nb * 9; ch += 32) {
-        const int v = ch / 9, k = ch - 9 * v;
-        cp_async16(srec + v * 18 + 2 * k, a.W + (long long)spos[v] * 18 + 2 * k);
-      }
-      for (int ch = lane; ch < nb * CW; ch += 32) {
-        const int v = ch / CW, k = ch - CW * v;
-        if (c0 + k < C)
-          cp_async8(sf + v * CW + k, fs + (long long)spos[v] * C + c0 + k);
-        else
-          sf[v * CW + k] = make_float2(0.f, 0.f);
-      }
-      cp_async_wait_all();
-      __syncwarp();
-      for (int v = 0; v < nb; v++) {
-        const int L = slin[v];
-        const int j2 = dy - L % Q2 + 5, j3 = dz - L / Q2 + 5;
-        if (j2 >= 0 && j2 < 6 && j3 >= 0 && j3 < 6) {
-          const float2 *rv = srec + v * 18;
-          const float2 v3 = cw_mul<REAL>(rv[12 + j3], sf[v * CW + cl]);
-          const float2 vv = cw_mul<REAL>(rv[6 + j2], v3);
-#pragma unroll
-          for (int j = 0; j < 6; j++) cmac_conj<REAL>(acc[j], rv[j], vv);
-        }
-      }
-      __syncwarp();  // the stage is read before the next batch refills it
-    }
-    // dense bins: their patches, in bin-line order
-    unsigned md0 = __ballot_sync(FULLM, n0 >= dmin && n0 > 0);
-    unsigned md1 = __ballot_sync(FULLM, n1 >= dmin && n1 > 0);
-    const bool had_dense = (md0 | md1) != 0;
-    while (md0 | md1) {
-      int L;
-      long long bb;
-      if (md0) {
-        L = __ffs(md0) - 1;
-        md0 &= md0 - 1;
-        bb = __shfl_sync(FULLM, base0, L);
+      if (part == PARTS - 1) cp_async16(&S.k0[buf][v], a.K0 + e);
+      const float2 *f = fs + (long long)e * C + c0;
+      if (even) {
+        for (int k = 16 * part; k < cb; k += 16 * PARTS)
+          cp_async16(&S.f[buf][v][k / 8], f + k / 8);
       } else {
-        const int l = __ffs(md1) - 1;
-        md1 &= md1 - 1;
-        bb = __shfl_sync(FULLM, base1, l);
-        L = l + 32;
-      }
-      const int dn = __ldg(dof + bb + wrapx(xb));
-      const int j2 = dy - L % Q2 + 5, j3 = dz - L / Q2 + 5;
-      if (on && j2 >= 0 && j2 < 6 && j3 >= 0 && j3 < 6) {
-        const float2 *pp = t.patch + ((long long)dn * 216 + (j3 * 6 + j2) * 6) * C + c0 + cl;
-#pragma unroll
-        for (int j = 0; j < 6; j++) {
-          const float2 v = __ldg(pp + (long long)j * C);
-          acc[j].x += v.x;
-          acc[j].y += v.y;
-        }
+        for (int k = 8 * part; k < cb; k += 8 * PARTS) cp_async8(&S.f[buf][v][k / 8], f + k / 8);
       }
     }
-    beg0 = end0;
-    beg1 = end1;
-    if (xb >= x0 && out_ok) out[(long long)xb * C] = acc[0];
+    cp_async_commit();
+  };
+  float2 acc[2][6];
 #pragma unroll
-    for (int j = 0; j < 5; j++) acc[j] = acc[j + 1];
-    acc[5] = make_float2(0.f, 0.f);
-    // skip-ahead: after a column with no sample, jump to the next column in
-    // which any of the bin lines holds one (the first tap column of each
-    // line's next sample); the columns in between receive nothing
-    if (V == 0 && !had_dense && xb >= 0 && xb + 1 < x1) {
-      const int nc0 = beg0 < rend0 ? __ldg(&a.K0[beg0].x) : x1;
-      const int nc1 = beg1 < rend1 ? __ldg(&a.K0[beg1].x) : x1;
-      const int xn = min(__reduce_min_sync(FULLM, min(nc0, nc1)), x1);
-      if (xn > xb + 1) {
-        int x = xb + 1;
-        for (int k = 0; k < 6 && x < xn; k++, x++) {
-          if (x >= x0 && out_ok) out[(long long)x * C] = acc[0];
+  for (int j = 0; j < 6; j++) acc[0][j] = acc[1][j] = make_float2(0.f, 0.f);
+  int x = pt.y;
+  auto advance = [&]() {
+    if (ok[0]) out[0][(long long)x * C] = acc[0][0];
+    if (ok[1]) out[1][(long long)x * C] = acc[1][0];
 #pragma unroll
-          for (int j = 0; j < 5; j++) acc[j] = acc[j + 1];
-          acc[5] = make_float2(0.f, 0.f);
-        }
-        for (; x < xn; x++)
-          if (x >= x0 && out_ok) out[(long long)x * C] = make_float2(0.f, 0.f);
-        xb = xn - 1;  // the loop moves on to column xn
-        if (xn < x1) {
-          if (base0 >= 0) e0n = __ldg(bs + base0 + xn + 1);
-          if (base1 >= 0) e1n = __ldg(bs + base1 + xn + 1);
+    for (int j = 0; j < 5; j++) {
+      acc[0][j] = acc[0][j + 1];
+      acc[1][j] = acc[1][j + 1];
+    }
+    acc[0][5] = acc[1][5] = make_float2(0.f, 0.f);
+    x++;
+  };
+  int e0, q0, e1, q1;
+  fetch(0, e0, q0);
+  if (n > 0) issue(0, e0);
+  fetch(1, e1, q1);
+  for (int b = 0; b * CAP < n; b++) {
+    const int buf = b & 1;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    // this batch's visits: their columns and bin lines, the first taps in pairs
+    if (part == 0) {
+      int col = 0, dn = -1;
+      if (e0 >= 0) {
+        col = S.k0[buf][v].x;
+      } else if (e0 != NONE) {
+        dn = ~e0;
+        col = __ldg(t.dense_bin + dn) % K1;
+      }
+      S.meta[v] = make_int4(dn < 0 ? col : col | NONE, 5 - q0 % Sh::Q2, 5 - q0 / Sh::Q2, dn);
+    }
+#pragma unroll
+    for (int k = 0; k < (6 + PARTS - 1) / PARTS; k++) {
+      const int j = k * PARTS + part;
+      if (j < 6) {
+        const float2 w = S.rec[buf][v][j];
+        S.w1[v][j] = make_float4(w.x, w.x, w.y, -w.y);
+      }
+    }
+    __syncwarp();
+    if ((b + 1) * CAP < n) issue(buf ^ 1, e1);
+    e0 = e1;
+    q0 = q1;
+    fetch(b + 2, e1, q1);
+    const int nb = min(CAP, n - b * CAP);
+#pragma unroll 1
+    for (int u = 0; u < nb; u++) {
+      const int4 m = S.meta[u];
+      while (x < (m.x & ~NONE)) advance();
+      const int j2 = dy + m.y, j3 = dz + m.z;
+      if ((unsigned)j3 < 6u && (unsigned)(j2 + 1) < 7u) {
+        if (m.x >= 0) {
+          const float2 *rv = S.rec[buf][u];
+          const float2 v3 = cw_mul<REAL>(rv[12 + j3], S.f[buf][u][cl]);
+          float4 w[6];
+#pragma unroll
+          for (int j = 0; j < 6; j++) w[j] = S.w1[u][j];
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            {
+              const bool in = (unsigned)(j2 + r) < 6u;
+              float2 vv = cw_mul<REAL>(rv[6 + j2 + r], v3);
+              vv.x = in ? vv.x : 0.f;
+              vv.y = in ? vv.y : 0.f;
+              const float2 vs = make_float2(vv.y, vv.x);
+#pragma unroll
+              for (int j = 0; j < 6; j++) {
+                acc[r][j] = __ffma2_rn(make_float2(w[j].x, w[j].y), vv, acc[r][j]);
+                if (!REAL) acc[r][j] = __ffma2_rn(make_float2(w[j].z, w[j].w), vs, acc[r][j]);
+              }
+            }
+          }
+        } else if (on) {
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            if ((unsigned)(j2 + r) < 6u) {
+              const float2 *pp =
+                  t.patch + ((long long)m.w * 216 + (j3 * 6 + j2 + r) * 6) * C + c0 + cl;
+#pragma unroll
+              for (int j = 0; j < 6; j++) {
+                const float2 p = __ldg(pp + (long long)j * C);
+                acc[r][j].x += p.x;
+                acc[r][j].y += p.y;
+              }
+            }
+          }
         }
       }
+      __syncwarp();  // (every lane comes here: they go on to the next visit together)
+    }
+    __syncwarp();
+  }
+  while (x < x1) advance();
+  // the five columns past the last
+  if (pt.w < 0) {
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+      if (ok[r])
+#pragma unroll
+        for (int j = 0; j < 5; j++) {
+          float2 *p = out[r] + (long long)j * C;
+          const float2 o = *p;
+          *p = make_float2(o.x + acc[r][j].x, o.y + acc[r][j].y);
+        }
+  } else {
+    float2 *tl = t.s3_tail + ((long long)pt.w * gridDim.y + blockIdx.y) * kSweep3Tail + lane;
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int j = 0; j < 5; j++) tl[(2 * j + r) * 32] = acc[r][j];
+  }
+  __syncwarp();
+}
+
+// Blocks of several parts: every part's tail added to the columns it reaches, in part
+// order (after the sweep; one warp a block and coil chunk).
+template <int CW>
+__global__ void __launch_bounds__(256) sweep3_fix_kernel(InterpArgs a, Tiling t,
+                                                         float2 *__restrict__ ck) {
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= t.s3_nfix) return;
+  const int4 fx = __ldg(t.s3_fix + t.s3_fix0 + i);
+  const Sweep3Lane<CW> L(a, (unsigned)blockIdx.y * CW);
+  float2 *out[2];
+  bool ok[2];
+  L.lines(a, fx.x, ck, out, ok);
+  const int K1 = a.g.K[0];
+  for (int p = 0; p < fx.z; p++) {
+    const int xe = __ldg(&t.s3_part[fx.y + p].z);
+    const float2 *tl = t.s3_tail +
+                       ((long long)(fx.w + p) * gridDim.y + blockIdx.y) * kSweep3Tail +
+                       (threadIdx.x & 31);
+#pragma unroll
+    for (int j = 0; j < 5; j++) {
+      const int x = xe + j < K1 ? xe + j : xe + j - K1;
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+        if (ok[r]) {
+          const float2 v = tl[(2 * j + r) * 32];
+          float2 *o = out[r] + (long long)x * a.C;
+          const float2 w = *o;
+          *o = make_float2(w.x + v.x, w.y + v.y);
+        }
     }
   }
 }
@@ -1187,25 +1236,19 @@ __device__ __forceinline__ void sweep3_team(const InterpArgs &a, const Tiling &t
 // Persistent 3D line sweep over the plan's heaviest-first work queue (one
 // counter per coil chunk); a warp is one team, with its own shared-memory stage.
 template <int CW, bool REAL>
-__global__ void __launch_bounds__(256) spread_sweep3_kernel(InterpArgs a, Tiling t,
-                                                            const int *__restrict__ bin_start,
-                                                            const float2 *__restrict__ fs,
-                                                            float2 *__restrict__ ck) {
+__global__ void __launch_bounds__(256, 3) spread_sweep3_kernel(InterpArgs a, Tiling t,
+                                                               const float2 *__restrict__ fs,
+                                                               float2 *__restrict__ ck) {
   extern __shared__ __align__(16) unsigned char sm3[];
-  constexpr int NL = 32 / CW;
-  constexpr int B2 = NL >= 2 ? 2 : 1;
-  constexpr int B3 = NL / B2;
+  using Sh = Sweep3<CW>;
   const int lane = threadIdx.x & 31;
-  unsigned char *wsm = sm3 + (threadIdx.x >> 5) * sweep3_warp_bytes<CW>();
-  const long long nteam = (long long)t.nslice * ((a.g.K[1] + B2 - 1) / B2) *
-                          ((a.g.K[2] + B3 - 1) / B3) * t.sweep;
+  Sh &S = reinterpret_cast<Sh *>(sm3)[threadIdx.x >> 5];
   for (;;) {
     int qi = 0;
     if (lane == 0) qi = atomicAdd(t.team_next + blockIdx.y, 1);
     qi = __shfl_sync(0xffffffffu, qi, 0);
-    if (qi >= nteam) break;
-    const long long team = t.team_order ? (long long)__ldg(t.team_order + qi) : qi;
-    sweep3_team<CW, REAL>(a, t, bin_start, fs, ck, team, wsm);
+    if (qi >= t.s3_nparts) break;
+    sweep3_team<CW, REAL>(a, t, fs, ck, t.s3_part0 + (t.team_order ? __ldg(t.team_order + qi) : qi), S);
   }
 }
 
@@ -1764,7 +1807,7 @@ cudaError_t run(Req &r) {
     if constexpr (D == 3 && JT == 6 && (CW == 8 || CW == 16 || CW == 32)) {
       if (t.sweep > 0) {
         const unsigned nchunk = (unsigned)((a.C + CW - 1) / CW);
-        if (!t.sorted || !t.team_next) return cudaErrorInvalidValue;
+        if (!t.sorted || !t.team_next || !t.s3_off) return cudaErrorInvalidValue;
         if (a.Mtot > 0) {
           const long long p0 = t.npos < 0 ? 0 : t.pos0;
           const long long np = t.npos < 0 ? a.Mtot : t.npos;
@@ -1781,7 +1824,8 @@ cudaError_t run(Req &r) {
           if (e != cudaSuccess) return e;
         }
         auto kern = spread_sweep3_kernel<CW, REAL>;
-        const size_t smem3 = 8 * (size_t)sweep3_warp_bytes<CW>();
+        using Sh = Sweep3<CW>;
+        const size_t smem3 = 8 * sizeof(Sh);
         int per_sm = 0, dev = 0, nsm = 0;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem3);
@@ -1790,15 +1834,16 @@ cudaError_t run(Req &r) {
         if (e != cudaSuccess) return e;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        constexpr int NL = 32 / CW, B2 = NL >= 2 ? 2 : 1, B3 = NL / B2;
-        const long long teams = (long long)t.nslice * ((a.g.K[1] + B2 - 1) / B2) *
-                                ((a.g.K[2] + B3 - 1) / B3) * t.sweep;
+        const long long teams = t.s3_nparts;
         long long nb = (long long)nsm * (per_sm > 0 ? per_sm : 1);
         if (nb > (teams + 7) / 8) nb = (teams + 7) / 8;
         if (nb < 1) nb = 1;
         e = cudaMemsetAsync(t.team_next, 0, nchunk * sizeof(int), r.st);
         if (e != cudaSuccess) return e;
-        kern<<<dim3((unsigned)nb, nchunk), 256, smem3, r.st>>>(a, t, r.bin_start, t.sorted, r.out);
+        kern<<<dim3((unsigned)nb, nchunk), 256, smem3, r.st>>>(a, t, t.sorted, r.out);
+        e = cudaGetLastError();
+        if (e != cudaSuccess || t.s3_nfix <= 0) return e;
+        sweep3_fix_kernel<CW><<<dim3((unsigned)(t.s3_nfix + 7) / 8, nchunk), 256, 0, r.st>>>(a, t, r.out);
         return cudaGetLastError();
       }
     }

@@ -73,6 +73,9 @@ struct mirt_interp_plan {
   mirt::DMem swept;        // row-sweep spread: the samples in plan order, [Mtot][C]
   mirt::DMem sweep_teams;  // row-sweep spread: balanced team list (int4 per team)
   std::vector<int4> team_host;  // the same list on the host
+  // 3D line sweep: the parts' visit lists and records, first part / fix of each slice
+  mirt::DMem s3_off, s3_pos, s3_line, s3_part, s3_fix, s3_tail;
+  std::vector<int> s3_slice_part, s3_slice_fix;
   mirt::DMem team_order, team_next;  // row-sweep work queue: heaviest-first order, counter
   mirt::DMem pt_task, pt_hdr, pt_scratch, pt_count;  // point spread (Tiling)
   mirt::DMem split_teams, split_next;                // split spread (Tiling)

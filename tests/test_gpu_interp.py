@@ -838,6 +838,42 @@ def test_3d_line_sweep_matches_oracle(C):
     plan.close()
 
 
+@pytest.mark.parametrize("C", [8, 9, 17])
+def test_3d_line_sweep_parts_and_tails(C):
+    """Lines cut into parts of few columns (crowded columns, some side by side, some
+    alone, at both ends of the lines): the parts' five columns past their last meet
+    in one column, wrap, and cross further parts; odd column counts (rows at odd
+    multiples of 8 bytes); an empty slice between two; a sample of infinities stays
+    within its own taps."""
+    import torch
+    rng = np.random.default_rng(5 + C)
+    K, J, L = [40, 11, 9], [6, 6, 6], [64, 64, 64]
+    h = [mb.minmax_kb_table(k // 2, 6, k, 64) for k in K]
+
+    def cluster(x, n):
+        return np.stack([x + rng.uniform(0, 1, n), rng.uniform(-4, 4, n), rng.uniform(-4, 4, n)], 1)
+    tms = [np.concatenate([cluster(x, n) for x, n in
+                           ((0, 700), (1, 600), (2, 30), (3, 900), (17, 500), (36, 10), (39, 800))]),
+           np.zeros((0, 3)), np.concatenate([cluster(38, 900), rng.uniform(-30, 30, (50, 3))])]
+    moff = np.concatenate([[0], np.cumsum([len(t) for t in tms])])
+    plan = mb.InterpPlan(K, J, L, h, np.concatenate(tms), C, slice_moff=moff)
+    plan.set_sweep(2)
+    fm = rng.standard_normal((moff[-1], C)) + 1j * rng.standard_normal((moff[-1], C))
+    fd = torch.from_numpy(fm.astype(np.complex64)).cuda()
+    out = plan.adjoint(fd).cpu().numpy()
+    assert np.array_equal(out, plan.adjoint(fd).cpu().numpy())
+    assert not out[1].any()
+    for s in (0, 2):
+        ref = oracle.interp_adj(fm[moff[s]:moff[s + 1]], h, J, L, tms[s], K, 0, impl=ref_impl())
+        got = np.transpose(out[s], (2, 1, 0, 3)).reshape(-1, C, order="F")
+        assert rel_l2(got, ref) <= ADJ_TOL, s
+    # the last sample's taps alone turn non-finite
+    fd[-1] = float("inf")
+    bad = ~np.isfinite(plan.adjoint(fd).cpu().numpy()[..., 0])
+    assert not bad[:2].any() and 0 < bad[2].sum() <= 216
+    plan.close()
+
+
 @pytest.mark.parametrize("order", [0, 1])
 def test_3d_line_sweep_real_tables_phase(order):
     """3D line sweep with real tables (order 0 and 1) and a per-sample phase,

@@ -308,3 +308,19 @@ def test_grids_through_cufft(N, K, C):
         assert rel_l2(X[sl, C - 1], nr.nufft(x[s, ..., C - 1].T, st_o, fw)) <= FWD_TOL
         assert rel_l2(z[s, ..., C - 1].T, nr.nufft_adj(y[sl, C - 1], st_o, ad)) <= ADJ_TOL
     plan.close()
+
+
+def test_host_calls_of_3d_slices():
+    """Slice ranges of the 3D line sweep (its parts and tails by slice): the pipelined
+    host adjoint against the device adjoint."""
+    import torch
+    rng = np.random.default_rng(8)
+    om = rng.uniform(-np.pi, np.pi, (9000, 3))
+    om[:4000] *= 0.1
+    plan = mb.NufftPlan(om, (16, 12, 10), (6, 6, 6), (32, 24, 20), Ld=64, ncol=8,
+                        slice_moff=[0, 4500, 4500, 7000, 9000])
+    y = (rng.standard_normal((9000, 8)) + 1j * rng.standard_normal((9000, 8))).astype(np.complex64)
+    a = plan.adjoint(torch.from_numpy(y).cuda()).cpu().numpy()
+    b = plan.adjoint_host(y)
+    assert rel_l2(b, a) <= 1e-6
+    plan.close()
