@@ -543,8 +543,11 @@ int set_line_sweep3(mirt_interp_plan *P, int nseg, cudaStream_t st) {
         }
       }
       if (part.size() - first > 1) {
-        fix.push_back(make_int4((int)b, (int)first, (int)(part.size() - first), slots));
-        for (size_t i = first; i < part.size(); i++) part[i].w = slots++;
+        const int n = (int)(part.size() - first), slot0 = slots;
+        for (size_t i = first; i < part.size(); i++) {
+          fix.push_back(make_int4((int)b, (int)first, n, slot0));
+          part[i].w = slots++;
+        }
       }
     }
     P->s3_slice_part[S] = (int)part.size();

@@ -81,8 +81,8 @@ struct Tiling {
   // major, then planes, rows) and meets visits s3_off[i] .. s3_off[i + 1) in order:
   // s3_pos = the sample's position, or ~d for dense bin d; s3_line = its bin line
   // around the block.  .w: the part's slot of s3_tail (the five columns past its
-  // last), -1 where it covers its block alone; s3_fix: the blocks of several parts,
-  // (block, first part, parts, first slot).  A launch covers parts [s3_part0,
+  // last), -1 where it covers its block alone; s3_fix[slot] = (block, its first part,
+  // its parts, its first slot).  A launch covers parts [s3_part0,
   // s3_part0 + s3_nparts) and fix records [s3_fix0, s3_fix0 + s3_nfix).
   const int4 *s3_part, *s3_fix;
   float2 *s3_tail;

@@ -856,8 +856,9 @@ __global__ void __launch_bounds__(256) spread_sweep_kernel(InterpArgs a, Tiling 
 // and the samples' sort order, into patch_part[i].  dense_reduce_kernel:
 // block d adds its bin's chunk sums in chunk order into patch[d].
 constexpr int DP_CH = 64;
+constexpr int kDenseThreads = 384;
 template <int D, bool REAL>
-__global__ void __launch_bounds__(256) dense_part_kernel(InterpArgs a, Tiling t,
+__global__ void __launch_bounds__(kDenseThreads) dense_part_kernel(InterpArgs a, Tiling t,
                                                          const float2 *__restrict__ fs) {
   constexpr int NR = D == 3 ? 36 : 6;  // (j3, j2) rows of a patch
   constexpr int SJ = D == 3 ? 18 : 12;
@@ -897,7 +898,8 @@ __global__ void __launch_bounds__(256) dense_reduce_kernel(InterpArgs a, Tiling 
   const int q0 = __ldg(t.dense_part0 + d), q1 = __ldg(t.dense_part0 + d + 1);
   const long long pn = (long long)NP * a.C;
   float2 *out = t.patch + (long long)d * pn;
-  for (long long e = threadIdx.x; e < pn; e += blockDim.x) {
+  for (long long e = blockIdx.y * blockDim.x + threadIdx.x; e < pn;
+       e += (long long)gridDim.y * blockDim.x) {
     const float2 *src = t.patch_part + e;
     float2 v = src[(long long)q0 * pn];
     int q = q0 + 1;
@@ -931,10 +933,16 @@ cudaError_t launch_dense_patches(const InterpArgs &a, const Tiling &t, const flo
   auto k1 = dense_part_kernel<D, REAL>;
   cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  k1<<<(unsigned)t.nchunks, 256, sm, st>>>(a, t, fs);
+  // as many threads as rows, or even shares of them (3D, 8 coils: 288 rows)
+  const int rows = (D == 3 ? 36 : 6) * a.C, turns = (rows + kDenseThreads - 1) / kDenseThreads;
+  const unsigned threads = (unsigned)(((rows + turns - 1) / turns + 31) / 32 * 32);
+  k1<<<(unsigned)t.nchunks, threads, sm, st>>>(a, t, fs);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  dense_reduce_kernel<D><<<(unsigned)t.ndense, 256, 0, st>>>(a, t);
+  // an entry a thread: one block a bin took as long as the central bin's chunks, read
+  // seven times over (kooshball of 8 coils: 236 us, 122 us so)
+  const long long pn = (long long)(D == 3 ? 216 : 36) * a.C;
+  dense_reduce_kernel<D><<<dim3((unsigned)t.ndense, (unsigned)((pn + 255) / 256)), 256, 0, st>>>(a, t);
   return cudaGetLastError();
 }
 
@@ -976,6 +984,9 @@ struct Sweep3 {
   static constexpr int B2 = 2 * G2, B3 = NL / G2;
   static constexpr int Q2 = B2 + 5, Q3 = B3 + 5;  // bin lines with taps in the block
   static constexpr int CAP = CW == 8 ? 16 : 8;    // visits staged at a time
+  // two visits in flight a warp against 24 warps an SM (8 coils 4305 against 4420 us,
+  // 16 coils -1 %, 32 coils +4 %)
+  static constexpr int UNROLL = CW == 32 ? 1 : 2, PER_SM = CW == 32 ? 3 : 2;
   static_assert(Q2 * Q3 <= 64, "bin line numbers are 6 bits");
   float2 rec[2][CAP][18];
   float2 f[2][CAP][CW];
@@ -1031,8 +1042,9 @@ struct Sweep3Lane {
 //
 // Bound by instruction issue.  4.19 M samples of 8 coils, 256^3: 5270 us with one line
 // a lane, two fixed segments and the visits found per column from the bin pointers
-// (1127 instructions a sample; the lines through the centre ended last), 4450 us so
-// (7.9 visits a sample in place of 12.3, 802 instructions; without the parts 7800).
+// (1127 instructions a sample; the lines through the centre ended last), 4305 us so
+// (7.9 visits a sample in place of 12.3, some 800 instructions; without the parts
+// 7800).
 template <int CW, bool REAL>
 __device__ __forceinline__ void sweep3_team(const InterpArgs &a, const Tiling &t,
                                             const float2 *__restrict__ fs,
@@ -1131,7 +1143,7 @@ __device__ __forceinline__ void sweep3_team(const InterpArgs &a, const Tiling &t
     q0 = q1;
     fetch(b + 2, e1, q1);
     const int nb = min(CAP, n - b * CAP);
-#pragma unroll 1
+#pragma unroll Sh::UNROLL
     for (int u = 0; u < nb; u++) {
       const int4 m = S.meta[u];
       while (x < (m.x & ~NONE)) advance();
@@ -1200,35 +1212,52 @@ __device__ __forceinline__ void sweep3_team(const InterpArgs &a, const Tiling &t
   __syncwarp();
 }
 
-// Blocks of several parts: every part's tail added to the columns it reaches, in part
-// order (after the sweep; one warp a block and coil chunk).
+// Blocks of several parts: the columns from a part's end to the next one's take the
+// tails that reach them, oldest part first (after the sweep; one warp a part and coil
+// chunk.  A warp a block waited on its parts one by one: 217 us for a kooshball, whose
+// central lines have a part a column, 92 us so).
 template <int CW>
 __global__ void __launch_bounds__(256) sweep3_fix_kernel(InterpArgs a, Tiling t,
                                                          float2 *__restrict__ ck) {
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= t.s3_nfix) return;
-  const int4 fx = __ldg(t.s3_fix + t.s3_fix0 + i);
+  const int4 fx = __ldg(t.s3_fix + t.s3_fix0 + i);  // block, first part, parts, first slot
+  const int p = t.s3_fix0 + i - fx.w;
   const Sweep3Lane<CW> L(a, (unsigned)blockIdx.y * CW);
   float2 *out[2];
   bool ok[2];
   L.lines(a, fx.x, ck, out, ok);
   const int K1 = a.g.K[0];
-  for (int p = 0; p < fx.z; p++) {
-    const int xe = __ldg(&t.s3_part[fx.y + p].z);
-    const float2 *tl = t.s3_tail +
-                       ((long long)(fx.w + p) * gridDim.y + blockIdx.y) * kSweep3Tail +
-                       (threadIdx.x & 31);
+  // the ends of this part and the four before it around the line (every part has a
+  // column, so no further one reaches past this end), and of the next
+  int end[5], slot[5];
 #pragma unroll
-    for (int j = 0; j < 5; j++) {
-      const int x = xe + j < K1 ? xe + j : xe + j - K1;
+  for (int b = 0; b < 5; b++) {
+    int q = p - b, e = 0;
+    while (q < 0) {
+      q += fx.z;
+      e -= K1;
+    }
+    end[b] = e + __ldg(&t.s3_part[fx.y + q].z);
+    slot[b] = fx.w + q;
+  }
+  const int next = p + 1 < fx.z ? __ldg(&t.s3_part[fx.y + p + 1].z) : K1 + __ldg(&t.s3_part[fx.y].z);
+  for (int x = end[0]; x < min(next, end[0] + 5); x++) {
+    const long long at = (long long)(x < K1 ? x : x - K1) * a.C;
 #pragma unroll
-      for (int r = 0; r < 2; r++)
-        if (ok[r]) {
-          const float2 v = tl[(2 * j + r) * 32];
-          float2 *o = out[r] + (long long)x * a.C;
-          const float2 w = *o;
-          *o = make_float2(w.x + v.x, w.y + v.y);
-        }
+    for (int r = 0; r < 2; r++) {
+      if (!ok[r]) continue;
+      float2 v = out[r][at];
+#pragma unroll
+      for (int b = 4; b >= 0; b--) {
+        const int j = x - end[b];
+        if (j > 4) continue;
+        const float2 w = t.s3_tail[((long long)slot[b] * gridDim.y + blockIdx.y) * kSweep3Tail +
+                                   (2 * j + r) * 32 + (threadIdx.x & 31)];
+        v.x += w.x;
+        v.y += w.y;
+      }
+      out[r][at] = v;
     }
   }
 }
@@ -1236,9 +1265,9 @@ __global__ void __launch_bounds__(256) sweep3_fix_kernel(InterpArgs a, Tiling t,
 // Persistent 3D line sweep over the plan's heaviest-first work queue (one
 // counter per coil chunk); a warp is one team, with its own shared-memory stage.
 template <int CW, bool REAL>
-__global__ void __launch_bounds__(256, 3) spread_sweep3_kernel(InterpArgs a, Tiling t,
-                                                               const float2 *__restrict__ fs,
-                                                               float2 *__restrict__ ck) {
+__global__ void __launch_bounds__(256, Sweep3<CW>::PER_SM)
+    spread_sweep3_kernel(InterpArgs a, Tiling t, const float2 *__restrict__ fs,
+                         float2 *__restrict__ ck) {
   extern __shared__ __align__(16) unsigned char sm3[];
   using Sh = Sweep3<CW>;
   const int lane = threadIdx.x & 31;
