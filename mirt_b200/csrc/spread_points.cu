@@ -221,9 +221,10 @@ __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
   const bool pairs = ((J1 | (D > 1 ? J2 : 0) | (D > 2 ? J3 : 0)) & 1) == 0;
   const int nq2 = BY + J2 - 1, nq = nq2 * (BZ + J3 - 1);
   const int ci = gl / LS, sub = gl % LS;  // the staged sample this lane copies, and its share
-  // pass 0: the tap rows' bins up to the brick's end; pass 1 (tiles at the
-  // grid's start): their bins before 0, at the end of the periodic row
-  const int npass = t1 == 0 && J1 > 1 ? 2 : 1;
+  // pass 0: the tap rows' bins up to the brick's end; pass 1 (tiles that start
+  // within J1 - 1 points of the grid's start, of which there may be several: a tile
+  // is 8 points wide or more): their bins before 0, at the end of the periodic row
+  const int npass = t1 * pt.W * (BX * X) < J1 - 1 ? 2 : 1;
   for (int ps = 0; ps < npass; ps++) {
     int total = 0;
     for (int e0 = 0; e0 < nq; e0 += GL) {

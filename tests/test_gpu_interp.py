@@ -986,6 +986,34 @@ def test_point_spread_matches_oracle(K, J, C, variant):
     plan.close()
 
 
+@pytest.mark.parametrize("K,J,C", [
+    # base tiles 8 points wide along dimension 1 (2D from 17 columns, 3D from 5): J1 - 1 taps
+    # within the first tile, up to its end, past it into the second
+    ((64, 40), (9, 6), 17), ((64, 40), (10, 10), 24), ((40, 33), (13, 5), 32), ((64, 40), (16, 16), 33),
+    ((19, 21), (16, 3), 24), ((16, 16), (16, 16), 20), ((24, 20, 18), (9, 4, 3), 5),
+    ((24, 20, 18), (10, 5, 4), 9), ((25, 18, 14), (13, 3, 6), 17), ((24, 16, 13), (16, 2, 5), 5),
+    ((16, 17, 18), (16, 16, 16), 3), ((40, 30), (16, 4), 1), ((70,), (16,), 33),
+])
+def test_point_spread_of_wide_kernels(K, J, C):
+    """Up to 16 taps: coordinates whose first-dimension taps wrap from the grid's end, which
+    then reach the tiles after the first one, spread over the grid and crowded at its start."""
+    import torch
+    D = len(K)
+    rng = np.random.default_rng(sum(K) + 7 * C)
+    L = [64] * D
+    h = [mb.newfft_kb_table(j, 64) for j in J]
+    tm = np.concatenate([rng.uniform(-2 * max(K), 2 * max(K), (500, D)),
+                         rng.uniform(-9, 9, (300, D))])
+    plan = mb.InterpPlan(list(K), list(J), L, h, tm, C, order=1)
+    assert plan.config()["spread_points"] > 0
+    fm = rng.standard_normal((len(tm), C)) + 1j * rng.standard_normal((len(tm), C))
+    out = plan.adjoint(torch.from_numpy(fm.astype(np.complex64)).cuda()).cpu().numpy()[0]
+    got = np.transpose(out, tuple(range(D - 1, -1, -1)) + (D,)).reshape(-1, C, order="F")
+    ref = oracle.interp_adj(fm, h, list(J), L, tm, list(K), 1, impl=ref_impl())
+    assert rel_l2(got, ref) <= ADJ_TOL
+    plan.close()
+
+
 @pytest.mark.parametrize("K,C,order", [((64, 48), 25, 0), ((41, 50), 32, 1), ((96, 80), 33, 0),
                                        ((6, 7), 64, 0)])
 def test_split_spread_matches_oracle(K, C, order):
