@@ -164,11 +164,76 @@ __global__ void point_count_kernel(InterpArgs a, Tiling t, PtTile pt, int ngrp,
   }
 }
 
+// One lane's sums again, tap by tap from global memory, over the samples of its
+// group's share (chunks part, part + 2^lg, ... of S samples of the brick's runs) in
+// the walk's order and operations: X points from (x, y, z), columns c, c + cw, ...
+// below C.  Called where the walk left a sum that is not finite; kept out of line, so
+// that the walk's registers don't pay for it (one real column, 26,750 samples on 402 x
+// 350: 22.9 -> 23.6 us, 16 columns on 384^2 112.0 -> 111.2; a test in the walk cost 2 to
+// 5 % of the one- to 24-column passes).
+template <int D, int NC, bool REAL>
+__device__ __noinline__ void points_redo(const InterpArgs &a, const Tiling &t, const int *bin_start,
+                                         const float2 *fm, int slice, int X0, int Y0, int Z0, int bw,
+                                         int by0, int bz0, int part, int lg, int S, int x, int y,
+                                         int z, int c, int cw, float2 *acc) {
+  const Geom &g = a.g;
+  const int *bs = bin_start + (long long)slice * t.nbins;
+  const int J1 = g.J[0], J2 = D > 1 ? g.J[1] : 1, J3 = D > 2 ? g.J[2] : 1;
+  const int K1 = g.K[0], K2 = D > 1 ? g.K[1] : 1, K3 = D > 2 ? g.K[2] : 1;
+  const int nq2 = by0 + J2 - 1, nq = nq2 * (bz0 + J3 - 1);
+  for (int k = 0; k < NC * PT_X; k++) acc[k] = make_float2(0.f, 0.f);
+  for (int ps = 0; ps < 2; ps++) {
+    int base = 0;  // samples of the runs before this one
+    for (int e = 0; e < nq; e++) {
+      const int yq = Y0 - J2 + 1 + e % nq2, zq = Z0 - J3 + 1 + e / nq2;
+      if (yq >= K2 || zq >= K3) continue;
+      const int *row = bs + ((zq < 0 ? zq + K3 : zq) * K2 + (yq < 0 ? yq + K2 : yq)) * K1;
+      const int u = X0 - J1 + 1;
+      int l = 0, n = 0;
+      if (ps == 0) {
+        l = row[max(u, 0)];
+        n = row[min(X0 + bw, K1)] - l;
+      } else if (u < 0) {
+        l = row[u + K1];
+        n = row[K1] - l;
+      }
+      const int j2 = y - yq, j3 = z - zq;
+      for (int v = base; v < base + n; v++) {
+        const int chunk = v / S;
+        if ((chunk & ((1 << lg) - 1)) != part) {  // to the share's next chunk
+          v = (chunk + ((part - chunk) & ((1 << lg) - 1))) * S - 1;
+          continue;
+        }
+        if (j2 < 0 || j2 >= J2 || j3 < 0 || j3 >= J3) continue;
+        const long long p = l + (v - base);
+        const int4 h = t.pt_hdr[p];
+        const float2 *w = a.W + p * a.SJ;
+        float2 wo = D > 1 ? w[J1 + j2] : make_float2(1.f, 0.f);
+        if (D > 2) {
+          const float2 w3 = w[J1 + J2 + j3];
+          wo = REAL ? make_float2(wo.x * w3.x, 0.f) : cmul(wo, w3);
+        }
+        for (int m = 0; m < NC; m++) {
+          if (c + m * cw >= a.C) break;
+          float2 f = fm[(long long)h.y * a.C + c + m * cw];
+          if (a.phase) f = cmulc(make_float2(__int_as_float(h.z), __int_as_float(h.w)), f);
+          if (D > 1) f = detail::cw_mul<REAL>(wo, f);
+          for (int k = 0; k < PT_X; k++) {
+            const int j1 = x + k - h.x + (ps ? K1 : 0);
+            if (j1 >= 0 && j1 < J1) detail::cmac_conj<REAL>(acc[m * PT_X + k], w[j1], f);
+          }
+        }
+      }
+      base += n;
+    }
+  }
+}
+
 template <int D, int CW, int NC, bool REAL>
 __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
-    spread_points_kernel(InterpArgs a, Tiling t, PtTile pt, PtSmem sm,
-                         const int *__restrict__ bin_start, const float2 *__restrict__ fm,
-                         float2 *__restrict__ ck) {
+    spread_points_kernel(const __grid_constant__ InterpArgs a, const __grid_constant__ Tiling t,
+                         PtTile pt, PtSmem sm, const int *__restrict__ bin_start,
+                         const float2 *__restrict__ fm, float2 *__restrict__ ck) {
   using Sh = PtShape<CW>;
   constexpr int LB = Sh::LB, GL = Sh::GL, NGRP = Sh::NGRP, S = Sh::S, LS = Sh::LS, X = PT_X;
   constexpr int BX = PtBrick<D, LB>::BX, BY = PtBrick<D, LB>::BY, BZ = PtBrick<D, LB>::BZ;
@@ -360,6 +425,24 @@ __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
         }
       }
       __syncwarp();
+    }
+  }
+  // A block's four points take the zeros beside the taps as well, which would make NaN
+  // of an infinite or NaN product.  Such a product never leaves a sum finite.
+  {
+    float chk = 0.f;  // 0 x of any sum: NaN where one is not finite
+#pragma unroll
+    for (int m = 0; m < NC; m++)
+#pragma unroll
+      for (int k = 0; k < X; k++) chk = fmaf(0.f, acc[m][k].x, fmaf(0.f, acc[m][k].y, chk));
+    if (__builtin_expect(chk != 0.f, 0)) {
+      float2 again[NC * X];
+      points_redo<D, NC, REAL>(a, t, bin_start, fm, slice, X0, Y0, Z0, BX * X, BY, BZ, part, lg, S,
+                               X0 + bx, Y0 + by, Z0 + bz, c0 + cl, CW, again);
+#pragma unroll
+      for (int m = 0; m < NC; m++)
+#pragma unroll
+        for (int k = 0; k < X; k++) acc[m][k] = again[m * X + k];
     }
   }
   // sum a brick's groups in order: those of this CTA, then those of the

@@ -1014,6 +1014,52 @@ def test_point_spread_of_wide_kernels(K, J, C):
     plan.close()
 
 
+def _taps_of(t, J, K):
+    """Mask [K_D, ..., K_1] of the grid points that a sample at t reaches."""
+    m = np.ones((), bool)
+    for d in range(len(K)):
+        row = np.zeros(K[d], bool)
+        row[(1 + int(np.floor(t[d] - J[d] / 2)) + np.arange(J[d])) % K[d]] = True
+        m = np.multiply.outer(row, m)
+    return m
+
+
+@pytest.mark.parametrize("K,J,C", [
+    ((50,), (6,), 2), ((64, 48), (6, 6), 1), ((33, 35), (5, 4), 3), ((40, 41), (6, 6), 7),
+    ((48, 40), (6, 6), 16), ((48, 40), (6, 6), 26), ((48, 40), (6, 6), 33), ((40, 36), (12, 5), 32),
+    ((20, 18, 16), (6, 6, 6), 1), ((17, 14, 13), (5, 4, 3), 5), ((16, 12, 14), (4, 6, 5), 18),
+])
+@pytest.mark.parametrize("value", ["inf", "nan", "large", "large taps"])
+def test_point_spread_keeps_non_finite_samples_to_their_taps(K, J, C, value):
+    """A sample that is infinite, NaN or overflows times its taps changes the grid points of its
+    own taps alone, all other points keep their bits: the point spread and the split spread
+    sum blocks of four points."""
+    import torch
+    D = len(K)
+    rng = np.random.default_rng(sum(K) + C)
+    L = [64] * D
+    h = [mb.newfft_kb_table(j, 64) for j in J]
+    if value == "large taps":
+        h[-1] = h[-1] * 2.0 ** 100
+    tm = np.concatenate([rng.uniform(-40, 40, (400, D)), rng.uniform(-2, 2, (1500, D))])
+    plan = mb.InterpPlan(list(K), list(J), L, h, tm, C, order=1)
+    assert plan.config()["spread_points"] > 0
+    fm = torch.from_numpy((rng.standard_normal((len(tm), C)) +
+                           1j * rng.standard_normal((len(tm), C))).astype(np.complex64)).cuda()
+    v = {"inf": complex(np.inf, -np.inf), "nan": complex(np.nan, 0), "large": 3e38 * (1 + 1j),
+         "large taps": 2.0 ** 40 * (1 + 1j)}[value]
+    for m in (0, 17, 399, 400, 1899):
+        fm0, fm1 = fm.clone(), fm.clone()
+        fm0[m] = 0
+        fm1[m] = v
+        a, b = plan.adjoint(fm0).cpu().numpy()[0], plan.adjoint(fm1).cpu().numpy()[0]
+        own = _taps_of(tm[m], J, K)
+        assert np.array_equal(a[~own], b[~own]), m
+        if not value.startswith("large"):
+            assert not np.isfinite(b[own]).any(), m
+    plan.close()
+
+
 @pytest.mark.parametrize("K,C,order", [((64, 48), 25, 0), ((41, 50), 32, 1), ((96, 80), 33, 0),
                                        ((6, 7), 64, 0)])
 def test_split_spread_matches_oracle(K, C, order):
