@@ -418,7 +418,10 @@ __device__ __forceinline__ void tile_copy5(const CUtensorMap *tm, void *dst, uin
 // copied as 9 x 9 rows of 9 x 8 coils (4-D map, 576-byte rows) instead of
 // 9 x 9 x 9 rows of 8 coils (5-D map, 64-byte rows); the same layout in shared
 // memory.
-// Wrapped tiles as in 2D (stage_issue).
+// Wrapped tiles: in pieces of their rows where the rows are contiguous (FLAT); else not
+// staged, their samples read the grid: the tile is 729 points of 64 bytes, and copying it
+// point by point takes longer than the taps of an item's 32 samples (64^3, 78,592 samples
+// of 16 coils on a kooshball: 503 us, 159 us tap by tap).
 template <bool FLAT>
 __device__ __forceinline__ void stage3_issue(const CUtensorMap *tm, const InterpArgs &a,
                                              const float2 *ck, const int4 *orec, unsigned char *st,
@@ -427,14 +430,13 @@ __device__ __forceinline__ void stage3_issue(const CUtensorMap *tm, const Interp
   constexpr unsigned PT = T3_CW * 8;
   const int lane = threadIdx.x & 31;
   const unsigned wb = (unsigned)r.n * 144u, kb = (unsigned)r.n * 16u;
-  const unsigned cb = 8u * (unsigned)min(T3_CW, a.C - chunk * T3_CW);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (lane == 0) {
     *hdr = r;
     if (no_copy)
       mbar_expect(bar, 16u);
     else
-      mbar_expect(bar, (r.interior ? T3_TILE_RAW : T3_TW * T3_TW * T3_TW * cb) + wb + 2 * kb);
+      mbar_expect(bar, (FLAT || r.interior ? T3_TILE_RAW : 0u) + wb + 2 * kb);
   }
   __syncwarp();
   if (no_copy) return;
@@ -450,29 +452,22 @@ __device__ __forceinline__ void stage3_issue(const CUtensorMap *tm, const Interp
     bulk_copy(st + T3_TILE + T3_W_BYTES, a.K0 + r.p0, kb, bar);
     bulk_copy(st + T3_TILE + T3_W_BYTES + T3_K_BYTES, orec + r.p0, kb, bar);
   }
-  if (r.interior) return;
+  if (!FLAT || r.interior) return;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2];
   const int x0 = r.bx * T3_GB, y0 = r.by * T3_GB, z0 = r.bz * T3_GB;
-  const float2 *gs = ck + (long long)r.slice * a.grid_elems + chunk * T3_CW;
+  const float2 *gs = ck + (long long)r.slice * a.grid_elems;
   auto at = [&](int x, int y, int z) -> const float2 * {
     y = y0 + y < K2 ? y0 + y : y0 + y - K2;
     z = z0 + z < K3 ? z0 + z : z0 + z - K3;
-    return gs + (((long long)z * K2 + y) * K1 + (x0 + x < K1 ? x0 + x : x0 + x - K1)) * a.C;
+    return gs + (((long long)z * K2 + y) * K1 + (x0 + x < K1 ? x0 + x : x0 + x - K1)) * T3_CW;
   };
-  if (FLAT) {
-    const unsigned n1 = (unsigned)min(T3_TW, K1 - x0);
-    for (int e = lane; e < T3_TW * T3_TW; e += 32) {
-      unsigned char *d = st + e * T3_TW * PT;
-      bulk_copy(d, at(0, e % T3_TW, e / T3_TW), n1 * PT, bar);
-      if (n1 < T3_TW)
-        bulk_copy(d + n1 * PT, at((int)n1, e % T3_TW, e / T3_TW), (T3_TW - n1) * PT, bar);
-    }
-  } else {
-    for (int e = lane; e < T3_TW * T3_TW * T3_TW; e += 32) {
-      const int x = e % T3_TW, yz = e / T3_TW;
-      bulk_copy(st + e * PT, at(x, yz % T3_TW, yz / T3_TW), cb, bar);
-    }
+  const unsigned n1 = (unsigned)min(T3_TW, K1 - x0);
+  for (int e = lane; e < T3_TW * T3_TW; e += 32) {
+    unsigned char *d = st + e * T3_TW * PT;
+    bulk_copy(d, at(0, e % T3_TW, e / T3_TW), n1 * PT, bar);
+    if (n1 < T3_TW)
+      bulk_copy(d + n1 * PT, at((int)n1, e % T3_TW, e / T3_TW), (T3_TW - n1) * PT, bar);
   }
 }
 
@@ -547,20 +542,46 @@ __global__ void __launch_bounds__(TG_THREADS, 2)
       const float2 *tl = tile +
                          (((k0.z - z0 + j30) * T3_TW + (k0.y - y0)) * T3_TW + (k0.x - x0)) *
                              T3_CW + cl;
+      if (FLAT || r.interior) {
 #pragma unroll
-      for (int j3 = 0; j3 < 3; j3++) {
-        detail::CAcc s2;
-        detail::cacc_zero(s2);
+        for (int j3 = 0; j3 < 3; j3++) {
+          detail::CAcc s2;
+          detail::cacc_zero(s2);
 #pragma unroll
-        for (int j2 = 0; j2 < 6; j2++) {
-          const float2 *row = tl + (j3 * T3_TW + j2) * T3_TW * T3_CW;
-          detail::CAcc s1;
-          detail::cacc_zero(s1);
+          for (int j2 = 0; j2 < 6; j2++) {
+            const float2 *row = tl + (j3 * T3_TW + j2) * T3_TW * T3_CW;
+            detail::CAcc s1;
+            detail::cacc_zero(s1);
 #pragma unroll
-          for (int j1 = 0; j1 < 6; j1++) detail::cacc_mac<REAL>(s1, w1[j1], row[j1 * T3_CW]);
-          detail::cacc_mac<false>(s2, Ws[6 + j2], detail::cacc_get<REAL>(s1));
+            for (int j1 = 0; j1 < 6; j1++) detail::cacc_mac<REAL>(s1, w1[j1], row[j1 * T3_CW]);
+            detail::cacc_mac<false>(s2, Ws[6 + j2], detail::cacc_get<REAL>(s1));
+          }
+          pl[j3] = detail::cacc_get<false>(s2);
         }
-        pl[j3] = detail::cacc_get<false>(s2);
+      } else {
+        // (lanes past the last coil read the first one's points)
+        const float2 *gs = ck + (long long)r.slice * a.grid_elems + (on ? c : 0);
+        const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2];
+        int xo[6];
+#pragma unroll
+        for (int j1 = 0; j1 < 6; j1++) xo[j1] = detail::tap_k(k0.x, j1, K1) * C;
+#pragma unroll
+        for (int j3 = 0; j3 < 3; j3++) {
+          const float2 *plane = gs + (long long)detail::tap_k(k0.z, j30 + j3, K3) * K2 * K1 * C;
+          detail::CAcc s2;
+          detail::cacc_zero(s2);
+#pragma unroll
+          for (int j2 = 0; j2 < 6; j2++) {
+            const float2 *row = plane + detail::tap_k(k0.y, j2, K2) * (K1 * C);
+            detail::CAcc s1;
+            detail::cacc_zero(s1);
+#pragma unroll
+            for (int j1 = 0; j1 < 6; j1++)
+              detail::cacc_mac<REAL>(s1, w1[j1], __ldg(row + xo[j1]));
+            detail::cacc_mac<false>(s2, Ws[6 + j2], detail::cacc_get<REAL>(s1));
+          }
+          pl[j3] = detail::cacc_get<false>(s2);
+        }
       }
       detail::CAcc s3;
       detail::cacc_zero(s3);

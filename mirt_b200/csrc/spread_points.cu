@@ -168,7 +168,7 @@ __global__ void point_count_kernel(InterpArgs a, Tiling t, PtTile pt, int ngrp,
 // group's share (chunks part, part + 2^lg, ... of S samples of the brick's runs) in
 // the walk's order and operations: X points from (x, y, z), columns c, c + cw, ...
 // below C.  Called where the walk left a sum that is not finite; kept out of line, so
-// that the walk's registers don't pay for it (one real column, 26,750 samples on 402 x
+// that the walk's registers don't pay for it (one real column, 63,114 samples on 402 x
 // 350: 22.9 -> 23.6 us, 16 columns on 384^2 112.0 -> 111.2; a test in the walk cost 2 to
 // 5 % of the one- to 24-column passes).
 template <int D, int NC, bool REAL>

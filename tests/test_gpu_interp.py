@@ -742,6 +742,42 @@ def test_tma_gather_3d_matches_plain_gather_and_oracle(C, K):
     p6.close()
 
 
+def _median_ms(f, n=15):
+    import torch
+    for _ in range(3):
+        f()
+    ms = []
+    for _ in range(n):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda._sleep(100000)                # the launches queue up behind it
+        a.record()
+        f()
+        b.record()
+        b.synchronize()
+        ms.append(a.elapsed_time(b))
+    return float(np.median(ms))
+
+
+@pytest.mark.parametrize("C", [16, 20])
+def test_3d_gather_time_follows_the_coil_chunks(C):
+    """A 3D gather of two or three chunks of eight coils takes no more than its chunks' share of
+    one chunk's time (30 % allowed), although the tiles of the blocks whose taps wrap, a
+    third of these, are not contiguous in a grid of more than eight coils."""
+    import torch
+    rng = np.random.default_rng(C)
+    K = [64, 64, 64]
+    tm = rng.uniform(-32, 32, (100000, 3))
+    ms = {}
+    for c in (8, C):
+        plan = mb.InterpPlan(K, [6] * 3, [64] * 3, [mb.newfft_kb_table(6, 64)] * 3, tm, c, order=1)
+        assert plan.config()["gather_tma"] == 1
+        ck = torch.randn(plan.grid_shape, dtype=torch.complex64, device="cuda")
+        out = torch.empty(plan.sample_shape, dtype=torch.complex64, device="cuda")
+        ms[c] = _median_ms(lambda: plan.forward(ck, out=out))
+        plan.close()
+    assert ms[C] <= 1.3 * -(-C // 8) * ms[8], ms
+
+
 @pytest.mark.parametrize("order", [0, 1])
 def test_tma_gather_3d_real_tables(order):
     """3D TMA gather with real tables (order 0 and 1): the plain 3D gather's
