@@ -319,15 +319,17 @@ int mirt_interp_plan_set_staged(mirt_interp_plan *plan, int32_t mode);
  * 13 x 13 x 32-coil grid tile (cp.async.bulk.tensor) and the item's tap
  * coefficients and first taps (1-D bulk copies) into shared memory, two
  * stages deep, and reads all taps and records from there; tiles that wrap
- * past K come in contiguous pieces.  Same arithmetic and summation order
+ * past K come in contiguous pieces, or are read from the grid where these
+ * pieces would be too many.  Same arithmetic and summation order
  * as the plain gather: identical results.  tma = 1: tiles of 32 coils (a warp
  * per sample, two CTAs per SM); 2: tiles of 16 coils (a half-warp per sample,
  * three CTAs per SM); 0 selects the plain gather.  3D plans (J = 6, an even
  * C >= 8, K >= 9): tma = 1 stages 9 x 9 x 9 x 8-coil tiles of 4 x 4 x 4
  * blocks of first taps (items of up to 32 samples, a half-warp per
  * sample); mode 2 is 2D only.  The autotuner times the forms that apply.
- * 2D plans of 16 to 31 columns (even) gather on tiles of 16 by default
- * (reported as 2; not selectable here, 0 selects the plain gather).
+ * 2D plans of 16 to 31 columns (even) with samples enough (two to 32 per 8 x 8
+ * block of first taps, by the columns) gather on tiles of 16 by default (reported
+ * as 2; not selectable here: 0 selects the plain gather, the autotuner either).
  * MIRT_ERR_ARG for other modes and where the plan has no TMA blocks.  No
  * reference counterpart. */
 int mirt_interp_plan_set_gather(mirt_interp_plan *plan, int32_t tma);

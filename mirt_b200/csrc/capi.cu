@@ -1292,8 +1292,10 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
                             t4.nbin[0], t4.nbin[1], t4.nbin[2]};
       CK(P->gfault.alloc(sizeof(int)));
       CK(cudaMemset(P->gfault.p, 0, sizeof(int)));
-      // the default where it applies; the autotuner times the forms
-      P->gtma = a.g.D == 2 && a.C < 32 ? 2 : 1;
+      // the default where it pays; the autotuner times the forms
+      P->gtma = a.g.D == 3 ? 1
+                : !gather_tma_default(a, (long long)items.size()) ? 0
+                : a.C < 32 ? 2 : 1;
     }
   }
   int rc2 = build_tasks(P, st);

@@ -42,6 +42,7 @@ namespace {
 constexpr int TG_GB = 8;               // block of first taps per dimension
 constexpr int TG_TW = TG_GB + 5;       // tile extent per dimension (J = 6)
 constexpr int TG_RC = 96;              // samples per work item
+constexpr int TG_WRAP = 24;            // samples of an item whose wrapped tile is copied point by point
 constexpr unsigned TG_W_BYTES = TG_RC * 12 * 8;                 // 9,216
 constexpr unsigned TG_K_BYTES = TG_RC * 16;                     // 1,536
 constexpr unsigned TG_O_BYTES = TG_RC * 16;                     // 1,536
@@ -124,9 +125,10 @@ __device__ __forceinline__ bool stage_release(int *done, int nwarp) {
 
 struct Item {
   int slice, bx, by, p0, n;
-  bool interior;
+  bool interior, staged;
 };
 
+template <int TCW>
 __device__ __forceinline__ Item item_of(const GatherBlocks &g, const InterpArgs &a, int4 it) {
   Item r;
   const long long per = (long long)g.nbx * g.nby;
@@ -137,6 +139,7 @@ __device__ __forceinline__ Item item_of(const GatherBlocks &g, const InterpArgs 
   r.p0 = it.y;
   r.n = it.z;
   r.interior = r.bx * TG_GB + TG_TW <= a.g.K[0] && r.by * TG_GB + TG_TW <= a.g.K[1];
+  r.staged = r.interior || a.C == TCW || r.n >= TG_WRAP;
   return r;
 }
 
@@ -146,7 +149,9 @@ __device__ __forceinline__ Item item_of(const GatherBlocks &g, const InterpArgs 
 // contiguous pieces, by all lanes: its rows, in two where they wrap, when the chunk
 // holds all coils, else point by point.  (Wrapped blocks hold the samples around the
 // k-space axes, 10 % of a radial 2D trajectory and a third of a 3D one; read from
-// global memory tap by tap they set the kernels' time.)  no_copy (the test of the
+// global memory tap by tap they set the kernels' time.)  Point by point is 169 copies:
+// an item of fewer than TG_WRAP samples reads their taps from the grid instead (128^2,
+// 48 coils, 8 slices of 6,552 samples: 39 us copied, 27 us so).  no_copy (the test of the
 // bounded waits): arm the barrier for bytes that no copy will deliver and issue no
 // copy, so that its wait runs out with nothing in flight.
 template <int TCW>
@@ -165,7 +170,7 @@ __device__ __forceinline__ void stage_issue(const CUtensorMap *tm, const InterpA
     if (no_copy)
       mbar_expect(bar, 16u);
     else
-      mbar_expect(bar, (r.interior ? TILE : TG_TW * TG_TW * cb) + wb + 2 * kb);
+      mbar_expect(bar, (r.interior ? TILE : r.staged ? TG_TW * TG_TW * cb : 0u) + wb + 2 * kb);
   }
   __syncwarp();
   if (no_copy) return;
@@ -176,7 +181,7 @@ __device__ __forceinline__ void stage_issue(const CUtensorMap *tm, const InterpA
     bulk_copy(st + TILE + TG_W_BYTES, a.K0 + r.p0, kb, bar);
     bulk_copy(st + TILE + TG_W_BYTES + TG_K_BYTES, orec + r.p0, kb, bar);
   }
-  if (r.interior) return;
+  if (r.interior || !r.staged) return;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   const int K1 = a.g.K[0], K2 = a.g.K[1], x0 = r.bx * TG_GB, y0 = r.by * TG_GB;
   const float2 *gs = ck + (long long)r.slice * a.grid_elems + chunk * TCW;
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(TG_THREADS, TgShape<TCW>::CTAS_PER_SM)
     for (int k = 0; k < 2; k++) {
       const long long i = it0 + blockIdx.x + (long long)k * gridDim.x;
       if (i < end)
-        stage_issue<TCW>(&tmap, a, ck, g.orec, smem + k * STAGE, &bar[k], &hdr[k], item_of(g, a, __ldg(g.item + i)),
+        stage_issue<TCW>(&tmap, a, ck, g.orec, smem + k * STAGE, &bar[k], &hdr[k], item_of<TCW>(g, a, __ldg(g.item + i)),
                          chunk, no_copy);
     }
   // the warps take their turns round robin over all items' samples
@@ -324,7 +329,30 @@ __global__ void __launch_bounds__(TG_THREADS, TgShape<TCW>::CTAS_PER_SM)
       }
       store(q, detail::cacc_get<false>(s2));
     };
-    if (SPW == 1) {
+    if (!r.staged) {
+      // a wrapped tile of few samples: their taps from the grid
+      const float2 *gs = ck + (long long)r.slice * a.grid_elems + (on ? c : 0);
+      const int K1 = a.g.K[0], K2 = a.g.K[1];
+      for (int q = wr * SPW + sub; q < r.n; q += NWARP * SPW) {
+        const int4 k0 = Kst[q];
+        const float2 *Ws = Wst + q * 12;
+        int xo[6];
+#pragma unroll
+        for (int j = 0; j < 6; j++) xo[j] = detail::tap_k(k0.x, j, K1) * C;
+        detail::CAcc s2;
+        detail::cacc_zero(s2);
+#pragma unroll
+        for (int j2 = 0; j2 < 6; j2++) {
+          const float2 *row = gs + detail::tap_k(k0.y, j2, K2) * (K1 * C);
+          detail::CAcc s1;
+          detail::cacc_zero(s1);
+#pragma unroll
+          for (int j1 = 0; j1 < 6; j1++) detail::cacc_mac<REAL>(s1, Ws[j1], __ldg(row + xo[j1]));
+          detail::cacc_mac<false>(s2, Ws[6 + j2], detail::cacc_get<REAL>(s1));
+        }
+        store(q, detail::cacc_get<false>(s2));
+      }
+    } else if (SPW == 1) {
       // neighbours in pairs: within a block the samples are sorted by first row, then
       // first column, so most neighbours share most of their tile rows
       for (int q = 2 * wr; q < r.n; q += 2 * NWARP) {
@@ -356,7 +384,7 @@ __global__ void __launch_bounds__(TG_THREADS, TgShape<TCW>::CTAS_PER_SM)
     // release the stage; the last warp out refills it with item k + 2
     if (stage_release(&done[s], NWARP) && i2 < end)
       stage_issue<TCW>(&tmap, a, ck, g.orec, smem + s * STAGE, &bar[s], &hdr[s],
-                       item_of(g, a, it2), chunk, no_copy);
+                       item_of<TCW>(g, a, it2), chunk, no_copy);
   }
 }
 
@@ -628,6 +656,18 @@ bool gather_tma_ok(const InterpArgs &a) {
   for (int d = 0; d < 2; d++)
     if (a.g.J[d] != 6 || a.g.K[d] < TG_TW) return false;
   return true;
+}
+
+// Whether the staged gather of the items is the default: from 32 columns on always.
+// Below, a tile of 16 columns costs the same for one sample as for many, and the second
+// one is partly idle, while the plain gather goes by samples and columns.  Samples an
+// item from which it was faster over 64^2 .. 1024^2, 1 and 8 slices, uniform, radial and
+// centred: 16 columns 2 (1.4 samples: 29 us against 18, 3.3: 18 and 18), 26 to 30 columns
+// 9 (6.8: 144 and 118, 9 to 14: 0.75 to 0.95 of the plain one's time), 20 to 24 columns 14
+// (9 to 14: 1.2 to 0.8, 14 to 20: 0.8), 18 columns 32 (20 to 32: 1.2 to 0.7).
+bool gather_tma_default(const InterpArgs &a, long long nitem) {
+  const int per = a.C >= 32 ? 0 : a.C == 16 ? 2 : a.C < 20 ? 32 : a.C < 26 ? 14 : 9;
+  return a.Mtot >= per * nitem;
 }
 
 int gather_tma_block() { return TG_GB; }

@@ -206,6 +206,7 @@ cudaError_t launch_sweep3_list(const InterpArgs &a, const Tiling &t, const int *
                                int B3, long long nblock, const long long *off, int *count, int *pos,
                                unsigned char *line, cudaStream_t st);
 bool gather_tma_ok(const InterpArgs &a);
+bool gather_tma_default(const InterpArgs &a, long long nitem);
 int gather_tma_block();
 int gather_tma_item();
 bool gather_tma3_ok(const InterpArgs &a);

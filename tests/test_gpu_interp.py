@@ -778,6 +778,52 @@ def test_3d_gather_time_follows_the_coil_chunks(C):
     assert ms[C] <= 1.3 * -(-C // 8) * ms[8], ms
 
 
+@pytest.mark.parametrize("C", [16, 18, 34, 40, 64])
+def test_tma_gather_of_wrapped_tiles_by_their_samples(C):
+    """Wrapped tiles of one to 30 samples, around the number from which they are copied to
+    shared memory, at the grid's right end, its top and its corner: the plain gather's bits."""
+    import torch
+    rng = np.random.default_rng(C)
+    K = [40, 48]
+    slices = []
+    for n in (1, 2, 22, 23, 24, 25, 30):
+        corner = np.array([[36.0, 20.0], [20.0, 44.0], [36.0, 44.0], [12.0, 20.0]])
+        slices.append(np.concatenate([c + rng.uniform(0, 2, (n, 2)) for c in corner]))
+    if C < 32:  # samples enough for the tiles to be the default
+        slices.append(rng.uniform(8, 30, (6000, 2)))
+    moff = np.concatenate([[0], np.cumsum([len(s) for s in slices])])
+    plan = mb.InterpPlan(K, [6, 6], [64, 64], [mb.newfft_kb_table(6, 64)] * 2,
+                         np.concatenate(slices), C, order=1, slice_moff=moff)
+    assert plan.config()["gather_tma"] == (2 if C < 32 else 1)
+    ck = torch.randn(plan.grid_shape, dtype=torch.complex64, device="cuda")
+    got = {mode: plan.forward(ck) for mode in ((None,) if C < 32 else (None, 2))
+           if mode is None or plan.set_gather(mode)}
+    plan.set_gather(False)
+    ref = plan.forward(ck)
+    assert all(torch.equal(g, ref) for g in got.values())
+    assert plan.fault() == 0
+    plan.close()
+
+
+@pytest.mark.parametrize("C,sparse,dense", [(16, 1000, 30000), (18, 20000, 200000), (20, 8000, 60000),
+                                            (24, 8000, 60000), (30, 5000, 40000)])
+def test_gather_of_16_to_30_columns_by_density(C, sparse, dense):
+    """Few samples a block of 8 x 8 first taps (1024 blocks): the plain gather, which goes by samples
+    and columns; many: the staged tiles; the autotuner may choose the tiles for either."""
+    import torch
+    rng = np.random.default_rng(C)
+    for M, tma in ((sparse, 0), (dense, 2)):
+        tm = rng.uniform(-128, 128, (M, 2))
+        plan = mb.InterpPlan([256, 256], [6, 6], [64, 64], [mb.newfft_kb_table(6, 64)] * 2, tm, C,
+                             order=1)
+        assert plan.config()["gather_tma"] == tma
+        ck = torch.randn(plan.grid_shape, dtype=torch.complex64, device="cuda")
+        a = plan.forward(ck)
+        assert plan.autotune()["gather_tma"] in (0, 2)
+        assert torch.equal(plan.forward(ck), a)
+        plan.close()
+
+
 @pytest.mark.parametrize("order", [0, 1])
 def test_tma_gather_3d_real_tables(order):
     """3D TMA gather with real tables (order 0 and 1): the plain 3D gather's
