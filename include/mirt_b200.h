@@ -243,10 +243,11 @@ int mirt_interp_plan_autotune(mirt_interp_plan *plan, void *stream);
  *  row-sweep dense-bin patches, staged row sweep mode, lane shape of the point
  *  spread (0: off), split spread}.  The point spread is the default where the
  *  sweeps are not, the split spread (the staged row sweep with the point spread
- *  on dense tiles) in 2D from 25 columns; mirt_interp_plan_set_sweep,
- *  _set_spread and _set_ownership turn them off, and where the row sweep is
- *  selected beneath the split spread (32 columns and more) so do _set_dense and
- *  _set_staged. */
+ *  on dense tiles) in 2D from 25 columns; from 32 columns the samples' number and
+ *  density choose between the split spread, the point spread alone and the row
+ *  sweep.  mirt_interp_plan_set_sweep, _set_spread and _set_ownership turn the
+ *  point and the split spread off, and where the row sweep is selected beneath
+ *  them (32 columns and more) so do _set_dense and _set_staged. */
 int mirt_interp_plan_config(mirt_interp_plan *plan, int32_t *out, int32_t n);
 
 /* Adjoint accumulation order.  deterministic = 1 (the default): every

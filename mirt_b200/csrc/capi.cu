@@ -435,6 +435,7 @@ int build_dense(mirt_interp_plan *P, int minc, cudaStream_t st) {
   t.chunk0 = 0;
   t.nchunks = 0;
   P->dense_slice.assign(t.nslice + 1, 0);
+  P->dense_samples = 0;
   // (a chunk's sample rows are staged in shared memory: at most 256 columns)
   if (minc <= 0 || a.C == 0 || a.C > 256) return MIRT_OK;
   const long long nb = (long long)t.nbins * t.nslice;
@@ -444,7 +445,10 @@ int build_dense(mirt_interp_plan *P, int minc, cudaStream_t st) {
   std::vector<int> db;
   for (long long b = 0; b < nb; b++) {
     if (b % t.nbins == 0) P->dense_slice[b / t.nbins] = (int)db.size();
-    if (bs[b + 1] - bs[b] >= minc) db.push_back((int)b);
+    if (bs[b + 1] - bs[b] >= minc) {
+      db.push_back((int)b);
+      P->dense_samples += bs[b + 1] - bs[b];
+    }
   }
   P->dense_slice[t.nslice] = (int)db.size();
   if (db.empty()) return MIRT_OK;
@@ -689,6 +693,41 @@ int build_sweep_records(mirt_interp_plan *P, cudaStream_t st) {
   return MIRT_OK;
 }
 
+// The default spread of 2D plans of 32 columns and more.  The row sweep with dense-bin
+// patches sums a bin of many samples once for all its rows, steps through every column
+// and ends with its heaviest team; the split spread visits a sample 2.25 times, the dense
+// tiles point by point, in two launches; the point spread alone is one, and cuts dense
+// bricks up.  Against the row sweep and the split spread as the only choice, over 1,119
+// plans (64^2 .. 1024^2, 32 to 128 columns, 1 to 16 slices, uniform, radial and centred,
+// 0.01 to 10 samples a point): 1.63 and 1.17 times as fast in the geometric mean, 0.91
+// and 0.74 at worst.
+enum class Spread2D { row, points, split };
+
+Spread2D choose_spread2d(const mirt_interp_plan *P, const std::vector<int> &most, int dense) {
+  const InterpArgs &a = P->a;
+  const double M = (double)a.Mtot, chunks = (a.C + 31) / 32;
+  // a fifth of the samples in dense bins: the split spread at 0.6 to 0.8 of the row
+  // sweep's speed, with up to 64,000 such samples at 0.9 to 2.5
+  if (P->dense_samples > 0.2 * M)
+    return P->dense_samples > 60000 ? Spread2D::row : Spread2D::split;
+  // few samples on a small grid: the point spread twice the row sweep's speed, and never
+  // behind it up to 16,000; large sparse grids pass the split spread's bands faster
+  const double cells = (double)P->t.nslice * a.g.K[0] * a.g.K[1] * chunks;
+  if (M <= 16000 && cells <= 2e6) return Spread2D::points;
+  double in_dense = 0, all = 0;
+  int largest = 0;
+  for (int m : most) {
+    all += m;
+    if (m > dense) in_dense += m;
+    largest = std::max(largest, m);
+  }
+  if (in_dense < 0.5 * all) return Spread2D::split;
+  // even grids whose every tile is dense against a small total: the row sweep (1.1 ns a
+  // sample and chunk, the point spread 1.4) if its heaviest team, a fifth of a microsecond
+  // a visit to at most 15 samples a bin, does not outlast the rest
+  return M * chunks > 200.0 * std::min(largest, 81 * kDenseBin) ? Spread2D::row : Spread2D::points;
+}
+
 // Split spread: the plane's tiles that a band's segment could not share out
 // evenly go to the point spread, which splits them over groups and CTAs; the
 // bands of four rows between them are cut into segments of about a quarter of a
@@ -713,6 +752,12 @@ int build_split(mirt_interp_plan *P, cudaStream_t st) {
   for (float v : vb) total += v + kSweepColumnCost;
   const double share = std::max(1.0, total * nch / kWarps);
   const int dense = (int)std::min(kSplitMost, std::max(64.0, kSplitDense * share));
+  const Spread2D form = P->ls.cw == 32 ? choose_spread2d(P, most, dense)
+                                       : Spread2D::split;
+  if (form == Spread2D::points) {
+    P->points_shape = shape;
+    return build_point_tasks(P, shape, most, -1, st);
+  }
   const double target = std::max(32.0, share / kSplitTeams);
   std::vector<int4> tk;
   std::vector<double> cost;
@@ -762,7 +807,9 @@ int build_split(mirt_interp_plan *P, cudaStream_t st) {
   t.split_next = P->split_next.as<int>();
   rc = build_point_tasks(P, shape, most, dense, st);
   if (rc) return rc;
-  P->split_ok = 1;
+  P->split_ok = 1;  // (the autotuner tries it where it is not the default)
+  t.split = form == Spread2D::split;
+  if (!t.split) t.points = 0;
   return MIRT_OK;
 }
 
@@ -1322,7 +1369,6 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     int rc3 = build_sweep_records(P, st);
     if (!rc3) rc3 = build_split(P, st);
     if (rc3) return rc3;
-    P->t.split = P->split_ok;
   }
   // 3D, J = 6, coil chunks of 8, 16 or 32: the line sweep, two segments per line
   if (sweep3_ok(a, P->t, P->ls.cw)) {
@@ -1337,7 +1383,7 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     int rc3 = build_points(P, st);
     if (rc3) return rc3;
   }
-  return P->t.sweep < 0 && !P->t.split ? sweep_teams_ready(P, st) : MIRT_OK;
+  return P->t.sweep < 0 && !P->t.points ? sweep_teams_ready(P, st) : MIRT_OK;
 }
 
 // Re-tile the spread (tiles of T[d] points, multiples of the sort bins) and
@@ -1435,9 +1481,9 @@ int validate_geometry(int D, const int *K, const int *J, const int *L, int order
 // The plan whose launches a setter tunes: a 4D plan's 3D plan, else the plan.
 static mirt_interp_plan *launch_plan(mirt_interp_plan *P) { return P->sub4 ? P->sub4 : P; }
 
-// A row-sweep setting was chosen: the row sweep itself, not the split spread.
+// A row-sweep setting was chosen: the row sweep itself, not the spread on top of it.
 static int leave_split(mirt_interp_plan *P) {
-  if (!P->t.sweep || !P->t.split) return MIRT_OK;
+  if (!P->t.sweep || !P->t.points) return MIRT_OK;
   P->t.points = P->t.split = 0;
   return sweep_teams_ready(P, as_stream(nullptr));
 }
@@ -1626,7 +1672,8 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
   if (sweep3_ok(a, P->t, cw) && sweep_buffer(P) == MIRT_OK)
     cands.push_back(SpreadCand{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, 2, 1});
   if (P->points_shape) {
-    SpreadCand c{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, 0, 1};
+    SpreadCand c{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0,
+                 sweep_ok(a, P->t) && cw == 32 ? -1 : 0, 1};
     c.points = P->points_shape;
     cands.push_back(c);
   }
@@ -3405,7 +3452,7 @@ int mirt_nufft_config(mirt_nufft *p, int32_t *out, int32_t n) {
   int spread = 1;  // the point spread: one launch
   if (t.split) {
     spread = (t.split_nteams > 0) + (t.n_pt_task > 0);
-  } else if (t.points && !p->ip->ls.atomic) {
+  } else if (t.points && (t.sweep || !p->ip->ls.atomic)) {
   } else if (t.sweep != 0) {
     // ordering pass, dense-bin patches (chunk sums, per-bin sums), sweep (and a
     // memset of the queue counters)

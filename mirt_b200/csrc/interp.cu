@@ -344,7 +344,7 @@ cudaError_t launch_spread(const InterpArgs &a, const Tiling &t, const Launch &l,
     }
     return launch_spread_points(a, t, bin_start, fm, ck, st);
   }
-  if (t.points && !l.atomic) return launch_spread_points(a, t, bin_start, fm, ck, st);
+  if (t.points && (t.sweep || !l.atomic)) return launch_spread_points(a, t, bin_start, fm, ck, st);
   detail::Req r{detail::SPREAD, &a, &t, &lc, bin_start, fm, ck, st};
   return dispatch(r);
 }

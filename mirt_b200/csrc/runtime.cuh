@@ -84,6 +84,7 @@ struct mirt_interp_plan {
   mirt::DMem dense_of, dense_bin, patch;  // the sweeps' dense bins and their patches
   mirt::DMem dense_chunk, dense_part0, patch_part;  // chunks of the patch sums
   std::vector<int> dense_slice;           // first dense bin of each slice (+ total)
+  long long dense_samples = 0;            // samples in dense bins
   std::vector<int> dense_part0_host;      // first chunk of each dense bin (+ total)
   // TMA gather: first position of each block of the gather order, work items
   // (block, first position, samples), the first item of each slice, fault flag

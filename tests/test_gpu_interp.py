@@ -1096,6 +1096,49 @@ def test_point_spread_of_wide_kernels(K, J, C):
     plan.close()
 
 
+@pytest.mark.parametrize("C", [32, 34, 64])
+@pytest.mark.parametrize("kind,K,M,form", [
+    ("even", (64, 48), 0, "points"), ("even", (64, 48), 4000, "points"), ("even", (128, 128), 16000, "points"),
+    ("even", (256, 200), 16001, "split"), ("even", (64, 48), 20000, "points"),
+    ("even", (200, 150), 40000, "row"), ("dense", (96, 80), 70000, "row"),
+    ("dense", (96, 80), 60000, "split"), ("radial", (512, 512), 204800, "split"),
+])
+def test_default_spread_of_32_columns(C, kind, K, M, form):
+    """The default of 2D plans of 32 columns and more by the samples in dense bins and in dense
+    tiles: the point spread alone, the split spread or the row sweep; each the oracle's adjoint,
+    the same bits again, and the row sweep when a row-sweep setting is chosen."""
+    import torch
+    rng = np.random.default_rng(M + C)
+    if kind == "even":
+        tm = rng.uniform(-1, 1, (M, 2)) * np.array(K)
+    elif kind == "dense":                       # nine tenths of them within a few points
+        tm = np.concatenate([rng.uniform(-5, 5, (M - M // 10, 2)), rng.uniform(-90, 90, (M // 10, 2))])
+    else:
+        tm = _radial(M // 512, 512) * 512 / (2 * np.pi)
+    h = [mb.newfft_kb_table(6, 64)] * 2
+    plan = mb.InterpPlan(list(K), [6, 6], [64, 64], h, tm, C, order=1)
+    cfg = plan.config()
+    assert cfg["spread_sweep"] == -1
+    got = "split" if cfg["spread_split"] else "points" if cfg["spread_points"] else "row"
+    assert got == form
+    fm = rng.standard_normal((len(tm), C)) + 1j * rng.standard_normal((len(tm), C))
+    fd = torch.from_numpy(fm.astype(np.complex64)).cuda()
+    out = plan.adjoint(fd)
+    assert torch.equal(out, plan.adjoint(fd))
+    plan.set_staged(2)
+    assert plan.config()["spread_points"] == 0 and plan.config()["spread_split"] == 0
+    row = plan.adjoint(fd).cpu().numpy()
+    out = out.cpu().numpy()
+    if M:
+        cols = [0, C - 1]
+        ref = oracle.interp_adj(fm[:, cols], h, [6, 6], [64, 64], tm, list(K), 1, impl=ref_impl())
+        for o in (out, row):
+            assert rel_l2(np.transpose(o[0], (1, 0, 2)).reshape(-1, C, order="F")[:, cols], ref) <= ADJ_TOL
+    else:
+        assert not out.any() and not row.any()
+    plan.close()
+
+
 def _taps_of(t, J, K):
     """Mask [K_D, ..., K_1] of the grid points that a sample at t reaches."""
     m = np.ones((), bool)
