@@ -939,10 +939,13 @@ cudaError_t launch_dense_patches(const InterpArgs &a, const Tiling &t, const flo
   k1<<<(unsigned)t.nchunks, threads, sm, st>>>(a, t, fs);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  // an entry a thread: one block a bin took as long as the central bin's chunks, read
-  // seven times over (kooshball of 8 coils: 236 us, 122 us so)
+  // 3D: an entry a thread; one block a bin took as long as the central bin's chunks, read
+  // seven times over (kooshball of 8 coils: 236 us, 122 us so).  2D: a block a bin, whose
+  // 36 C entries are few and whose bins are many (400^2, 32 coils, 1.6 M centred samples:
+  // the whole adjoint 1,145 us with five blocks a bin, 1,082 us so)
   const long long pn = (long long)(D == 3 ? 216 : 36) * a.C;
-  dense_reduce_kernel<D><<<dim3((unsigned)t.ndense, (unsigned)((pn + 255) / 256)), 256, 0, st>>>(a, t);
+  const unsigned per_bin = D == 3 ? (unsigned)((pn + 255) / 256) : 1u;
+  dense_reduce_kernel<D><<<dim3((unsigned)t.ndense, per_bin), 256, 0, st>>>(a, t);
   return cudaGetLastError();
 }
 
