@@ -1954,10 +1954,9 @@ int mirt_interp_plan_set_ownership(mirt_interp_plan *P, int32_t own, void *strea
     return fail(MIRT_ERR_ARG, "ownership spread needs 2D, J = 6, tiles of >= 5 points and an "
                               "even number of tiles (last one >= 5 points) per dimension");
   P->t.own = own ? 1 : 0;
-  P->t.points = P->t.split = 0;
-  if (own) {
+  if (own) {  // (off leaves another spread as it is)
     P->ls.atomic = 0;
-    P->t.sweep = 0;
+    P->t.sweep = P->t.points = P->t.split = 0;
   }
   int T[MIRT_DMAX] = {P->t.T[0], P->t.T[1], P->t.T[2]};
   int rc = set_spread_tiles(P, T, as_stream(stream));

@@ -1139,6 +1139,34 @@ def test_default_spread_of_32_columns(C, kind, K, M, form):
     plan.close()
 
 
+@pytest.mark.parametrize("K,C,M", [((64, 48), 8, 3000), ((41, 50), 32, 7500), ((96, 80), 40, 1000),
+                                   ((64, 60), 26, 5000)])
+def test_ownership_off_leaves_the_spread(K, C, M):
+    """set_ownership(False) on a plan whose spread is another one changes nothing; after
+    set_ownership(True) it is the tiled spread."""
+    import torch
+    rng = np.random.default_rng(C)
+    tm = np.concatenate([rng.uniform(-60, 60, (M // 2, 2)), rng.uniform(-3, 3, (M - M // 2, 2))])
+    h = [mb.newfft_kb_table(6, 64)] * 2
+    plan = mb.InterpPlan(list(K), [6, 6], [64, 64], h, tm, C, order=1)
+    fm = rng.standard_normal((M, C)) + 1j * rng.standard_normal((M, C))
+    fd = torch.from_numpy(fm.astype(np.complex64)).cuda()
+    cfg, out = plan.config(), plan.adjoint(fd)
+    plan.set_ownership(False)
+    assert plan.config() == cfg
+    got = torch.full_like(out, float("nan"))
+    assert torch.equal(plan.adjoint(fd, out=got), out)
+    ref = oracle.interp_adj(fm, h, [6, 6], [64, 64], tm, list(K), 1, impl=ref_impl())
+    assert rel_l2(np.transpose(out.cpu().numpy()[0], (1, 0, 2)).reshape(-1, C, order="F"), ref) <= ADJ_TOL
+    if all(k % 16 == 0 for k in K):             # an even number of 8-point tiles per dimension
+        plan.set_spread((8, 8))
+        plan.set_ownership(True)
+        plan.set_ownership(False)
+        assert plan.config()["spread_own"] == plan.config()["spread_sweep"] == 0
+        assert rel_l2(plan.adjoint(fd).cpu().numpy(), out.cpu().numpy()) <= 5e-6
+    plan.close()
+
+
 def _taps_of(t, J, K):
     """Mask [K_D, ..., K_1] of the grid points that a sample at t reaches."""
     m = np.ones((), bool)
