@@ -637,11 +637,27 @@ int build_point_tasks(mirt_interp_plan *P, int shape, const std::vector<int> &mo
       task[at[lg[i]]++] = e;
     }
   const size_t nch = points_chunks(shape, a.C);
+  // the same tasks grouped by slice, for the slice ranges of the host-buffer adjoint
+  std::vector<int4> by_slice;
+  P->pt_slice.clear();
+  if (t.nslice > 1 && t.sweep) {
+    const long long per = n / t.nslice;
+    std::vector<long long> first(t.nslice + 1, 0);
+    for (const int4 &e : task) first[e.x / per + 1]++;
+    for (int s = 0; s < t.nslice; s++) first[s + 1] += first[s];
+    P->pt_slice = first;
+    by_slice.resize(total);
+    for (const int4 &e : task) by_slice[first[e.x / per]++] = e;
+  }
   CK(P->pt_task.alloc(std::max<long long>(total, 1) * sizeof(int4)));
+  CK(P->pt_slice_task.alloc(by_slice.size() * sizeof(int4)));
   CK(P->pt_scratch.alloc(slots * nch * points_slot_bytes(shape)));
   CK(P->pt_count.alloc(slots * nch * sizeof(int)));
   if (total)
     CK(cudaMemcpyAsync(P->pt_task.p, task.data(), total * sizeof(int4), cudaMemcpyHostToDevice, st));
+  if (!by_slice.empty())
+    CK(cudaMemcpyAsync(P->pt_slice_task.p, by_slice.data(), by_slice.size() * sizeof(int4),
+                       cudaMemcpyHostToDevice, st));
   if (slots) CK(cudaMemsetAsync(P->pt_count.p, 0, slots * nch * sizeof(int), st));
   CK(cudaStreamSynchronize(st));
   t.points = shape;
@@ -791,18 +807,35 @@ int build_split(mirt_interp_plan *P, cudaStream_t st) {
         }
       }
     }
-  std::vector<int> order(tk.size());
-  for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+  // the teams lie slice after slice, heaviest first in each; a launch over all slices
+  // takes them heaviest first by split_order, one over a range in place
+  std::vector<int> place(tk.size()), order(tk.size());
+  for (size_t k = 0; k < place.size(); k++) place[k] = order[k] = (int)k;
+  std::stable_sort(place.begin(), place.end(), [&](int x, int y) {
+    return tk[x].x != tk[y].x ? tk[x].x < tk[y].x : cost[x] > cost[y];
+  });
   std::vector<int4> sorted(tk.size());
-  for (size_t i = 0; i < order.size(); i++) sorted[i] = tk[order[i]];
+  P->split_slice.assign(t.nslice + 1, 0);
+  for (size_t k = 0; k < place.size(); k++) {
+    sorted[k] = tk[place[k]];
+    P->split_slice[sorted[k].x + 1] = (int)k + 1;
+  }
+  for (int s = 0; s < t.nslice; s++)
+    P->split_slice[s + 1] = std::max(P->split_slice[s], P->split_slice[s + 1]);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int x, int y) { return cost[place[x]] > cost[place[y]]; });
   CK(P->split_teams.alloc(std::max<size_t>(sorted.size(), 1) * sizeof(int4)));
+  CK(P->split_order.alloc(std::max<size_t>(sorted.size(), 1) * sizeof(int)));
   CK(P->split_next.alloc((size_t)nch * sizeof(int)));
-  if (!sorted.empty())
+  if (!sorted.empty()) {
     CK(cudaMemcpyAsync(P->split_teams.p, sorted.data(), sorted.size() * sizeof(int4),
                        cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(P->split_order.p, order.data(), order.size() * sizeof(int),
+                       cudaMemcpyHostToDevice, st));
+  }
   CK(cudaStreamSynchronize(st));
   t.split_team = P->split_teams.as<int4>();
+  t.split_order = P->split_order.as<int>();
   t.split_nteams = (int)sorted.size();
   t.split_next = P->split_next.as<int>();
   rc = build_point_tasks(P, shape, most, dense, st);
@@ -897,6 +930,7 @@ void choose_config(mirt_interp_plan *P) {
   t.sweep_rows = 1;
   t.split = 0;
   t.split_team = nullptr;
+  t.split_order = nullptr;
   t.split_nteams = 0;
   t.split_next = nullptr;
   t.points = 0;
@@ -3233,14 +3267,23 @@ int nufft_forward_range(mirt_nufft *p, int s0, int s1, const float2 *x, float2 *
   return MIRT_OK;
 }
 
-// Slices [s0, s1) of the adjoint NUFFT (row-sweep spread) on the full-size
-// buffers.
+// Slices [s0, s1) of the adjoint NUFFT on the full-size buffers: the spread of the
+// device call over the slices' tasks, teams or parts, the same sums.
 int nufft_adjoint_range(mirt_nufft *p, int s0, int s1, const float2 *X, float2 *x,
                         cufftHandle fft, cudaStream_t st) {
   mirt_interp_plan *P = p->ip;
   Tiling t = P->t;
-  t.points = t.split = 0;
-  if (t.sweep < 0) t.sweep = 2;  // a chunk: uniform halves of rows (same sums)
+  if (t.points) {                // the chunk's point tasks and split teams
+    t.pt_task = P->pt_slice_task.as<int4>() + P->pt_slice[s0];
+    t.n_pt_task = (int)(P->pt_slice[s1] - P->pt_slice[s0]);
+    if (t.split) {
+      t.split_team += P->split_slice[s0];
+      t.split_nteams = P->split_slice[s1] - P->split_slice[s0];
+      t.split_order = nullptr;
+    }
+  } else if (t.sweep < 0) {
+    t.sweep = 2;                 // the row sweep: uniform halves of rows
+  }
   t.team_order = nullptr;        // the chunk's teams in index order
   if (t.ndense > 0) {            // the chunk's dense bins and their sample chunks
     t.dense0 = P->dense_slice[s0];
@@ -3343,7 +3386,8 @@ int host_pipelined(mirt_nufft *p, const float *in, float *out, cudaStream_t st) 
   return MIRT_OK;
 }
 
-// the chunked path needs several slices and, for the adjoint, the row sweep
+// the chunked path needs several slices and, for the adjoint, a sweep (or the point
+// spread on top of one)
 bool host_pipeline_ok(const mirt_nufft *p, bool fwd) {
   return p->nslice > 1 && p->C > 0 && (fwd || p->ip->t.sweep != 0);
 }

@@ -335,7 +335,7 @@ cudaError_t launch_spread(const InterpArgs &a, const Tiling &t, const Launch &l,
       ts.dense_on = 0;
       ts.sweep_team = t.split_team;
       ts.nteams = t.split_nteams;
-      ts.team_order = nullptr;
+      ts.team_order = t.split_order;
       ts.team_next = t.split_next;
       lc.cw = 32;
       detail::Req r{detail::SPREAD, &a, &ts, &lc, bin_start, fm, ck, st};

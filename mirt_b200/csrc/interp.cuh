@@ -131,10 +131,12 @@ struct Tiling {
   int *pt_count;
   const int4 *pt_hdr;    // per position: first tap k1, caller's sample index, phase (float bits)
   // Split spread (2D, J = 6, many columns): the staged row sweep over the team
-  // list `split_team` (bands of four rows, segments of their columns, heaviest
-  // first), which leaves out the dense tiles; the point spread's tasks are those
+  // list `split_team` (bands of four rows, segments of their columns, slice after
+  // slice; split_order: heaviest first, null in place), which leaves out the dense
+  // tiles; the point spread's tasks are those
   int split;             // 0: off
   const int4 *split_team;
+  const int *split_order;
   int split_nteams;
   int *split_next;       // its queue counters, one per chunk of 32 columns
   int color_beg[9];

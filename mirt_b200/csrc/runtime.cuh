@@ -78,7 +78,10 @@ struct mirt_interp_plan {
   std::vector<int> s3_slice_part, s3_slice_fix;
   mirt::DMem team_order, team_next;  // row-sweep work queue: heaviest-first order, counter
   mirt::DMem pt_task, pt_hdr, pt_scratch, pt_count;  // point spread (Tiling)
-  mirt::DMem split_teams, split_next;                // split spread (Tiling)
+  mirt::DMem pt_slice_task;            // the point tasks slice after slice, and the first
+  std::vector<long long> pt_slice;     // of each slice (+ total); empty without a sweep
+  mirt::DMem split_teams, split_order, split_next;   // split spread (Tiling)
+  std::vector<int> split_slice;        // first split team of each slice (+ total)
   int split_ok = 0;                  // 1: the plan has the split spread's lists
   int points_shape = 0;              // its lane shape (0: the plan has none)
   mirt::DMem dense_of, dense_bin, patch;  // the sweeps' dense bins and their patches

@@ -310,6 +310,35 @@ def test_grids_through_cufft(N, K, C):
     plan.close()
 
 
+@pytest.mark.parametrize("form,C,nslice", [("points", 32, 3), ("split", 32, 9), ("split", 34, 11),
+                                            ("split", 40, 2), ("row", 32, 4)])
+def test_host_adjoint_gives_the_device_adjoints_bits(form, C, nslice):
+    """The host-buffer adjoint of several slices runs the device adjoint's spread over slice
+    ranges: the same bits, for each of the default spreads, with an empty slice, uneven ones and
+    dense centres that several blocks share."""
+    import torch
+    rng = np.random.default_rng(C + nslice)
+    N, K = (64, 50), (128, 100)
+    M = {"points": 2000, "split": 20000, "row": 40000}[form]
+    counts = rng.integers(M // 2, M, nslice)
+    counts[1] = 0
+    moff = np.concatenate([[0], np.cumsum(counts)])
+    om = rng.uniform(-np.pi, np.pi, (int(moff[-1]), 2))
+    om[moff[0]:moff[0] + M // 6] *= 0.02
+    if form == "row":
+        om *= 0.08
+    plan = mb.NufftPlan(om, N, (6, 6), K, n_shift=(32, 25), Ld=256, ncol=C, slice_moff=moff)
+    cfg = plan.config()
+    assert form == ("split" if cfg["spread_split"] else "points" if cfg["spread_points"] else "row")
+    X = (rng.standard_normal(plan.sample_shape) + 1j * rng.standard_normal(plan.sample_shape))
+    X = X.astype(np.complex64)
+    dev = plan.adjoint(torch.from_numpy(X).cuda()).cpu().numpy()
+    for _ in range(2):
+        assert np.array_equal(plan.adjoint_host(X), dev)
+    assert np.array_equal(plan.adjoint(torch.from_numpy(X).cuda()).cpu().numpy(), dev)
+    plan.close()
+
+
 def test_host_calls_of_3d_slices():
     """Slice ranges of the 3D line sweep (its parts and tails by slice): the pipelined
     host adjoint against the device adjoint."""
