@@ -50,6 +50,12 @@ const char *mirt_last_error(void);
 /* Library version, major * 10000 + minor * 100 + patch. */
 int mirt_version(void);
 
+/* Test hook of the handling of failed device allocations: the process's n-th
+ * next one (0: the next) fails, negative: none.  Returns what was left of an
+ * earlier count, negative where it was used up or none was set.  No reference
+ * counterpart. */
+int mirt_test_fail_alloc(int32_t n);
+
 /* ------------------------------------------------------------------------
  * 1. mex gateway drop-ins
  *

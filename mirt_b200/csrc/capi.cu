@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include <atomic>
 #include <cmath>
 #include <complex>
 #include <algorithm>
@@ -112,6 +113,7 @@ int api_fail(int code, const std::string &msg) { return fail(code, msg); }
 namespace {
 std::mutex g_cache_mu;
 std::multimap<std::pair<int, size_t>, void *> g_free;
+std::atomic<int> g_alloc_left{-1};  // mirt_test_fail_alloc
 }  // namespace
 
 size_t round_block(size_t b) {
@@ -123,6 +125,7 @@ size_t round_block(size_t b) {
 cudaError_t dalloc(void **p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) return cudaSuccess;
+  if (g_alloc_left >= 0 && g_alloc_left-- == 0) return cudaErrorMemoryAllocation;
   int dev = 0;
   cudaGetDevice(&dev);
   const size_t r = round_block(bytes);
@@ -143,6 +146,7 @@ cudaError_t dalloc(void **p, size_t bytes) {
     for (auto &kv : g_free) cudaFree(kv.second);
     g_free.clear();
     e = cudaMalloc(p, r);
+    if (e != cudaSuccess) cudaGetLastError();
   }
   return e;
 }
@@ -249,13 +253,6 @@ int sweep_buffer(mirt_interp_plan *P) {
   return MIRT_OK;
 }
 
-// Balanced row-sweep teams: each band of `rows` grid rows of each slice is
-// cut into column segments of about equal cost, cost = visits (samples of the
-// rows + 5 bin rows in the segment's columns and its five warm-up columns)
-// + 2 per column step; segments of at least 8 columns, about `target` teams
-// in all, in grid order (neighbouring bands read the same samples, so they
-// run together; heaviest-first order measured slower at full size).  Teams
-// write disjoint points, each summed in the same fixed order.
 // Columns from which the split spread is the default (2D, J = 6): its sweep's
 // lanes are 32 columns whatever their use, while the point spread's chunks fit
 // the columns (20 columns, 115,968 samples on 384^2: 151 against 139 us; 24
@@ -321,58 +318,14 @@ double sweep_team_cost(const float *v, int K1, int x0, int x1) {
   return c;
 }
 
-// The sweep's work queue: teams heaviest first (ties in index order), and the
-// queue counter.  Teams are the list (t.sweep < 0) or the uniform segments.
-int build_sweep_order(mirt_interp_plan *P, const std::vector<float> &vb, cudaStream_t st) {
-  const InterpArgs &a = P->a;
-  Tiling &t = P->t;
-  const int K1 = a.g.K[0], K2 = a.g.K[1], rows = t.sweep_rows;
-  const int nband = (K2 + rows - 1) / rows;
-  std::vector<int4> tk;
-  if (t.sweep < 0) {
-    tk = P->team_host;
-  } else {
-    const int nseg = t.sweep, sw = (K1 + nseg - 1) / nseg;
-    for (int s = 0; s < t.nslice; s++)
-      for (int bi = 0; bi < nband; bi++)
-        for (int g = 0; g < nseg; g++)
-          tk.push_back(make_int4(s, bi * rows, g * sw, std::min(K1, g * sw + sw)));
-  }
-  std::vector<double> cost(tk.size());
-  for (size_t i = 0; i < tk.size(); i++) {
-    const int4 k = tk[i];
-    cost[i] = k.z < k.w ? sweep_team_cost(vb.data() + ((size_t)k.x * nband + k.y / rows) * K1, K1,
-                                          k.z, k.w)
-                        : 0.0;
-  }
-  std::vector<int> order(tk.size());
-  for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-  if (P->team_order.bytes < std::max<size_t>(order.size(), 1) * sizeof(int))
-    CK(P->team_order.alloc(std::max<size_t>(order.size(), 1) * sizeof(int)));
-  if (!order.empty())
-    CK(cudaMemcpyAsync(P->team_order.p, order.data(), order.size() * sizeof(int),
-                       cudaMemcpyHostToDevice, st));
-  // one queue counter per coil chunk
-  const size_t nq = (size_t)std::max(1, (a.C + P->ls.cw - 1) / std::max(P->ls.cw, 1));
-  if (P->team_next.bytes < nq * sizeof(int)) CK(P->team_next.alloc(nq * sizeof(int)));
-  CK(cudaStreamSynchronize(st));
-  t.team_order = P->team_order.as<int>();
-  t.team_next = P->team_next.as<int>();
-  return MIRT_OK;
-}
-
 // Balanced row-sweep teams: each band of `rows` grid rows of each slice is
 // cut into column segments of about equal cost (sweep_team_cost), segments of
-// at least 8 columns, about `target` teams in all.  Teams write disjoint
+// at least 8 columns, about `target` teams in all, in grid order (neighbouring
+// bands read the same samples, so they run together).  Teams write disjoint
 // points, each summed in the same fixed order.
-int build_sweep_teams(mirt_interp_plan *P, int rows, long long target, cudaStream_t st) {
-  const InterpArgs &a = P->a;
-  Tiling &t = P->t;
-  const int K1 = a.g.K[0], K2 = a.g.K[1], S = t.nslice;
-  std::vector<float> vb;
-  int rc = sweep_band_visits(P, rows, st, vb);
-  if (rc) return rc;
+std::vector<int4> balanced_teams(const mirt_interp_plan *P, int rows, long long target,
+                                 const std::vector<float> &vb) {
+  const int K1 = P->a.g.K[0], K2 = P->a.g.K[1], S = P->t.nslice;
   const double alpha = kSweepColumnCost;
   const int nband = (K2 + rows - 1) / rows;
   double total = 0;
@@ -399,27 +352,92 @@ int build_sweep_teams(mirt_interp_plan *P, int rows, long long target, cudaStrea
         x0 = x1;
       }
     }
-  if (P->sweep_teams.bytes < tk.size() * sizeof(int4)) CK(P->sweep_teams.alloc(tk.size() * sizeof(int4)));
-  CK(cudaMemcpyAsync(P->sweep_teams.p, tk.data(), tk.size() * sizeof(int4), cudaMemcpyHostToDevice,
-                     st));
-  CK(cudaStreamSynchronize(st));
-  P->team_host = tk;
-  t.sweep_team = P->sweep_teams.as<int4>();
-  t.nteams = (int)tk.size();
-  t.sweep = -1;
-  t.sweep_rows = rows;
-  return build_sweep_order(P, vb, st);
+  return tk;
 }
 
-// The balanced team list of the row sweep's default (one-row bands, about 64k
-// teams), made when it is first needed.
-int sweep_teams_ready(mirt_interp_plan *P, cudaStream_t st) {
-  if (P->t.sweep >= 0 || P->t.sweep_team) return MIRT_OK;
-  return build_sweep_teams(P, P->t.sweep_rows, 65536, st);
+// The row sweep's teams, the balanced list (nseg < 0, about 64k teams) or nseg uniform
+// segments, and its work queue: teams heaviest first (ties in index order) and the
+// queue counters.  Where it fails, the plan and its lists are as they were.
+int set_row_sweep(mirt_interp_plan *P, int nseg, int rows, cudaStream_t st) {
+  const InterpArgs &a = P->a;
+  Tiling &t = P->t;
+  const int K1 = a.g.K[0], K2 = a.g.K[1], nband = (K2 + rows - 1) / rows;
+  std::vector<float> vb;
+  int rc = sweep_band_visits(P, rows, st, vb);
+  if (rc) return rc;
+  std::vector<int4> tk;
+  if (nseg < 0) {
+    tk = balanced_teams(P, rows, 65536, vb);
+  } else {
+    const int sw = (K1 + nseg - 1) / nseg;
+    for (int s = 0; s < t.nslice; s++)
+      for (int bi = 0; bi < nband; bi++)
+        for (int g = 0; g < nseg; g++)
+          tk.push_back(make_int4(s, bi * rows, g * sw, std::min(K1, g * sw + sw)));
+  }
+  std::vector<double> cost(tk.size());
+  for (size_t i = 0; i < tk.size(); i++) {
+    const int4 k = tk[i];
+    cost[i] = k.z < k.w ? sweep_team_cost(vb.data() + ((size_t)k.x * nband + k.y / rows) * K1, K1,
+                                          k.z, k.w)
+                        : 0.0;
+  }
+  std::vector<int> order(tk.size());
+  for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+  // one queue counter per coil chunk
+  const size_t nq = (size_t)std::max(1, (a.C + P->ls.cw - 1) / std::max(P->ls.cw, 1));
+  DMem d_teams, d_order, d_next;
+  if (nseg < 0) CK(d_teams.alloc(std::max<size_t>(tk.size(), 1) * sizeof(int4)));
+  CK(d_order.alloc(std::max<size_t>(order.size(), 1) * sizeof(int)));
+  if (P->team_next.bytes < nq * sizeof(int)) CK(d_next.alloc(nq * sizeof(int)));
+  if (nseg < 0 && !tk.empty())
+    CK(cudaMemcpyAsync(d_teams.p, tk.data(), tk.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+  if (!order.empty())
+    CK(cudaMemcpyAsync(d_order.p, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice,
+                       st));
+  CK(cudaStreamSynchronize(st));
+  swap_mem(P->sweep_teams, d_teams);
+  swap_mem(P->team_order, d_order);
+  if (d_next.p) swap_mem(P->team_next, d_next);
+  t.sweep_team = nseg < 0 ? P->sweep_teams.as<int4>() : nullptr;
+  t.nteams = nseg < 0 ? (int)tk.size() : 0;
+  P->team_rows = nseg < 0 ? rows : 0;
+  t.team_order = P->team_order.as<int>();
+  t.team_next = P->team_next.as<int>();
+  t.sweep = nseg;
+  t.sweep_rows = rows;
+  return MIRT_OK;
+}
+
+// The patches of the plan's dense bins (J^D taps x C per dense bin) and of their chunks.
+int dense_patches(mirt_interp_plan *P) {
+  Tiling &t = P->t;
+  if (!t.dense_of || t.patch) return MIRT_OK;
+  const size_t taps = P->a.g.D == 3 ? 216 : 36;
+  CK(P->patch.alloc((size_t)t.ndense * taps * P->a.C * sizeof(float2)));
+  CK(P->patch_part.alloc((size_t)t.nchunks * taps * P->a.C * sizeof(float2)));
+  t.patch = P->patch.as<float2>();
+  t.patch_part = P->patch_part.as<float2>();
+  return MIRT_OK;
+}
+
+// What the row sweep needs beyond the plan: its copy of the samples and the patches.
+// Made when it is first selected: the spreads on top of it read neither.
+int row_buffers(mirt_interp_plan *P) {
+  int rc = sweep_buffer(P);
+  return rc ? rc : dense_patches(P);
+}
+
+// ... and, for its default (balanced teams), their list.
+int row_sweep_ready(mirt_interp_plan *P, cudaStream_t st) {
+  int rc = row_buffers(P);
+  if (rc || P->t.sweep >= 0 || P->team_rows == P->t.sweep_rows) return rc;
+  return set_row_sweep(P, P->t.sweep, P->t.sweep_rows, st);
 }
 
 // The sweeps' dense bins: bins with at least `minc` samples (0: none), their
-// index map and patch buffer (J^D taps x C per dense bin).
+// index map and the chunks of their sums (the patches: dense_patches).
 int build_dense(mirt_interp_plan *P, int minc, cudaStream_t st) {
   const InterpArgs &a = P->a;
   Tiling &t = P->t;
@@ -452,8 +470,6 @@ int build_dense(mirt_interp_plan *P, int minc, cudaStream_t st) {
   }
   P->dense_slice[t.nslice] = (int)db.size();
   if (db.empty()) return MIRT_OK;
-  int taps = 1;
-  for (int d = 0; d < a.g.D; d++) taps *= 6;
   // chunks of at most 64 samples per dense bin, summed apart, then per bin
   constexpr int kChunk = 64;
   std::vector<int4> chunks;
@@ -467,10 +483,8 @@ int build_dense(mirt_interp_plan *P, int minc, cudaStream_t st) {
   part0[db.size()] = (int)chunks.size();
   CK(P->dense_of.alloc(nb * sizeof(int)));
   CK(P->dense_bin.alloc(db.size() * sizeof(int)));
-  CK(P->patch.alloc(db.size() * (size_t)taps * a.C * sizeof(float2)));
   CK(P->dense_chunk.alloc(chunks.size() * sizeof(int4)));
   CK(P->dense_part0.alloc(part0.size() * sizeof(int)));
-  CK(P->patch_part.alloc(chunks.size() * (size_t)taps * a.C * sizeof(float2)));
   CK(cudaMemcpyAsync(P->dense_chunk.p, chunks.data(), chunks.size() * sizeof(int4),
                      cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(P->dense_part0.p, part0.data(), part0.size() * sizeof(int),
@@ -483,119 +497,131 @@ int build_dense(mirt_interp_plan *P, int minc, cudaStream_t st) {
   CK(cudaStreamSynchronize(st));
   t.dense_of = P->dense_of.as<int>();
   t.dense_bin = P->dense_bin.as<int>();
-  t.patch = P->patch.as<float2>();
   t.ndense = (int)db.size();
   t.dense_chunk = P->dense_chunk.as<int4>();
   t.dense_part0 = P->dense_part0.as<int>();
-  t.patch_part = P->patch_part.as<float2>();
   t.chunk0 = 0;
   t.nchunks = (int)chunks.size();
   return MIRT_OK;
 }
 
 // 3D line sweep: the visit lists of its blocks, their parts and the work queue of
-// these, heaviest first (cost: visits + 2 per column step), made once per plan.
-int set_line_sweep3(mirt_interp_plan *P, int nseg, cudaStream_t st) {
+// these, heaviest first (cost: visits + 2 per column step).
+int line_lists3(mirt_interp_plan *P, cudaStream_t st) {
   const InterpArgs &a = P->a;
   Tiling &t = P->t;
   const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2], S = t.nslice;
-  if (!t.s3_off) {
-    // the kernel's blocks of lines (Sweep3): 4 x 2 for 8 coils, 4 x 1 for 16, 2 x 1 for 32
-    const int cw = P->ls.cw, nl = 32 / cw, g2 = nl >= 2 ? 2 : 1, B2 = 2 * g2, B3 = nl / g2;
-    const long long per = (long long)((K2 + B2 - 1) / B2) * ((K3 + B3 - 1) / B3);
-    const long long nblock = per * S;
-    const size_t nchunk = (size_t)std::max(1, (a.C + cw - 1) / cw);
-    // visits per block and column
-    std::vector<int> n((size_t)nblock * K1);
-    {
-      DMem cnt;
-      CK(cnt.alloc(n.size() * sizeof(int)));
-      CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, nullptr, cnt.as<int>(),
-                            nullptr, nullptr, st));
-      CK(cudaMemcpyAsync(n.data(), cnt.p, n.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-    }
-    long long total = 0;
-    for (int v : n) total += v;
-    // parts: runs of columns of a block with about `most` visits, an eighth of a
-    // warp's share at full occupancy (so that the heaviest one ends with the others)
-    const long long most = std::min<long long>(std::max<long long>(total / (148 * 24 * 8), 64), 1024);
-    std::vector<int4> part, fix;
-    std::vector<long long> off(1, 0), boff(nblock);
-    P->s3_slice_part.assign(S + 1, 0);
-    P->s3_slice_fix.assign(S + 1, 0);
-    int slots = 0;
-    long long at = 0;
-    for (long long b = 0; b < nblock; b++) {
-      if (b % per == 0) {
-        P->s3_slice_part[b / per] = (int)part.size();
-        P->s3_slice_fix[b / per] = (int)fix.size();
-      }
-      boff[b] = at;
-      const size_t first = part.size();
-      const int *v = n.data() + (size_t)b * K1;
-      long long run = 0;
-      int x0 = 0;
-      for (int x = 0; x < K1; x++) {
-        run += v[x];
-        at += v[x];
-        if (x + 1 == K1 || run + v[x + 1] > most) {
-          part.push_back(make_int4((int)b, x0, x + 1, -1));
-          off.push_back(at);
-          x0 = x + 1;
-          run = 0;
-        }
-      }
-      if (part.size() - first > 1) {
-        const int n = (int)(part.size() - first), slot0 = slots;
-        for (size_t i = first; i < part.size(); i++) {
-          fix.push_back(make_int4((int)b, (int)first, n, slot0));
-          part[i].w = slots++;
-        }
-      }
-    }
-    P->s3_slice_part[S] = (int)part.size();
-    P->s3_slice_fix[S] = (int)fix.size();
-    const long long np = (long long)part.size();
-    std::vector<int> order(np);
-    for (long long i = 0; i < np; i++) order[i] = (int)i;
-    auto cost = [&](int i) {
-      return (double)(off[i + 1] - off[i]) + kSweepColumnCost * (part[i].z - part[i].y);
-    };
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
-    DMem d_boff;
-    CK(d_boff.alloc(std::max<long long>(nblock, 1) * sizeof(long long)));
-    CK(P->s3_off.alloc(off.size() * sizeof(long long)));
-    CK(P->s3_pos.alloc(std::max<long long>(total, 1) * sizeof(int)));
-    CK(P->s3_line.alloc(std::max<long long>(total, 1)));
-    CK(P->s3_part.alloc(std::max<long long>(np, 1) * sizeof(int4)));
-    CK(P->s3_fix.alloc(std::max<size_t>(fix.size(), 1) * sizeof(int4)));
-    CK(P->s3_tail.alloc(std::max<size_t>(slots * nchunk * kSweep3Tail, 1) * sizeof(float2)));
-    CK(P->team_order.alloc(std::max<long long>(np, 1) * sizeof(int)));
-    CK(P->team_next.alloc(nchunk * sizeof(int)));
-    auto up = [&](DMem &d, const void *p, size_t bytes) {
-      return bytes ? cudaMemcpyAsync(d.p, p, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
-    };
-    CK(up(d_boff, boff.data(), boff.size() * sizeof(long long)));
-    CK(up(P->s3_off, off.data(), off.size() * sizeof(long long)));
-    CK(up(P->s3_part, part.data(), part.size() * sizeof(int4)));
-    CK(up(P->s3_fix, fix.data(), fix.size() * sizeof(int4)));
-    CK(up(P->team_order, order.data(), order.size() * sizeof(int)));
-    CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, d_boff.as<long long>(),
-                          nullptr, P->s3_pos.as<int>(), P->s3_line.as<unsigned char>(), st));
+  // the kernel's blocks of lines (Sweep3): 4 x 2 for 8 coils, 4 x 1 for 16, 2 x 1 for 32
+  const int cw = P->ls.cw, nl = 32 / cw, g2 = nl >= 2 ? 2 : 1, B2 = 2 * g2, B3 = nl / g2;
+  const long long per = (long long)((K2 + B2 - 1) / B2) * ((K3 + B3 - 1) / B3);
+  const long long nblock = per * S;
+  const size_t nchunk = (size_t)std::max(1, (a.C + cw - 1) / cw);
+  // visits per block and column
+  std::vector<int> n((size_t)nblock * K1);
+  {
+    DMem cnt;
+    CK(cnt.alloc(n.size() * sizeof(int)));
+    CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, nullptr, cnt.as<int>(),
+                          nullptr, nullptr, st));
+    CK(cudaMemcpyAsync(n.data(), cnt.p, n.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    t.s3_pos = P->s3_pos.as<int>();
-    t.s3_line = P->s3_line.as<unsigned char>();
-    t.s3_part = P->s3_part.as<int4>();
-    t.s3_fix = P->s3_fix.as<int4>();
-    t.s3_tail = P->s3_tail.as<float2>();
-    t.s3_part0 = t.s3_fix0 = 0;
-    t.s3_nparts = (int)np;
-    t.s3_nfix = (int)fix.size();
-    t.team_order = P->team_order.as<int>();
-    t.team_next = P->team_next.as<int>();
-    t.s3_off = P->s3_off.as<long long>();
   }
+  long long total = 0;
+  for (int v : n) total += v;
+  // parts: runs of columns of a block with about `most` visits, an eighth of a
+  // warp's share at full occupancy (so that the heaviest one ends with the others)
+  const long long most = std::min<long long>(std::max<long long>(total / (148 * 24 * 8), 64), 1024);
+  std::vector<int4> part, fix;
+  std::vector<long long> off(1, 0), boff(nblock);
+  P->s3_slice_part.assign(S + 1, 0);
+  P->s3_slice_fix.assign(S + 1, 0);
+  int slots = 0;
+  long long at = 0;
+  for (long long b = 0; b < nblock; b++) {
+    if (b % per == 0) {
+      P->s3_slice_part[b / per] = (int)part.size();
+      P->s3_slice_fix[b / per] = (int)fix.size();
+    }
+    boff[b] = at;
+    const size_t first = part.size();
+    const int *v = n.data() + (size_t)b * K1;
+    long long run = 0;
+    int x0 = 0;
+    for (int x = 0; x < K1; x++) {
+      run += v[x];
+      at += v[x];
+      if (x + 1 == K1 || run + v[x + 1] > most) {
+        part.push_back(make_int4((int)b, x0, x + 1, -1));
+        off.push_back(at);
+        x0 = x + 1;
+        run = 0;
+      }
+    }
+    if (part.size() - first > 1) {
+      const int n = (int)(part.size() - first), slot0 = slots;
+      for (size_t i = first; i < part.size(); i++) {
+        fix.push_back(make_int4((int)b, (int)first, n, slot0));
+        part[i].w = slots++;
+      }
+    }
+  }
+  P->s3_slice_part[S] = (int)part.size();
+  P->s3_slice_fix[S] = (int)fix.size();
+  const long long np = (long long)part.size();
+  std::vector<int> order(np);
+  for (long long i = 0; i < np; i++) order[i] = (int)i;
+  auto cost = [&](int i) {
+    return (double)(off[i + 1] - off[i]) + kSweepColumnCost * (part[i].z - part[i].y);
+  };
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
+  DMem d_boff;
+  CK(d_boff.alloc(std::max<long long>(nblock, 1) * sizeof(long long)));
+  CK(P->s3_off.alloc(off.size() * sizeof(long long)));
+  CK(P->s3_pos.alloc(std::max<long long>(total, 1) * sizeof(int)));
+  CK(P->s3_line.alloc(std::max<long long>(total, 1)));
+  CK(P->s3_part.alloc(std::max<long long>(np, 1) * sizeof(int4)));
+  CK(P->s3_fix.alloc(std::max<size_t>(fix.size(), 1) * sizeof(int4)));
+  CK(P->s3_tail.alloc(std::max<size_t>(slots * nchunk * kSweep3Tail, 1) * sizeof(float2)));
+  CK(P->team_order.alloc(std::max<long long>(np, 1) * sizeof(int)));
+  CK(P->team_next.alloc(nchunk * sizeof(int)));
+  auto up = [&](DMem &d, const void *p, size_t bytes) {
+    return bytes ? cudaMemcpyAsync(d.p, p, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
+  };
+  CK(up(d_boff, boff.data(), boff.size() * sizeof(long long)));
+  CK(up(P->s3_off, off.data(), off.size() * sizeof(long long)));
+  CK(up(P->s3_part, part.data(), part.size() * sizeof(int4)));
+  CK(up(P->s3_fix, fix.data(), fix.size() * sizeof(int4)));
+  CK(up(P->team_order, order.data(), order.size() * sizeof(int)));
+  CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, d_boff.as<long long>(),
+                        nullptr, P->s3_pos.as<int>(), P->s3_line.as<unsigned char>(), st));
+  CK(cudaStreamSynchronize(st));
+  t.s3_pos = P->s3_pos.as<int>();
+  t.s3_line = P->s3_line.as<unsigned char>();
+  t.s3_part = P->s3_part.as<int4>();
+  t.s3_fix = P->s3_fix.as<int4>();
+  t.s3_tail = P->s3_tail.as<float2>();
+  t.s3_part0 = t.s3_fix0 = 0;
+  t.s3_nparts = (int)np;
+  t.s3_nfix = (int)fix.size();
+  t.team_order = P->team_order.as<int>();
+  t.team_next = P->team_next.as<int>();
+  t.s3_off = P->s3_off.as<long long>();
+  return MIRT_OK;
+}
+
+// The lists are made once per plan; where they find no room it is as it was.
+int set_line_sweep3(mirt_interp_plan *P, int nseg, cudaStream_t st) {
+  Tiling &t = P->t;
+  int rc = sweep_buffer(P);
+  if (!rc) rc = dense_patches(P);
+  if (!rc && !t.s3_off) {
+    rc = line_lists3(P, st);
+    if (rc)
+      for (DMem *d : {&P->s3_off, &P->s3_pos, &P->s3_line, &P->s3_part, &P->s3_fix, &P->s3_tail,
+                      &P->team_order, &P->team_next})
+        d->release();
+  }
+  if (rc) return rc;
   // (the parts follow the visits, not the segments)
   t.sweep = nseg;
   t.sweep_rows = 1;
@@ -844,16 +870,6 @@ int build_split(mirt_interp_plan *P, cudaStream_t st) {
   t.split = form == Spread2D::split;
   if (!t.split) t.points = 0;
   return MIRT_OK;
-}
-
-// Uniform segments: the work queue of their teams.
-int set_uniform_sweep(mirt_interp_plan *P, int nseg, int rows, cudaStream_t st) {
-  P->t.sweep = nseg;
-  P->t.sweep_rows = rows;
-  std::vector<float> vb;
-  int rc = sweep_band_visits(P, rows, st, vb);
-  if (rc) return rc;
-  return build_sweep_order(P, vb, st);
 }
 
 // The plan's gather over slices [s0, s1) (all: s1 < 0): the TMA-staged tiles
@@ -1390,9 +1406,9 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     P->t.dense_on = P->t.dense_of ? 1 : 0;
   }
   if (sweep_ok(a, P->t) && P->ls.cw == 32) {
-    int rc3 = sweep_buffer(P);
+    int rc3 = row_buffers(P);
     if (rc3) return rc3;
-    // (its team list is made when it is first needed: sweep_teams_ready)
+    // (its team list is made when it is first needed: row_sweep_ready)
     P->t.sweep = -1;
     P->t.sweep_rows = 1;
     const size_t nq = (size_t)(a.C + 31) / 32;  // the queue counters of slice ranges
@@ -1406,18 +1422,15 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
   }
   // 3D, J = 6, coil chunks of 8, 16 or 32: the line sweep, two segments per line
   if (sweep3_ok(a, P->t, P->ls.cw)) {
-    int rc3 = sweep_buffer(P);
-    if (rc3) return rc3;
-    rc3 = set_line_sweep3(P, 2, st);
-    if (rc3 && rc3 != MIRT_ERR_ALLOC) return rc3;
-    if (rc3) cudaGetLastError();  // no room for the visit lists: the point spread
+    int rc3 = set_line_sweep3(P, 2, st);
+    if (rc3 && rc3 != MIRT_ERR_ALLOC) return rc3;  // (no room: the point spread)
   }
   // everything else: the point spread
   if (!P->t.sweep && !P->t.split && a.C > 0) {
     int rc3 = build_points(P, st);
     if (rc3) return rc3;
   }
-  return P->t.sweep < 0 && !P->t.points ? sweep_teams_ready(P, st) : MIRT_OK;
+  return P->t.sweep < 0 && !P->t.points ? row_sweep_ready(P, st) : MIRT_OK;
 }
 
 // Re-tile the spread (tiles of T[d] points, multiples of the sort bins) and
@@ -1518,8 +1531,9 @@ static mirt_interp_plan *launch_plan(mirt_interp_plan *P) { return P->sub4 ? P->
 // A row-sweep setting was chosen: the row sweep itself, not the spread on top of it.
 static int leave_split(mirt_interp_plan *P) {
   if (!P->t.sweep || !P->t.points) return MIRT_OK;
-  P->t.points = P->t.split = 0;
-  return sweep_teams_ready(P, as_stream(nullptr));
+  int rc = row_sweep_ready(P, as_stream(nullptr));
+  if (!rc) P->t.points = P->t.split = 0;
+  return rc;
 }
 
 extern "C" {
@@ -1527,6 +1541,8 @@ extern "C" {
 const char *mirt_last_error(void) { return g_err.c_str(); }
 
 int mirt_version(void) { return 100; }
+
+int mirt_test_fail_alloc(int32_t n) { return g_alloc_left.exchange(n); }
 
 int mirt_interp_plan_create(mirt_interp_plan **plan, int32_t D, const int32_t *K,
                             const int32_t *J, const int32_t *L, const double *const *h_re,
@@ -1692,7 +1708,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
   }
   // row sweep (no tiles): bands of 1, 2 or 4 rows, whole rows or uniform
   // segments of at least 32 columns, or balanced teams (sweep = -1)
-  if (sweep_ok(a, P->t) && sweep_buffer(P) == MIRT_OK)
+  if (sweep_ok(a, P->t))
     for (int dense : {0, 1})
       for (int rows : {1, 2, 4})
         for (int nseg = -1; nseg <= 16 && (nseg <= 1 || a.g.K[0] / nseg >= 32);
@@ -1703,7 +1719,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
                 cands.push_back(SpreadCand{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0,
                                            0, 0, nseg, rows, dense, staged});
   // 3D line sweep
-  if (sweep3_ok(a, P->t, cw) && sweep_buffer(P) == MIRT_OK)
+  if (sweep3_ok(a, P->t, cw))
     cands.push_back(SpreadCand{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, 2, 1});
   if (P->points_shape) {
     SpreadCand c{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0,
@@ -1717,10 +1733,20 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     c.split = 1;
     cands.push_back(c);
   }
-  SpreadCand best{};
-  float best_ms = 1e30f;
-  int built_rows = 0;  // rows of the team list last built
-  for (const SpreadCand &c : cands) {
+  // One candidate, its lists first: where they find no room the plan stays at the last
+  // one.  (The point and the split spread on top of a row sweep need none of its own.)
+  auto apply = [&](const SpreadCand &c) -> int {
+    int rc = MIRT_OK;
+    if (c.sweep && !c.points) {
+      if (D == 3) {
+        rc = set_line_sweep3(P, c.sweep, st);
+      } else {
+        rc = row_buffers(P);
+        if (!rc && (c.sweep > 0 || P->team_rows != c.sweep_rows))
+          rc = set_row_sweep(P, c.sweep, c.sweep_rows, st);
+      }
+    }
+    if (rc) return rc;
     P->t.own = c.own;
     P->t.sweep = c.sweep;
     P->t.sweep_rows = c.sweep_rows;
@@ -1728,27 +1754,43 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     P->t.sweep_staged = c.staged;
     P->t.points = c.points;
     P->t.split = c.split;
-    if (c.sweep < 0 && built_rows != c.sweep_rows) {
-      int rc = build_sweep_teams(P, c.sweep_rows, 65536, st);
-      if (rc) return rc;
-      built_rows = c.sweep_rows;
-    } else if (c.sweep > 0) {
-      int rc = D == 3 ? set_line_sweep3(P, c.sweep, st)
-                      : set_uniform_sweep(P, c.sweep, c.sweep_rows, st);
-      if (rc) return rc;
-      built_rows = 0;  // the work queue now orders uniform segments
-    }
-    int rc = set_spread_tiles(P, c.T, st);
-    if (rc) continue;
     P->ls.threads = c.threads;
     P->t.padc = c.padc;
     P->ls.atomic = c.atomic;
+    return set_spread_tiles(P, c.T, st);
+  };
+  // The plan as it came, for where the tuning ends early (the tiled spread where even
+  // that finds no room).
+  SpreadCand now{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, P->t.padc, P->ls.atomic,
+                 P->t.own, P->t.sweep, P->t.sweep_rows};
+  now.dense = P->t.dense_on;
+  now.staged = P->t.sweep_staged;
+  now.points = P->t.points;
+  now.split = P->t.split;
+  const int chunk_now = P->split_chunk, heavy_now = P->heavy_first, tma_now = P->gtma;
+  const Launch gather_now = P->lg;
+  auto give_up = [&](int rc) -> int {
+    const std::string msg = g_err;
+    P->split_chunk = chunk_now;
+    P->heavy_first = heavy_now;
+    P->gtma = tma_now;
+    P->lg = gather_now;
+    if (apply(now)) {
+      P->t.sweep = P->t.points = P->t.split = P->t.own = 0;
+      set_spread_tiles(P, now.T, st);
+    }
+    return fail(rc, msg);
+  };
+  SpreadCand best = now;
+  float best_ms = 1e30f;
+  for (const SpreadCand &c : cands) {
+    if (apply(c)) continue;
     float ms = 0;
-    rc = time_launch([&]() {
+    int rc = time_launch([&]() {
       return launch_spread(P->a, P->t, P->ls, P->bin_start.as<int>(), samp.as<float2>(),
                            grid.as<float2>(), st);
     }, st, &ms);
-    if (rc) return rc;
+    if (rc) return give_up(rc);
     if (autotune_log())
       std::fprintf(stderr,
                    "mirt autotune spread: tile %dx%dx%d threads %d padc %d atomic %d own %d "
@@ -1760,27 +1802,9 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
       best = c;
     }
   }
-  if (best_ms < 1e30f) {
-    P->t.own = best.own;
-    P->t.sweep = best.sweep;
-    P->t.sweep_rows = best.sweep_rows;
-    P->t.dense_on = best.dense;
-    P->t.sweep_staged = best.staged;
-    P->t.points = best.points;
-    P->t.split = best.split;
-    if (best.sweep < 0 && built_rows != best.sweep_rows) {
-      int rc = build_sweep_teams(P, best.sweep_rows, 65536, st);
-      if (rc) return rc;
-    } else if (best.sweep > 0) {
-      int rc = D == 3 ? set_line_sweep3(P, best.sweep, st)
-                      : set_uniform_sweep(P, best.sweep, best.sweep_rows, st);
-      if (rc) return rc;
-    }
-    int rc = set_spread_tiles(P, best.T, st);
-    if (rc) return rc;
-    P->ls.threads = best.threads;
-    P->t.padc = best.padc;
-    P->ls.atomic = best.atomic;
+  {
+    int rc = apply(best);
+    if (rc) return give_up(rc);
   }
   // split size of heavy tiles (sample visits per spread task)
   if (!P->t.sweep && !P->t.points) {
@@ -1789,13 +1813,13 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     for (int chunk : {256, 512, 1024, 2048, 4096, 16384}) {
       P->split_chunk = chunk;
       int rc = build_tasks(P, st);
-      if (rc) return rc;
+      if (rc) return give_up(rc);
       float ms = 0;
       rc = time_launch([&]() {
         return launch_spread(P->a, P->t, P->ls, P->bin_start.as<int>(), samp.as<float2>(),
                              grid.as<float2>(), st);
       }, st, &ms);
-      if (rc) return rc;
+      if (rc) return give_up(rc);
       if (ms < bc_ms) {
         bc_ms = ms;
         best_chunk = chunk;
@@ -1808,16 +1832,16 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     for (int hf = 0; hf < 2; hf++) {
       P->heavy_first = hf;
       int rc = build_tasks(P, st);
-      if (rc) return rc;
+      if (rc) return give_up(rc);
       rc = time_launch([&]() {
         return launch_spread(P->a, P->t, P->ls, P->bin_start.as<int>(), samp.as<float2>(),
                              grid.as<float2>(), st);
       }, st, &order_ms[hf]);
-      if (rc) return rc;
+      if (rc) return give_up(rc);
     }
     P->heavy_first = order_ms[1] <= order_ms[0] ? 1 : 0;
     int rc = build_tasks(P, st);
-    if (rc) return rc;
+    if (rc) return give_up(rc);
   }
   // gather candidates: CTA size of the plain gather, and the TMA-staged gather
   Launch bestg = P->lg;
@@ -1829,12 +1853,13 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
     Launch l = P->lg;
     l.threads = threads;
     l.grid = 0;
-    CK(query_gather_grid(P->a, l));
+    if (query_gather_grid(P->a, l) != cudaSuccess)
+      return give_up(fail(MIRT_ERR_CUDA, "gather occupancy"));
     float ms = 0;
     int rc = time_launch([&]() {
       return launch_gather(P->ag, l, grid.as<float2>(), samp.as<float2>(), st);
     }, st, &ms);
-    if (rc) return rc;
+    if (rc) return give_up(rc);
     if (ms < bestg_ms) {
       bestg_ms = ms;
       bestg = l;
@@ -1848,7 +1873,7 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
       int rc = time_launch([&]() {
         return plan_gather(P, grid.as<float2>(), samp.as<float2>(), st);
       }, st, &ms);
-      if (rc) return rc;
+      if (rc) return give_up(rc);
       if (autotune_log())
         std::fprintf(stderr, "mirt autotune gather: TMA tiles of %d coils: %.3f ms\n",
                      a.g.D == 3 ? 8 : mode == 2 ? 16 : 32, ms);
@@ -1921,13 +1946,12 @@ int mirt_interp_plan_set_sweep(mirt_interp_plan *P, int32_t segments, int32_t ro
                                 "chunks of 8, 16 or 32");
     if (segments < 0 || segments > P->a.g.K[0])
       return fail(MIRT_ERR_ARG, "3D line-sweep segments must be in 1..K1 (0: off)");
-    P->t.points = P->t.split = 0;
     if (segments) {
-      int rc = sweep_buffer(P);
+      int rc = set_line_sweep3(P, segments, as_stream(nullptr));
       if (rc) return rc;
-      return set_line_sweep3(P, segments, as_stream(nullptr));
     }
-    P->t.sweep = 0;
+    P->t.sweep = segments;
+    P->t.points = P->t.split = 0;
     return MIRT_OK;
   }
   if (segments && !sweep_ok(P->a, P->t))
@@ -1936,18 +1960,12 @@ int mirt_interp_plan_set_sweep(mirt_interp_plan *P, int32_t segments, int32_t ro
     return fail(MIRT_ERR_ARG, "row-sweep segments must be in 1..K1 (0: off, -1: balanced)");
   if (segments && rows != 1 && rows != 2 && rows != 4)
     return fail(MIRT_ERR_ARG, "row-sweep rows per band must be 1, 2 or 4");
-  P->t.points = P->t.split = 0;
   if (segments) {
-    int rc = sweep_buffer(P);
+    int rc = row_buffers(P);
+    if (!rc) rc = set_row_sweep(P, segments, rows, as_stream(nullptr));
     if (rc) return rc;
   }
-  if (segments < 0) {
-    int rc = build_sweep_teams(P, rows, 65536, as_stream(nullptr));
-    if (rc) return rc;
-  } else if (segments > 0) {
-    int rc = set_uniform_sweep(P, segments, rows, as_stream(nullptr));
-    if (rc) return rc;
-  }
+  P->t.points = P->t.split = 0;
   P->t.sweep = segments;
   if (segments) P->t.sweep_rows = rows;
   if (segments) {
@@ -1963,8 +1981,9 @@ int mirt_interp_plan_set_dense(mirt_interp_plan *P, int32_t on) try {
   if (!P) return fail(MIRT_ERR_ARG, "plan is NULL");
   P = launch_plan(P);
   if (on && !P->t.dense_of) return fail(MIRT_ERR_ARG, "the plan has no dense bins");
-  P->t.dense_on = on ? 1 : 0;
-  return leave_split(P);
+  int rc = leave_split(P);
+  if (!rc) P->t.dense_on = on ? 1 : 0;
+  return rc;
 } catch (const std::bad_alloc &) {
   return fail(MIRT_ERR_ALLOC, "out of host memory");
 }
@@ -1975,8 +1994,9 @@ int mirt_interp_plan_set_staged(mirt_interp_plan *P, int32_t mode) try {
   if (mode < 0 || mode > 2) return fail(MIRT_ERR_ARG, "staged mode must be 0, 1 or 2");
   if (mode && (P->ls.cw != 32 || !P->t.wsw))
     return fail(MIRT_ERR_ARG, "the staged row sweep needs 32-coil lanes (C >= 32)");
-  P->t.sweep_staged = mode;
-  return leave_split(P);
+  int rc = leave_split(P);
+  if (!rc) P->t.sweep_staged = mode;
+  return rc;
 } catch (const std::bad_alloc &) {
   return fail(MIRT_ERR_ALLOC, "out of host memory");
 }

@@ -37,8 +37,9 @@ struct DMem {
   }
   cudaError_t alloc(size_t b) {
     release();
-    bytes = b;
-    return dalloc(&p, b);
+    const cudaError_t e = dalloc(&p, b);
+    if (e == cudaSuccess) bytes = b;
+    return e;
   }
   template <class T>
   T *as() const {
@@ -72,7 +73,7 @@ struct mirt_interp_plan {
   mirt::DMem wsw;           // staged 2D row sweep: tap records with FFMA2 operand pairs, plan order
   mirt::DMem swept;        // row-sweep spread: the samples in plan order, [Mtot][C]
   mirt::DMem sweep_teams;  // row-sweep spread: balanced team list (int4 per team)
-  std::vector<int4> team_host;  // the same list on the host
+  int team_rows = 0;       // rows per band of the list (0: none, or its order is another's)
   // 3D line sweep: the parts' visit lists and records, first part / fix of each slice
   mirt::DMem s3_off, s3_pos, s3_line, s3_part, s3_fix, s3_tail;
   std::vector<int> s3_slice_part, s3_slice_fix;

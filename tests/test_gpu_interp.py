@@ -1167,6 +1167,74 @@ def test_ownership_off_leaves_the_spread(K, C, M):
     plan.close()
 
 
+def _each_failing_allocation(f, steps=range(400)):
+    """Yields f's result, or None where it raised for want of memory, with the n-th device
+    allocation failing for the n of steps, until one run needs fewer."""
+    lib = mb.load()
+    for n in steps:
+        lib.mirt_test_fail_alloc(n)
+        try:
+            out = f()
+        except mb.MirtError as e:
+            out = None
+            assert e.code == 3, e               # MIRT_ERR_ALLOC
+        finally:
+            left = lib.mirt_test_fail_alloc(-1)
+        yield n, out
+        if left >= 0:
+            return
+    raise AssertionError("allocations without end")
+
+
+ALLOC_PLANS = [((64, 48), 26, 1500), ((64, 48), 32, 1500), ((96, 80), 32, 30000), ((128, 100), 34, 60000),
+               ((16, 14, 12), 8, 6000)]
+
+
+@pytest.mark.parametrize("K,C,M,what", [
+    p + (w,) for p in ALLOC_PLANS for w in ("sweep", "balanced", "dense", "staged", "autotune")
+    if not (w == "staged" and p[1] < 32 or w == "autotune" and p[2] > 6000)])
+def test_failed_allocations_leave_the_plan_working(K, C, M, what):
+    """A setter or the autotuner whose device allocation fails, whichever it is, returns an error
+    or does without; the plan computes the adjoint and the forward as before either way, and the
+    same call succeeds with memory again."""
+    import torch
+    D = len(K)
+    rng = np.random.default_rng(C + M)
+    tm = np.concatenate([rng.uniform(-60, 60, (M // 2, D)), rng.uniform(-3, 3, (M - M // 2, D))])
+    h = [mb.newfft_kb_table(6, 64)] * D
+
+    def call(plan):
+        if what == "sweep":
+            plan.set_sweep(3, 2)
+        elif what == "balanced":
+            plan.set_sweep(-1 if D == 2 else 1, 4)
+        elif what == "dense":
+            plan.set_dense(True)
+        elif what == "staged":
+            plan.set_staged(2)
+        else:
+            plan.autotune()
+        return True
+    first = mb.InterpPlan(list(K), [6] * D, [64] * D, h, tm, C, order=1)
+    fm = torch.randn(first.sample_shape, dtype=torch.complex64, device="cuda")
+    ck = torch.randn(first.grid_shape, dtype=torch.complex64, device="cuda")
+    adj, fwd = first.adjoint(fm).cpu().numpy(), first.forward(ck)
+    first.close()
+    plan = mb.InterpPlan(list(K), [6] * D, [64] * D, h, tm, C, order=1)
+    # (the autotuner builds hundreds of tile lists: its first allocations, then one in 197)
+    steps = range(400) if what != "autotune" else list(range(8)) + list(range(8, 9999, 197))
+    for n, ok in _each_failing_allocation(lambda: call(plan), steps):
+        out = torch.full(first.grid_shape, float("nan"), dtype=torch.complex64, device="cuda")
+        assert rel_l2(plan.adjoint(fm, out=out).cpu().numpy(), adj) <= 5e-6, (n, ok)
+        assert torch.equal(plan.forward(ck), fwd), (n, ok)
+        if what != "autotune" and ok is None:   # a plan that has its lists needs none again
+            plan.close()
+            plan = mb.InterpPlan(list(K), [6] * D, [64] * D, h, tm, C, order=1)
+    assert ok
+    assert rel_l2(plan.adjoint(fm).cpu().numpy(), adj) <= 5e-6
+    plan.close()
+
+
 def _taps_of(t, J, K):
     """Mask [K_D, ..., K_1] of the grid points that a sample at t reaches."""
     m = np.ones((), bool)
