@@ -1406,9 +1406,7 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     P->t.dense_on = P->t.dense_of ? 1 : 0;
   }
   if (sweep_ok(a, P->t) && P->ls.cw == 32) {
-    int rc3 = row_buffers(P);
-    if (rc3) return rc3;
-    // (its team list is made when it is first needed: row_sweep_ready)
+    // (its buffers and team list are made when it is selected: row_sweep_ready)
     P->t.sweep = -1;
     P->t.sweep_rows = 1;
     const size_t nq = (size_t)(a.C + 31) / 32;  // the queue counters of slice ranges

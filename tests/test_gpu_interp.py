@@ -1235,6 +1235,23 @@ def test_failed_allocations_leave_the_plan_working(K, C, M, what):
     plan.close()
 
 
+def test_plan_holds_the_row_sweeps_buffers_when_it_is_selected():
+    """500,000 samples of 256 columns whose default is the split spread: the row sweep's copy of
+    them, a gigabyte, is there once the row sweep is."""
+    import torch
+    rng = np.random.default_rng(1)
+    M, C, K = 500000, 256, [256, 256]
+    tm = rng.uniform(-128, 128, (M, 2))
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    plan = mb.InterpPlan(K, [6, 6], [64, 64], [mb.newfft_kb_table(6, 64)] * 2, tm, C, order=1)
+    assert plan.config()["spread_split"] == 1
+    assert free - torch.cuda.mem_get_info()[0] < 0.9 * 8 * M * C
+    plan.set_staged(2)
+    assert free - torch.cuda.mem_get_info()[0] > 8 * M * C
+    plan.close()
+
+
 def _taps_of(t, J, K):
     """Mask [K_D, ..., K_1] of the grid points that a sample at t reaches."""
     m = np.ones((), bool)
