@@ -722,6 +722,17 @@ int build_points(mirt_interp_plan *P, cudaStream_t st) {
   return build_point_tasks(P, shape, most, -1, st);
 }
 
+// No point or split spread: what their lists have found room for is given back.
+void drop_points(mirt_interp_plan *P) {
+  Tiling &t = P->t;
+  for (DMem *d : {&P->wsw, &P->pt_task, &P->pt_slice_task, &P->pt_hdr, &P->pt_scratch, &P->pt_count,
+                  &P->split_teams, &P->split_order, &P->split_next})
+    d->release();
+  t.wsw = nullptr;
+  t.points = t.split = t.split_nteams = t.n_pt_task = t.pt_slots = 0;
+  P->points_shape = P->split_ok = 0;
+}
+
 // The staged sweep's records (FFMA2 operand pairs of the taps).
 int build_sweep_records(mirt_interp_plan *P, cudaStream_t st) {
   const long long M = P->a.Mtot;
@@ -1413,22 +1424,32 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     CK(P->team_next.alloc(nq * sizeof(int)));
     P->t.team_next = P->team_next.as<int>();
   }
+  // The lists of the spreads below may find no room: the plan then takes the next one
+  // that needs less, in the end the tiled spread, whose tasks are built.
   if (sweep_ok(a, P->t) && a.C >= kSplitColumns) {
     int rc3 = build_sweep_records(P, st);
     if (!rc3) rc3 = build_split(P, st);
-    if (rc3) return rc3;
+    if (rc3 == MIRT_ERR_ALLOC) drop_points(P);
+    else if (rc3) return rc3;
   }
-  // 3D, J = 6, coil chunks of 8, 16 or 32: the line sweep, two segments per line
+  // 3D, J = 6, coil chunks of 8, 16 or 32: the line sweep
   if (sweep3_ok(a, P->t, P->ls.cw)) {
     int rc3 = set_line_sweep3(P, 2, st);
-    if (rc3 && rc3 != MIRT_ERR_ALLOC) return rc3;  // (no room: the point spread)
+    if (rc3 && rc3 != MIRT_ERR_ALLOC) return rc3;
   }
   // everything else: the point spread
   if (!P->t.sweep && !P->t.split && a.C > 0) {
     int rc3 = build_points(P, st);
-    if (rc3) return rc3;
+    if (rc3 == MIRT_ERR_ALLOC) drop_points(P);
+    else if (rc3) return rc3;
   }
-  return P->t.sweep < 0 && !P->t.points ? row_sweep_ready(P, st) : MIRT_OK;
+  if (P->t.sweep >= 0 || P->t.points) return MIRT_OK;
+  int rc4 = row_sweep_ready(P, st);
+  if (rc4 == MIRT_ERR_ALLOC && P->split_ok) {  // without the autotuner's split lists
+    drop_points(P);
+    rc4 = row_sweep_ready(P, st);
+  }
+  return rc4;
 }
 
 // Re-tile the spread (tiles of T[d] points, multiples of the sort bins) and
