@@ -501,11 +501,12 @@ int mirt_sense_create(mirt_sense **out, mirt_nufft *G, const void *sens, const d
                               cudaMemcpyHostToDevice, st);
   if (!e && G->own_fft && op->S > 0 && op->C > 0) {
     const long long n = (long long)nimg * op->C;
-    if (op->sens_sn.alloc(n * sizeof(float2)))
-      return bail(api_fail(MIRT_ERR_ALLOC, "CG-SENSE buffers"));
-    k_maps_sn<<<nblocks(n), 256, 0, st>>>(op->sens.as<float2>(), G->sn.as<float2>(),
-                                          op->sens_sn.as<float2>(), n, op->np, op->C);
-    e = cudaGetLastError();
+    // (no room for a second set of maps: A expands the coil images)
+    if (op->sens_sn.alloc(n * sizeof(float2)) == cudaSuccess) {
+      k_maps_sn<<<nblocks(n), 256, 0, st>>>(op->sens.as<float2>(), G->sn.as<float2>(),
+                                            op->sens_sn.as<float2>(), n, op->np, op->C);
+      e = cudaGetLastError();
+    }
   }
   if (!e) e = cudaStreamSynchronize(st);
   if (e) return bail(api_fail(MIRT_ERR_CUDA, cudaGetErrorString(e)));

@@ -45,6 +45,41 @@ def _batch(seed, N, K, C, spokes, beta=None):
     return A, refs, xt, ys, moff
 
 
+def test_system_without_room_for_the_second_set_of_maps():
+    """SenseSystem creation with each device allocation failing in turn: an error, or (the last
+    one, the maps times sn) a system whose A expands the coil images instead."""
+    import torch
+    rng = np.random.default_rng(2)
+    N, C = 32, 4
+    om = wl.ga_radial(20, 2 * N)
+    G = mb.NufftPlan(om, (N, N), (6, 6), (2 * N, 2 * N), n_shift=(N / 2, N / 2), Ld=1024, ncol=C)
+    assert G.fft_config()["fused_fft"] == 1
+    sens = torch.randn((1, N, N, C), dtype=torch.complex64, device="cuda")
+    x = torch.randn((1, N, N), dtype=torch.complex64, device="cuda")
+    y = torch.randn((len(om), C), dtype=torch.complex64, device="cuda")
+    A = ms.SenseSystem(G, sens, 0.1)
+    ref, adj = A.forward(x).cpu().numpy(), A.adjoint(y)
+    A.close()
+    made = []
+    for n in range(40):
+        G.lib.mirt_test_fail_alloc(n)
+        try:
+            A = ms.SenseSystem(G, sens, 0.1)
+        except mb.MirtError as e:
+            A = None
+            assert e.code == 3
+        left = G.lib.mirt_test_fail_alloc(-1)
+        made.append(A is not None)
+        if A is not None:
+            assert rel_l2(A.forward(x).cpu().numpy(), ref) <= 1e-6
+            assert torch.equal(A.adjoint(y), adj)
+            A.close()
+        if left >= 0:
+            break
+    assert made[-2] and made[-1] and not made[0]
+    G.close()
+
+
 def test_operators_match_oracle():
     import torch
     A, refs, xt, ys, moff = _batch(1, 32, 64, 4, [20, 14, 27])
