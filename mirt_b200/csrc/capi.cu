@@ -3532,9 +3532,10 @@ int mirt_nufft_config(mirt_nufft *p, int32_t *out, int32_t n) {
   const int glue = p->own_fft ? p->gg.D : p->one_col ? 1 : 2;  // around the interpolation
   const int fwd = glue + 1;
   int spread = 1;  // the point spread: one launch
-  if (t.split) {
+  const bool fixed = t.sweep || !p->ip->ls.atomic;  // as launch_spread
+  if (t.split && fixed) {
     spread = (t.split_nteams > 0) + (t.n_pt_task > 0);
-  } else if (t.points && (t.sweep || !p->ip->ls.atomic)) {
+  } else if (t.points && fixed) {
   } else if (t.sweep != 0) {
     // ordering pass, dense-bin patches (chunk sums, per-bin sums), sweep (and a
     // memset of the queue counters)

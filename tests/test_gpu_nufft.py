@@ -339,6 +339,21 @@ def test_host_adjoint_gives_the_device_adjoints_bits(form, C, nslice):
     plan.close()
 
 
+@pytest.mark.parametrize("C", [8, 26])
+def test_launch_count_of_the_atomic_spread(C):
+    """set_deterministic(False) moves plans without a sweep from the point or the split spread
+    (a dense tile among sparse ones) to the tiled one, and the reported launches with it."""
+    rng = np.random.default_rng(C)
+    om = np.concatenate([rng.uniform(-np.pi, np.pi, (900, 2)), rng.uniform(-0.05, 0.05, (150, 2))])
+    plan = mb.NufftPlan(om, (32, 32), (6, 6), (64, 64), Ld=64, ncol=C)
+    assert plan.fft_config() == {"fused_fft": 1, "launches_forward": 3,
+                                 "launches_adjoint": 4 if C == 26 else 3}
+    cfg = plan.set_deterministic(False)
+    assert cfg["spread_tasks"] > 0 and cfg["spread_reductions"] == 0
+    assert plan.fft_config()["launches_adjoint"] == 3
+    plan.close()
+
+
 def test_host_calls_of_3d_slices():
     """Slice ranges of the 3D line sweep (its parts and tails by slice): the pipelined
     host adjoint against the device adjoint."""
