@@ -229,7 +229,8 @@ int mirt_interp_plan_create(mirt_interp_plan **plan, int32_t D,
 /* fm = interp(ck) on device buffers, asynchronous on `stream`. */
 int mirt_interp_plan_forward(mirt_interp_plan *plan, const void *ck, void *fm, void *stream);
 
-/* ck = interp_adj(fm) on device buffers; overwrites all of ck. */
+/* ck = interp_adj(fm) on device buffers; overwrites all of ck.  A plan's
+ * adjoints share its scratch and work queues: order those on several streams. */
 int mirt_interp_plan_adjoint(mirt_interp_plan *plan, const void *fm, void *ck, void *stream);
 
 /* Autotune: time candidate spread tile shapes (multiples of the sort bins),

@@ -12,16 +12,17 @@
 // times conj(phase) into the group's shared-memory stage, all loads of a chunk
 // in flight together, and then every lane adds each staged sample's taps into
 // its own block where the block's row and plane are among the sample's.  The
-// samples are read through the sort permutation: no ordering pass, no per-plan
-// copy, nothing shared between calls.
+// samples are read through the sort permutation: no ordering pass and no per-plan
+// copy.
 //
 // Dense bricks (the k-space centre of radial and kooshball trajectories): the
 // plan gives each base tile of bricks a split G, a power of two, so that no
 // group walks more than about pt_visits() samples: the tile becomes G CTAs of 1/G
 // of its bricks, with G groups per brick that take every G-th chunk and are
 // summed in a fixed order; CTAs that share a brick leave their sums in the plan's
-// scratch, and the last of them to finish adds them in order.  G depends on the trajectory alone: every grid point
-// is summed in one order, bitwise reproducible, with no atomics.
+// scratch, and the last of them to finish adds them in order (one launch of a plan at a
+// time).  G depends on the trajectory alone: every grid point is summed in one order,
+// bitwise reproducible, with no atomics on the sums.
 //
 // Bound by instruction issue (about 100 warp instructions per sample at one
 // column in 2D, 46 % of the lanes of a visit useful).  Against the tiled spread,
@@ -445,8 +446,8 @@ __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
         for (int k = 0; k < X; k++) acc[m][k] = again[m * X + k];
     }
   }
-  // sum a brick's groups in order: those of this CTA, then those of the
-  // cluster's CTAs that share it
+  // sum a brick's groups in order: those of this CTA, then those of the CTAs that
+  // share it
   if (lg > 0) {
     __syncthreads();
     float2 *red = reinterpret_cast<float2 *>(smem);  // [NGRP][NC X][GL]
@@ -480,9 +481,9 @@ __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
       __threadfence();
       __syncthreads();
       if (threadIdx.x == 0) {
+        // (counts round: zero again once every CTA has counted, whatever launch it is of)
         int *c = t.pt_count + (size_t)blockIdx.y * t.pt_slots + tk.w;
-        last = atomicAdd(c, 1) == nc - 1;
-        if (last) *c = 0;  // for the next launch
+        last = atomicInc(reinterpret_cast<unsigned *>(c), (unsigned)nc - 1u) == (unsigned)nc - 1u;
       }
       __syncthreads();
       if (!last || grp) return;
