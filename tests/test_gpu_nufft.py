@@ -354,6 +354,38 @@ def test_launch_count_of_the_atomic_spread(C):
     plan.close()
 
 
+@pytest.mark.parametrize("M,C,points", [(0, 8, True), (4000, 8, True), (4001, 8, False), (900, 24, True),
+                                        (300, 96, False)])
+def test_3d_adjoint_of_few_samples(M, C, points):
+    """Few samples on a small 3D grid: the point spread in place of the line sweep, against the
+    line sweep and the oracle; the host-buffer call of the slices gives its bits, other settings
+    leave it, the sweep's own turns to the line sweep."""
+    import torch
+    rng = np.random.default_rng(M + C)
+    N, K = (20, 18, 16), (40, 36, 32)
+    om = rng.uniform(-np.pi, np.pi, (M, 3))
+    om[:M // 3] *= 0.1
+    moff = np.array([0, M // 2, M])
+    plan = mb.NufftPlan(om, N, (6, 6, 6), K, n_shift=(10, 9, 8), Ld=256, ncol=C, slice_moff=moff)
+    cfg = plan.config()
+    assert cfg["spread_sweep"] == 2 and (cfg["spread_points"] > 0) == points
+    X = torch.randn((M, C), dtype=torch.complex64, device="cuda")
+    out = plan.adjoint(X)
+    assert rel_l2(plan.adjoint_host(X.cpu().numpy()), out.cpu().numpy()) <= 1e-6 if M else not out.any()
+    plan.set_deterministic(False)
+    plan.set_dense(False)
+    assert (plan.config()["spread_points"] > 0) == points and torch.equal(plan.adjoint(X), out)
+    for s in range(2 if M else 0):
+        sl = slice(moff[s], moff[s + 1])
+        st_o = nr.nufft_init_table(om[sl], N, (6, 6, 6), K, (10, 9, 8), 256)
+        fw, ad = _oracle_pair(st_o)
+        assert rel_l2(out[s, ..., 0].cpu().numpy().T,
+                      nr.nufft_adj(X[sl, 0].cpu().numpy(), st_o, ad)) <= ADJ_TOL
+    assert plan.set_sweep(1)["spread_points"] == 0
+    assert rel_l2(plan.adjoint(X).cpu().numpy(), out.cpu().numpy()) <= 5e-6 if M else not plan.adjoint(X).any()
+    plan.close()
+
+
 def test_host_calls_of_3d_slices():
     """Slice ranges of the 3D line sweep (its parts and tails by slice): the pipelined
     host adjoint against the device adjoint."""
