@@ -2,6 +2,7 @@
 // lengths and their dispatch, and the forward and adjoint pass sequences.
 #include "fft_impl.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace mirt {
@@ -33,6 +34,14 @@ int vec_width(long long v) {
   int w = 1;
   while (w < 16 && v % (2 * w) == 0) w *= 2;
   return w;
+}
+
+// ... for a pass of `lines` of n: 8 where few lines of 16 would take a block two turns
+int pass_width(int n, long long v, long long lines) {
+  const int w = vec_width(v);
+  int r1 = 0, r2 = 0;
+  fft_radix(n, &r1, &r2);
+  return w == 16 && lines * (v / w) < 74 && 16 * std::max(r1, r2) > fftk::kThreads ? 8 : w;
 }
 
 FftPass base_pass(const NufftFft &f, int d, int s0, int s1, bool inverse) {
@@ -145,7 +154,7 @@ cudaError_t fft_nufft_forward(const NufftFft &f, const float2 *x, float2 *grid, 
     p.os[1] = (long long)K2 * K1 * C;
     p.os[2] = (long long)K1 * C;
     p.es_in = p.es_out = C;
-    p.vw = vec_width(C);
+    p.vw = pass_width(p.n, C, (long long)(s1 - s0) * p.nr1 * p.nr2);
     p.nvec = (int)(C / p.vw);
     p.nin = N1;
     p.nout = K1;
@@ -231,7 +240,7 @@ cudaError_t fft_nufft_adjoint(const NufftFft &f, float2 *grid, float2 *x, int s0
   p.os[1] = (long long)N2 * N1 * C;
   p.os[2] = (long long)N1 * C;
   p.es_in = p.es_out = C;
-  p.vw = vec_width(C);
+  p.vw = pass_width(p.n, C, (long long)(s1 - s0) * p.nr1 * p.nr2);
   p.nvec = (int)(C / p.vw);
   p.nin = K1;
   p.nout = N1;

@@ -29,6 +29,7 @@
 // Taylor series in FP64; the pass twiddles W_n^{p1 q} come from an FP64-built
 // table.  Arithmetic is FP32.
 #pragma once
+#include <algorithm>
 #include <type_traits>
 #include <utility>
 
@@ -209,10 +210,12 @@ __device__ __forceinline__ void dft_half_out(float2 *x) {
 // width at compile time (8 or 16) with the element counts exactly the transform's
 // (nin = n/2 pruned or n, nout = n/2 pruned or n: no bounds tests), or 0 (any
 // width and counts, read from the pass).
+constexpr bool pow2(int r) { return (r & (r - 1)) == 0; }
 template <int R1, int R2, bool INV, bool PRUNE, int VW>
-__global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : VW == 8 || !pow2(R1 * R2) ? 2 : 1)
     fft_pass_kernel(FftPass P, int lpb, int pitch_rt, int ahead) {
   constexpr bool EXACT = VW != 0;
+  const int nthr = pow2(R1 * R2) ? kThreads : (int)blockDim.x;
   extern __shared__ __align__(16) float2 sm[];
   __shared__ long long base_in[kMaxLpb], base_out[kMaxLpb], base_nx[kMaxLpb];
   __shared__ int snrow[kMaxLpb];
@@ -252,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
   constexpr int KH = (PRUNE && !INV) ? R1 / 2 : R1;
   const int n1 = (lpb * R2) << lvw;
 #pragma unroll 1
-  for (int i = threadIdx.x; i < n1; i += blockDim.x) {
+  for (int i = threadIdx.x; i < n1; i += nthr) {
     const int v = i & (vw - 1);
     const int q = (i >> lvw) % R2;
     const int g = (i >> lvw) / R2;
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
   // three blocks an SM keep too few loads in flight for the memory's latency (16
   // slices of 512^2 x 32: passes of 172 and 362 us -> 155 and 296, 5.4 TB/s).
   if (VW == 16 && ahead) {
-    for (int i = threadIdx.x; i < lpb * P.nin; i += blockDim.x) {
+    for (int i = threadIdx.x; i < lpb * P.nin; i += nthr) {
       const int g = i / P.nin;
       if (base_nx[g] >= 0)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(P.in + base_nx[g] +
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
   constexpr int PH = (PRUNE && INV) ? R2 / 2 : R2;
   const int n2 = (lpb * R1) << lvw;
 #pragma unroll 1
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+  for (int i = threadIdx.x; i < n2; i += nthr) {
     const int v = i & (vw - 1);
     const int p1 = (i >> lvw) % R1;
     const int g = (i >> lvw) / R1;
@@ -482,10 +485,14 @@ __global__ void __launch_bounds__(kThreads, VW == 16 ? 3 : 2)
 }
 
 // lines per block and the block size whose sweeps over the stages' items (lpb R2
-// vw twice or once, lpb R1 vw) idle least
+// vw twice or once, lpb R1 vw) idle least.  Few lines: fewer per block, so that they
+// lie on more SMs and a thread takes one turn (1D forward, K = 560, 124 lines: 24.9 us
+// in 11 blocks of 12, 15.7 us in 31 of 4)
 template <int R1, int R2>
-void block_shape(int vw, int stages_r2, int *lpb, unsigned *threads) {
+void block_shape(int vw, int stages_r2, long long nlines, int *lpb, unsigned *threads) {
   *lpb = kThreads / ((R1 < R2 ? R1 : R2) * vw);
+  const int least = 64 / ((R1 < R2 ? R1 : R2) * vw) + 1;  // two warps' items
+  if (*lpb > (nlines + 147) / 148) *lpb = std::max(least, (int)((nlines + 147) / 148));
   if (*lpb < 1) *lpb = 1;
   if (*lpb > kMaxLpb) *lpb = kMaxLpb;
   const unsigned n1 = *lpb * R2 * vw, n2 = *lpb * R1 * vw;
@@ -503,11 +510,11 @@ template <int R1, int R2>
 cudaError_t launch_c(const CirculantPass &P, cudaStream_t st) {
   int lpb = 1;
   unsigned threads = kThreads;
-  block_shape<R1, R2>(P.vw, 2, &lpb, &threads);
-  const int pitch = R2 * P.vw + (P.vw < 16 ? P.vw : 0);
-  const size_t smem = (size_t)lpb * R1 * pitch * sizeof(float2);
   const long long nlines = (long long)P.nslice * P.nvec;
   if (nlines <= 0) return cudaSuccess;
+  block_shape<R1, R2>(P.vw, 2, nlines, &lpb, &threads);
+  const int pitch = R2 * P.vw + (P.vw < 16 ? P.vw : 0);
+  const size_t smem = (size_t)lpb * R1 * pitch * sizeof(float2);
   const unsigned grid = (unsigned)((nlines + lpb - 1) / lpb);
   auto kern = P.vw == 16 ? circulant_pass_kernel<R1, R2, 16> : circulant_pass_kernel<R1, R2, 0>;
   cudaError_t e =
@@ -524,12 +531,12 @@ cudaError_t launch_r(const FftPass &P, cudaStream_t st) {
   const int vw = P.vw;
   int lpb = 1;
   unsigned threads = kThreads;
-  block_shape<R1, R2>(vw, 1, &lpb, &threads);
+  const long long nlines = (long long)P.nslice * P.nr2 * P.nr1 * P.nvec;
+  if (nlines <= 0) return cudaSuccess;
+  block_shape<R1, R2>(vw, 1, nlines, &lpb, &threads);
   if (!EXTRA) threads = kThreads;
   const int pitch = R2 * vw + (vw < 16 ? vw : 0);
   const size_t smem = (size_t)lpb * R1 * pitch * sizeof(float2);
-  const long long nlines = (long long)P.nslice * P.nr2 * P.nr1 * P.nvec;
-  if (nlines <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((nlines + lpb - 1) / lpb);
   const bool prune = P.inverse ? (2 * P.nout <= P.n) : (2 * P.nin <= P.n);
   // the exact forms: 16- or 8-wide vectors, inputs and outputs exactly the

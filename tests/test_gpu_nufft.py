@@ -339,6 +339,31 @@ def test_host_adjoint_gives_the_device_adjoints_bits(form, C, nslice):
     plan.close()
 
 
+@pytest.mark.parametrize("N,K", [((448,), (560,)), ((180,), (360,)), ((256,), (512,)), ((40, 50), (80, 100)),
+                                 ((32, 32), (64, 64)), ((33, 24, 40), (80, 64, 96))])
+@pytest.mark.parametrize("C", [1, 5, 16, 31])
+def test_fused_fft_of_few_lines(N, K, C):
+    """One slice, whose few lines spread over more blocks (and narrower vectors), against the same
+    slice in a batch of 40: the same bits forward; the adjoint, whose spread cuts its work by
+    the number of its tiles, to FP32 rounding."""
+    import torch
+    rng = np.random.default_rng(C)
+    D, S, M = len(N), 40, 50
+    om = rng.uniform(-np.pi, np.pi, (M, D))
+    one = mb.NufftPlan(om, N, (6,) * D, K, Ld=64, ncol=C)
+    many = mb.NufftPlan(np.tile(om, (S, 1)), N, (6,) * D, K, Ld=64, ncol=C,
+                        slice_moff=np.arange(S + 1) * M)
+    assert one.fft_config()["fused_fft"] == many.fft_config()["fused_fft"] == 1
+    x = torch.randn(one.image_shape, dtype=torch.complex64, device="cuda")
+    y = torch.randn(one.sample_shape, dtype=torch.complex64, device="cuda")
+    X = many.forward(x.expand((S,) + tuple(x.shape[1:])).contiguous()).view(S, M, C)
+    a = many.adjoint(y.expand((S, M, C)).reshape(S * M, C).contiguous())
+    assert torch.equal(X[0], one.forward(x)) and torch.equal(X[S - 1], X[0])
+    assert rel_l2(one.adjoint(y)[0].cpu().numpy(), a[0].cpu().numpy()) <= 1e-6
+    one.close()
+    many.close()
+
+
 @pytest.mark.parametrize("C", [8, 26])
 def test_launch_count_of_the_atomic_spread(C):
     """set_deterministic(False) moves plans without a sweep from the point or the split spread
