@@ -525,8 +525,8 @@ int line_lists3(mirt_interp_plan *P, cudaStream_t st) {
   {
     DMem cnt;
     CK(cnt.alloc(n.size() * sizeof(int)));
-    CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, nullptr, cnt.as<int>(),
-                          nullptr, nullptr, st));
+    CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock * K1, nullptr, nullptr,
+                          cnt.as<int>(), nullptr, nullptr, st));
     CK(cudaMemcpyAsync(n.data(), cnt.p, n.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
   }
@@ -536,7 +536,11 @@ int line_lists3(mirt_interp_plan *P, cudaStream_t st) {
   // warp's share at full occupancy (so that the heaviest one ends with the others)
   const long long most = std::min<long long>(std::max<long long>(total / (148 * 24 * 8), 64), 1024);
   std::vector<int4> part, fix;
-  std::vector<long long> off(1, 0), boff(nblock);
+  std::vector<long long> off(1, 0);
+  const size_t about = (size_t)(nblock + total / std::max<long long>(most / 2, 1));
+  part.reserve(about);
+  fix.reserve(about);
+  off.reserve(about + 1);
   P->s3_slice_part.assign(S + 1, 0);
   P->s3_slice_fix.assign(S + 1, 0);
   int slots = 0;
@@ -546,7 +550,6 @@ int line_lists3(mirt_interp_plan *P, cudaStream_t st) {
       P->s3_slice_part[b / per] = (int)part.size();
       P->s3_slice_fix[b / per] = (int)fix.size();
     }
-    boff[b] = at;
     const size_t first = part.size();
     const int *v = n.data() + (size_t)b * K1;
     long long run = 0;
@@ -572,14 +575,29 @@ int line_lists3(mirt_interp_plan *P, cudaStream_t st) {
   P->s3_slice_part[S] = (int)part.size();
   P->s3_slice_fix[S] = (int)fix.size();
   const long long np = (long long)part.size();
-  std::vector<int> order(np);
-  for (long long i = 0; i < np; i++) order[i] = (int)i;
-  auto cost = [&](int i) {
-    return (double)(off[i + 1] - off[i]) + kSweepColumnCost * (part[i].z - part[i].y);
-  };
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
-  DMem d_boff;
-  CK(d_boff.alloc(std::max<long long>(nblock, 1) * sizeof(long long)));
+  // heaviest first, ties in index order: the few above 4,096 compared, the others counted
+  // (33,000 parts: 3.8 ms all compared, 0.2 ms so)
+  constexpr int kCounted = 4096;
+  std::vector<long long> cost(np);
+  std::vector<int> order, at_cost(kCounted + 1, 0);
+  order.reserve(np);
+  for (long long i = 0; i < np; i++) {
+    cost[i] = off[i + 1] - off[i] + (long long)kSweepColumnCost * (part[i].z - part[i].y);
+    if (cost[i] >= kCounted)
+      order.push_back((int)i);
+    else
+      at_cost[kCounted - 1 - cost[i]]++;
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+  int first_of = (int)order.size();
+  for (int &c : at_cost) {
+    const int here = c;
+    c = first_of;
+    first_of += here;
+  }
+  order.resize(np);
+  for (long long i = 0; i < np; i++)
+    if (cost[i] < kCounted) order[at_cost[kCounted - 1 - cost[i]]++] = (int)i;
   CK(P->s3_off.alloc(off.size() * sizeof(long long)));
   CK(P->s3_pos.alloc(std::max<long long>(total, 1) * sizeof(int)));
   CK(P->s3_line.alloc(std::max<long long>(total, 1)));
@@ -591,13 +609,13 @@ int line_lists3(mirt_interp_plan *P, cudaStream_t st) {
   auto up = [&](DMem &d, const void *p, size_t bytes) {
     return bytes ? cudaMemcpyAsync(d.p, p, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
   };
-  CK(up(d_boff, boff.data(), boff.size() * sizeof(long long)));
   CK(up(P->s3_off, off.data(), off.size() * sizeof(long long)));
   CK(up(P->s3_part, part.data(), part.size() * sizeof(int4)));
   CK(up(P->s3_fix, fix.data(), fix.size() * sizeof(int4)));
   CK(up(P->team_order, order.data(), order.size() * sizeof(int)));
-  CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, nblock, d_boff.as<long long>(),
-                        nullptr, P->s3_pos.as<int>(), P->s3_line.as<unsigned char>(), st));
+  CK(launch_sweep3_list(a, t, P->bin_start.as<int>(), B2, B3, np, P->s3_part.as<int4>(),
+                        P->s3_off.as<long long>(), nullptr, P->s3_pos.as<int>(),
+                        P->s3_line.as<unsigned char>(), st));
   CK(cudaStreamSynchronize(st));
   t.s3_pos = P->s3_pos.as<int>();
   t.s3_line = P->s3_line.as<unsigned char>();
@@ -727,12 +745,11 @@ int build_points(mirt_interp_plan *P, cudaStream_t st) {
 }
 
 // No point or split spread: what their lists have found room for is given back.
-void drop_points(mirt_interp_plan *P) {
+void drop_lists(mirt_interp_plan *P) {
   Tiling &t = P->t;
-  for (DMem *d : {&P->wsw, &P->pt_task, &P->pt_slice_task, &P->pt_hdr, &P->pt_scratch, &P->pt_count,
+  for (DMem *d : {&P->pt_task, &P->pt_slice_task, &P->pt_hdr, &P->pt_scratch, &P->pt_count,
                   &P->split_teams, &P->split_order, &P->split_next})
     d->release();
-  t.wsw = nullptr;
   t.points = t.split = t.split_nteams = t.n_pt_task = t.pt_slots = 0;
   P->points_shape = P->split_ok = 0;
 }
@@ -789,7 +806,7 @@ Spread2D choose_spread2d(const mirt_interp_plan *P, const std::vector<int> &most
 // evenly go to the point spread, which splits them over groups and CTAs; the
 // bands of four rows between them are cut into segments of about a quarter of a
 // warp's share of the whole cost (at least eight columns).
-int build_split(mirt_interp_plan *P, cudaStream_t st) {
+int build_split(mirt_interp_plan *P, cudaStream_t st, bool for_autotune = false) {
   const InterpArgs &a = P->a;
   Tiling &t = P->t;
   constexpr int kRows = 4, kWarps = 148 * 16;
@@ -809,8 +826,11 @@ int build_split(mirt_interp_plan *P, cudaStream_t st) {
   for (float v : vb) total += v + kSweepColumnCost;
   const double share = std::max(1.0, total * nch / kWarps);
   const int dense = (int)std::min(kSplitMost, std::max(64.0, kSplitDense * share));
-  const Spread2D form = P->ls.cw == 32 ? choose_spread2d(P, most, dense)
-                                       : Spread2D::split;
+  const Spread2D form = P->ls.cw == 32 ? choose_spread2d(P, most, dense) : Spread2D::split;
+  if (form == Spread2D::row && !for_autotune) {
+    P->pt_hdr.release();
+    return MIRT_OK;
+  }
   if (form == Spread2D::points) {
     P->points_shape = shape;
     return build_point_tasks(P, shape, most, -1, st);
@@ -881,7 +901,7 @@ int build_split(mirt_interp_plan *P, cudaStream_t st) {
   t.split_next = P->split_next.as<int>();
   rc = build_point_tasks(P, shape, most, dense, st);
   if (rc) return rc;
-  P->split_ok = 1;  // (the autotuner tries it where it is not the default)
+  P->split_ok = 1;
   t.split = form == Spread2D::split;
   if (!t.split) t.points = 0;
   return MIRT_OK;
@@ -1433,8 +1453,14 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
   if (sweep_ok(a, P->t) && a.C >= kSplitColumns) {
     int rc3 = build_sweep_records(P, st);
     if (!rc3) rc3 = build_split(P, st);
-    if (rc3 == MIRT_ERR_ALLOC) drop_points(P);
-    else if (rc3) return rc3;
+    if (rc3 && rc3 != MIRT_ERR_ALLOC) return rc3;
+    if (rc3) {
+      drop_lists(P);
+      if (P->ls.cw != 32) {  // (else the staged row sweep's)
+        P->wsw.release();
+        P->t.wsw = nullptr;
+      }
+    }
   }
   // 3D, J = 6, coil chunks of 8, 16 or 32: few samples on a small grid the point spread,
   // whose one launch is done before the line sweep has run its five (48^3, 8 coils, 300
@@ -1445,7 +1471,7 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
     P->t.sweep = 2;  // beneath it
     int rc3 = build_points(P, st);
     if (rc3 && rc3 != MIRT_ERR_ALLOC) return rc3;
-    if (rc3) drop_points(P);
+    if (rc3) drop_lists(P);
     if (!P->t.points) P->t.sweep = 0;
   }
   if (sweep3_ok(a, P->t, P->ls.cw) && !P->t.points) {
@@ -1455,16 +1481,16 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
   // everything else: the point spread
   if (!P->t.sweep && !P->t.split && a.C > 0) {
     int rc3 = build_points(P, st);
-    if (rc3 == MIRT_ERR_ALLOC) drop_points(P);
+    if (rc3 == MIRT_ERR_ALLOC) drop_lists(P);
     else if (rc3) return rc3;
   }
   if (P->t.sweep >= 0 || P->t.points) return MIRT_OK;
   int rc4 = row_sweep_ready(P, st);
-  if (rc4 == MIRT_ERR_ALLOC && P->split_ok) {  // without the autotuner's split lists
-    drop_points(P);
-    rc4 = row_sweep_ready(P, st);
-  }
-  return rc4;
+  if (rc4 != MIRT_ERR_ALLOC) return rc4;
+  for (DMem *d : {&P->swept, &P->patch, &P->patch_part}) d->release();
+  P->t.sorted = P->t.patch = P->t.patch_part = nullptr;
+  P->t.sweep = 0;
+  return MIRT_OK;
 }
 
 // Re-tile the spread (tiles of T[d] points, multiples of the sort bins) and
@@ -1760,6 +1786,18 @@ int mirt_interp_plan_autotune(mirt_interp_plan *P, void *stream) try {
                  sweep_ok(a, P->t) && cw == 32 ? -1 : 0, 1};
     c.points = P->points_shape;
     cands.push_back(c);
+  }
+  // the split spread's lists where the row sweep is the default (with points on all
+  // tiles there are no lists of the dense ones)
+  if (D == 2 && cw == 32 && P->t.wsw && !P->split_ok && !P->points_shape) {
+    const Tiling before = P->t;
+    if (build_split(P, st, true)) {
+      P->t = before;
+      drop_lists(P);
+    } else {
+      P->t.points = before.points;
+      P->t.split = before.split;
+    }
   }
   if (P->split_ok) {
     SpreadCand c{{P->t.T[0], P->t.T[1], P->t.T[2]}, P->ls.threads, 0, 0, 0, cw == 32 ? -1 : 0, 1};

@@ -199,17 +199,20 @@ cudaError_t radix_sort_bins(const uint32_t *keys, long long n, int nbins, void *
 // visit lists of the 3D line sweep
 // ------------------------------------------------------------------------
 namespace {
-// One warp a block: per bin column, the samples of the bin lines around the block
-// (lane l keeps lines l and l + 32) in line and sort order, then the column's dense
-// bins in line order.
+// Per bin column, the samples of the bin lines around the block (lane l keeps lines l
+// and l + 32) in line and sort order, then the column's dense bins in line order: one
+// warp a column counts them (count), one warp a part lists its columns (64^3, a million
+// samples: 84 and 167 us).
 __global__ void sweep3_list_kernel(InterpArgs a, Tiling t, const int *__restrict__ bin_start, int B2,
-                                   int B3, long long nblock, const long long *__restrict__ off,
-                                   int *__restrict__ count, int *__restrict__ pos,
-                                   unsigned char *__restrict__ line) {
-  const long long block = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  if (block >= nblock) return;
+                                   int B3, long long n, const int4 *__restrict__ part,
+                                   const long long *__restrict__ off, int *__restrict__ count,
+                                   int *__restrict__ pos, unsigned char *__restrict__ line) {
+  const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  if (i >= n) return;
   const int lane = threadIdx.x & 31;
   const int K1 = a.g.K[0], K2 = a.g.K[1], K3 = a.g.K[2];
+  const int4 pt = count ? make_int4((int)(i / K1), (int)(i % K1), (int)(i % K1) + 1, 0) : part[i];
+  const long long block = pt.x;
   const int Q2 = B2 + 5, nl = Q2 * (B3 + 5);
   const int nby = (K2 + B2 - 1) / B2, nbz = (K3 + B3 - 1) / B3;
   const int y0 = (int)(block % nby) * B2;
@@ -226,9 +229,8 @@ __global__ void sweep3_list_kernel(InterpArgs a, Tiling t, const int *__restrict
     if (z < 0) z += K3;
     base[h] = l < nl ? ((long long)z * K2 + r) * K1 : -1;
   }
-  long long at = off ? off[block] : 0;
-  for (int x = 0; x < K1; x++) {
-    const long long at0 = at;
+  long long at = count ? 0 : off[i];
+  for (int x = pt.y; x < pt.z; x++) {
     for (int h = 0; h < 2; h++) {
       const int b0 = base[h] >= 0 ? bs[base[h] + x] : 0;
       const int n = base[h] >= 0 ? bs[base[h] + x + 1] - b0 : 0;
@@ -255,17 +257,17 @@ __global__ void sweep3_list_kernel(InterpArgs a, Tiling t, const int *__restrict
       }
       at += __popc(m);
     }
-    if (count && lane == 0) count[block * K1 + x] = (int)(at - at0);
   }
+  if (count && lane == 0) count[i] = (int)at;
 }
 }  // namespace
 
 cudaError_t launch_sweep3_list(const InterpArgs &a, const Tiling &t, const int *bin_start, int B2,
-                               int B3, long long nblock, const long long *off, int *count, int *pos,
-                               unsigned char *line, cudaStream_t st) {
-  if (nblock <= 0) return cudaSuccess;
-  sweep3_list_kernel<<<(unsigned)((nblock + 7) / 8), 256, 0, st>>>(a, t, bin_start, B2, B3, nblock,
-                                                                  off, count, pos, line);
+                               int B3, long long n, const int4 *part, const long long *off,
+                               int *count, int *pos, unsigned char *line, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  sweep3_list_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(a, t, bin_start, B2, B3, n, part, off,
+                                                             count, pos, line);
   return cudaGetLastError();
 }
 

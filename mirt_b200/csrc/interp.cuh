@@ -202,11 +202,11 @@ struct GatherBlocks {
 };
 // float2 of a part's tail slot: 5 columns x 2 lines a lane x 32 lanes
 constexpr int kSweep3Tail = 5 * 2 * 32;
-// The 3D line sweep's visit lists for blocks of B2 x B3 lines: counts per block and
-// column (off null), or the lists from the blocks' offsets.
+// The 3D line sweep's visit lists for blocks of B2 x B3 lines: the counts of n columns
+// (block-major; count given), or the lists of n parts from the parts' offsets.
 cudaError_t launch_sweep3_list(const InterpArgs &a, const Tiling &t, const int *bin_start, int B2,
-                               int B3, long long nblock, const long long *off, int *count, int *pos,
-                               unsigned char *line, cudaStream_t st);
+                               int B3, long long n, const int4 *part, const long long *off,
+                               int *count, int *pos, unsigned char *line, cudaStream_t st);
 bool gather_tma_ok(const InterpArgs &a);
 bool gather_tma_default(const InterpArgs &a, long long nitem);
 int gather_tma_block();
