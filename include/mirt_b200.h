@@ -284,16 +284,16 @@ int mirt_interp_plan_set_ownership(mirt_interp_plan *plan, int32_t own, void *st
  * tiles, shared memory or reduction launches.  segments: 1..K1 uniform
  * segments per row (more segments, more parallel teams, five warm-up columns
  * each); -1 a balanced team list built from the sort's bins (rows cut into
- * segments of about equal visit counts, about 64k teams: the default for
- * 32-coil plans); 0 returns to the tiled spread.  Teams are taken by the
+ * segments of about equal visit counts, about 64k teams: the row sweep's
+ * default for 32-coil plans); 0 returns to the tiled spread.  Teams are taken by the
  * kernel's warps from a work queue, heaviest first.  3D plans (J = 6, K >= 6
  * per dimension, coil chunks of 8, 16 or 32): the line sweep, in which a
  * warp owns a block of 4 x 2, 4 x 1 or 2 x 1 grid lines along k1 (lanes = coils
  * x pairs of lines) and a part of their columns, and sums the samples of the bin
  * lines around the block, listed by column in the plan, with six columns of
  * accumulators per line in registers (any segments in 1..K1 turn it on; the parts
- * follow the samples; rows unused; the default there, reported as
- * two segments).  MIRT_ERR_ARG where it does not apply.  The autotuner tries
+ * follow the samples; rows unused; the default there but for few samples on a small
+ * grid, which take the point spread; reported as two segments).  MIRT_ERR_ARG where it does not apply.  The autotuner tries
  * it where it applies.  No reference counterpart. */
 int mirt_interp_plan_set_sweep(mirt_interp_plan *plan, int32_t segments, int32_t rows);
 

@@ -253,10 +253,10 @@ int sweep_buffer(mirt_interp_plan *P) {
   return MIRT_OK;
 }
 
-// Columns from which the split spread is the default (2D, J = 6): its sweep's
+// Columns from which the split spread is a default (2D, J = 6): its sweep's
 // lanes are 32 columns whatever their use, while the point spread's chunks fit
 // the columns (20 columns, 115,968 samples on 384^2: 151 against 139 us; 24
-// columns, 145,920 on 5 x 384^2: 203 and 200 us; 32 columns, 204,800 on 512^2:
+// columns, 145,920 on 5 x 384^2: 203 and 197 us; 32 columns, 204,800 on 512^2:
 // 240 us against 313 us of the unstaged sweep with dense-bin patches).
 constexpr int kSplitColumns = 25;
 // 3D: most samples, and most grid points times chunks of 32 columns, of the point
@@ -300,7 +300,7 @@ int sweep_band_visits(mirt_interp_plan *P, int rows, cudaStream_t st, std::vecto
 
 // Split spread: a tile is dense when a brick of it takes more samples than one
 // warp's share of the whole cost (heaviest teams run first, so a team up to that
-// share ends with the rest), and a team takes about a third of a share.  Measured
+// share ends with the rest), and a team takes up to a third of a share.  Measured
 // on batches of 1, 4, 16 and 64 slices (K = 512^2, 32 columns): shares of 0.3, 0.6,
 // 1.0, 1.5 and 2.5 give 299, 240, 254, 250, 327 us (1), 484, 457, 443, 553, 572 us
 // (4) and 1372, 1346, 1393, 1573, 1535 us (16); teams of 1/2, 1/4, 1/8 share 4667,
@@ -804,7 +804,7 @@ Spread2D choose_spread2d(const mirt_interp_plan *P, const std::vector<int> &most
 
 // Split spread: the plane's tiles that a band's segment could not share out
 // evenly go to the point spread, which splits them over groups and CTAs; the
-// bands of four rows between them are cut into segments of about a quarter of a
+// bands of four rows between them are cut into segments of up to a third of a
 // warp's share of the whole cost (at least eight columns).
 int build_split(mirt_interp_plan *P, cudaStream_t st, bool for_autotune = false) {
   const InterpArgs &a = P->a;
@@ -1373,8 +1373,7 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
       t4.nbins *= t4.nbin[d];
     }
     const long long nb4 = (long long)t4.nbins * nslice;
-    DMem keys4, tmp4;
-    DMem &bs4 = P->gblk;
+    DMem keys4, tmp4, bs4;
     CK(keys4.alloc(Mtot * sizeof(uint32_t)));
     CK(bs4.alloc((nb4 + 1) * sizeof(int)));
     CK(tmp4.alloc(radix_sort_tmp_bytes(Mtot)));
@@ -1433,8 +1432,8 @@ int plan_finish(mirt_interp_plan *P, long long Mtot, const long long *moff, int 
   int rc2 = build_tasks(P, st);
   if (rc2) return rc2;
   CK(query_gather_grid(a, P->lg));
-  // 2D, J = 6, 32-coil chunks: the row sweep by default, one grid row per
-  // team, balanced segments (about 64k teams, heaviest first)
+  // The sweeps' dense bins; 2D, J = 6, 32-coil chunks: the row sweep, one grid row per
+  // team, balanced segments (about 64k teams, heaviest first), or a spread on top of it
   if (sweep_ok(a, P->t) || sweep3_ok(a, P->t, P->ls.cw)) {
     int rc3 = build_dense(P, kDenseBin, st);
     if (rc3) return rc3;

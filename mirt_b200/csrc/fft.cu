@@ -10,7 +10,8 @@ namespace {
 
 // Transform lengths n = R1 R2.  R1 and R2 are multiples of 4 where the length
 // allows it (a folded grid phase needs it, fft_fold_ok); the lengths off the powers of
-// two are those of the usual image sizes (N = 40 .. 448 in steps of 8 to 32) at K = 2 N.
+// two are K = 2 N of 26 usual image sizes N between 40 and 448; others that the same
+// radices would give (140, 168, 180, 196, 216, 252, 324, 392, 432, 504) are left to cuFFT.
 struct FftLen {
   int n, r1, r2, unit;  // unit: the translation unit that instantiates it (0: here)
 };

@@ -130,7 +130,7 @@ struct Tiling {
   float2 *pt_scratch;
   int *pt_count;
   const int4 *pt_hdr;    // per position: first tap k1, caller's sample index, phase (float bits)
-  // Split spread (2D, J = 6, many columns): the staged row sweep over the team
+  // Split spread (2D, J = 6, 25 columns and more): the staged row sweep over the team
   // list `split_team` (bands of four rows, segments of their columns, slice after
   // slice; split_order: heaviest first, null in place), which leaves out the dense
   // tiles; the point spread's tasks are those
@@ -187,14 +187,12 @@ struct Launch {
 };
 
 // The gather over TMA-staged grid tiles and records (gather_tma.cu): 2D, J = 6,
-// C even and >= 32, K >= 13 per dimension; or 3D, J = 6, C even and >= 8,
+// C even and >= 16, K >= 13 per dimension; or 3D, J = 6, C even and >= 8,
 // K >= 9 per dimension.  Samples in the gather order are grouped by blocks of
-// gb points per dimension of their first taps; start[b] is the first position
-// of block b = ((slice * nbz + bz) * nby + by) * nbx + bx (start[nblocks] =
-// Mtot); a work item (block, first position) covers up to gather_tma_item()
-// (3D: gather_tma3_item()) samples of one block, items in block order;
-// orec[pos] = (caller's sample index, 0, phase as float bits), staged with the
-// tap records.
+// gb points per dimension of their first taps; a work item is up to
+// gather_tma_item() (3D: gather_tma3_item()) samples of one block b = ((slice *
+// nbz + bz) * nby + by) * nbx + bx, items in block order; orec[pos] = (caller's
+// sample index, 0, phase as float bits), staged with the tap records.
 struct GatherBlocks {
   const int4 *item;  // block (slice-major), first position, samples
   const int4 *orec;

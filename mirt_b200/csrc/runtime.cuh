@@ -71,7 +71,7 @@ struct mirt_interp_plan {
   mirt::DMem wtap_g, k0tap_g, perm_g, phase_g;
   mirt::DMem orec_g;        // TMA gather: output records (sample index, phase) in gather order
   mirt::DMem wsw;           // staged 2D row sweep: tap records with FFMA2 operand pairs, plan order
-  mirt::DMem swept;        // row-sweep spread: the samples in plan order, [Mtot][C]
+  mirt::DMem swept;        // the sweeps: the samples in plan order, [Mtot][C]
   mirt::DMem sweep_teams;  // row-sweep spread: balanced team list (int4 per team)
   int team_rows = 0;       // rows per band of the list (0: none, or its order is another's)
   // 3D line sweep: the parts' visit lists and records, first part / fix of each slice
@@ -90,9 +90,9 @@ struct mirt_interp_plan {
   std::vector<int> dense_slice;           // first dense bin of each slice (+ total)
   long long dense_samples = 0;            // samples in dense bins
   std::vector<int> dense_part0_host;      // first chunk of each dense bin (+ total)
-  // TMA gather: first position of each block of the gather order, work items
-  // (block, first position, samples), the first item of each slice, fault flag
-  mirt::DMem gblk, gitem, gfault;
+  // TMA gather: work items (block, first position, samples), the first item of
+  // each slice, fault flag
+  mirt::DMem gitem, gfault;
   std::vector<long long> gitem_slice;
   mirt::GatherBlocks gbk{};
   int gtma = 0;            // the gather's TMA-staged tiles: 1 of 32 coils (3D: 8), 2 of 16

@@ -29,7 +29,7 @@
 // whose 32 lanes held the 6 taps of one column and whose warps walked a dense
 // tile alone: 2D, one column, 8,192 samples on K = 128^2 1314 -> 15 us; 491,520
 // samples on 6 x 512^2 1730 -> 110 us; 16 columns, 115,968 samples on 384^2 2457
-// -> 112 us; 24 columns, 145,920 samples on 5 x 384^2 2481 -> 215 us (the
+// -> 112 us; 24 columns, 145,920 samples on 5 x 384^2 2481 -> 197 us (the
 // unstaged row sweep with its dense-bin patches 570 us there); 3D, one column,
 // 216,000 samples on 144 x 120 x 96 4530 -> 287 us.
 #include <algorithm>

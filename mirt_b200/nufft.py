@@ -171,15 +171,17 @@ class InterpPlan:
         """Row-sweep spread (2D, J = 6; see mirt_interp_plan_set_sweep):
         uniform segments per grid row (True = 1; 0 / False = tiled spread;
         -1 = balanced team list) and grid rows per band (1, 2 or 4).  3D
-        plans (J = 6, coil chunks of 8, 16 or 32): the line sweep with
-        `segments` uniform segments per line block (rows unused)."""
+        plans (J = 6, coil chunks of 8, 16 or 32): any `segments` turns the
+        line sweep on, whose parts follow the samples (rows unused)."""
         check(self.lib.mirt_interp_plan_set_sweep(self.handle, int(segments), int(rows)))
         return self.config()
 
     def set_gather(self, tma=True):
-        """TMA-staged gather (2D, J = 6, even C >= 32) or the plain gather
-        (see mirt_interp_plan_set_gather): True / 1 tiles of 32 coils, 2 tiles
-        of 16 coils, False / 0 the plain gather."""
+        """TMA-staged gather (2D, J = 6, even C >= 32; 3D, J = 6, even C >= 8)
+        or the plain gather (see mirt_interp_plan_set_gather): True / 1 tiles
+        of 32 coils (3D: 8), 2 tiles of 16 coils (2D), False / 0 the plain
+        gather.  2D plans of 16 to 30 columns choose by their samples; for
+        them only 0 can be set here, the autotuner times both."""
         check(self.lib.mirt_interp_plan_set_gather(self.handle, int(tma)))
         return self.config()
 
