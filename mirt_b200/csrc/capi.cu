@@ -303,8 +303,9 @@ int sweep_band_visits(mirt_interp_plan *P, int rows, cudaStream_t st, std::vecto
 // share ends with the rest), and a team takes up to a third of a share.  Measured
 // on batches of 1, 4, 16 and 64 slices (K = 512^2, 32 columns): shares of 0.3, 0.6,
 // 1.0, 1.5 and 2.5 give 299, 240, 254, 250, 327 us (1), 484, 457, 443, 553, 572 us
-// (4) and 1372, 1346, 1393, 1573, 1535 us (16); teams of 1/2, 1/4, 1/8 share 4667,
-// 4532, 4545 us (64).
+// (4) and 1372, 1346, 1393, 1573, 1535 us (16); teams of 1/2, 1/3, 1/4 share 190, 200,
+// 177 us (1), 440, 450, 462 us (4), 1321, 1320, 1336 us (16), 4990, 4936, 4798 us (64);
+// 400^2, 128 columns, 48,000 samples: 172 us by thirds, 199 by quarters.
 constexpr double kSplitDense = 1.0, kSplitTeams = 3;
 // ... and in any case when a brick (a window of 81 bins, 36 of them a point's)
 // takes more than this many, so that no point of the sweep sums over about 450
