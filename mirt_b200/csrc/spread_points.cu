@@ -169,9 +169,10 @@ __global__ void point_count_kernel(InterpArgs a, Tiling t, PtTile pt, int ngrp,
 // group's share (chunks part, part + 2^lg, ... of S samples of the brick's runs) in
 // the walk's order and operations: X points from (x, y, z), columns c, c + cw, ...
 // below C.  Called where the walk left a sum that is not finite; kept out of line, so
-// that the walk's registers don't pay for it (one real column, 63,114 samples on 402 x
-// 350: 22.9 -> 23.6 us, 16 columns on 384^2 112.0 -> 111.2; a test in the walk cost 2 to
-// 5 % of the one- to 24-column passes).
+// that the walk's registers don't pay for it (without and with it: one real column,
+// 63,114 samples on 402 x 350 22.0 and 23.0 us; 12 columns on 6 x 512^2 481 and 502; 16 on
+// 384^2 121 and 118; 24 on 5 x 384^2 197 and 199; a test in the walk cost 2 to 5 % of the
+// one- to 24-column passes).
 template <int D, int NC, bool REAL>
 __device__ __noinline__ void points_redo(const InterpArgs &a, const Tiling &t, const int *bin_start,
                                          const float2 *fm, int slice, int X0, int Y0, int Z0, int bw,
@@ -431,12 +432,15 @@ __global__ void __launch_bounds__(PT_THREADS, D == 3 ? 5 : NC <= 2 ? 8 : 6)
   // A block's four points take the zeros beside the taps as well, which would make NaN
   // of an infinite or NaN product.  Such a product never leaves a sum finite.
   {
-    float chk = 0.f;  // 0 x of any sum: NaN where one is not finite
+    float chk[X] = {};  // 0 x of any sum: NaN where one is not finite; four short chains
 #pragma unroll
     for (int m = 0; m < NC; m++)
 #pragma unroll
-      for (int k = 0; k < X; k++) chk = fmaf(0.f, acc[m][k].x, fmaf(0.f, acc[m][k].y, chk));
-    if (__builtin_expect(chk != 0.f, 0)) {
+      for (int k = 0; k < X; k++)
+        chk[k] = fmaf(0.f, acc[m][k].x, fmaf(0.f, acc[m][k].y, chk[k]));
+    static_assert(X == 4, "sums of a block");
+    const float bad = (chk[0] + chk[1]) + (chk[2] + chk[3]);
+    if (__builtin_expect(bad != 0.f, 0)) {
       float2 again[NC * X];
       points_redo<D, NC, REAL>(a, t, bin_start, fm, slice, X0, Y0, Z0, BX * X, BY, BZ, part, lg, S,
                                X0 + bx, Y0 + by, Z0 + bz, c0 + cl, CW, again);
