@@ -165,10 +165,21 @@ def traffic_from_profiles(workload, kernel):
             t = json.load(f)
         e = t.get(workload, {}).get(kernel)
         if e:
-            return e["bytes"], "profiles/traffic.json: " + e["source"]
+            return e["bytes"], e["source"]
     except (OSError, ValueError, KeyError):
         pass
     return None, None
+
+
+def rounded(v):
+    """`v` with its floats at seven digits, for a result line of one screen."""
+    if isinstance(v, float):
+        return float(f"{v:.7g}")
+    if isinstance(v, dict):
+        return {k: rounded(e) for k, e in v.items()}
+    if isinstance(v, (list, tuple)):
+        return [rounded(e) for e in v]
+    return v
 
 
 # ---------------------------------------------------------------------------
@@ -442,10 +453,15 @@ def run_gpu(args, w):
     variant = {"spread": "sweep" if tuned.get("spread_sweep", 0) != 0 else "tiled",
                "gather": "tma" if tuned.get("gather_tma", 0) else "plain"}
     rows, staged = tuned.get("spread_sweep_rows", 1), tuned.get("spread_staged", 0)
+    # the split and the point spread lie on top of the sweep or the tiled spread,
+    # which runs in their place only when the spread is asked to be atomic
+    top = variant["spread"] == "sweep" or not tuned.get("spread_atomic")
+    if top and tuned.get("spread_split", 0):
+        variant["spread"] = "split"
+    elif top and tuned.get("spread_points", 0):
+        variant["spread"] = "points"
     if D == 3:
         sweep_kernel = "spread_sweep3_kernel"
-    elif tuned.get("spread_split", 0):
-        sweep_kernel = "spread_sweep2s_kernel + spread_points_kernel (dense tiles)"
     elif staged == 2:
         sweep_kernel = f"spread_sweep2s_kernel rows={rows} (caller-order samples)"
     elif staged == 1:
@@ -453,10 +469,12 @@ def run_gpu(args, w):
     else:
         sweep_kernel = f"sweep_order_kernel + spread_sweep_kernel rows={rows}"
     tma_coils = 16 if tuned.get("gather_tma", 0) == 2 else 32
-    kernels = {"gather": (f"gather_tma_kernel ({tma_coils}-coil tiles)" if variant["gather"] == "tma"
-                          else "gather_kernel"),
-               "spread": (sweep_kernel if variant["spread"] == "sweep"
-                          else "spread_kernel (+ spread_reduce_kernel)")}
+    kernels = {"gather": ("gather_kernel" if variant["gather"] != "tma"
+                          else "gather_tma3_kernel" if D == 3
+                          else f"gather_tma_kernel ({tma_coils}-coil tiles)"),
+               "spread": {"sweep": sweep_kernel, "points": "spread_points_kernel",
+                          "split": "spread_sweep2s_kernel + spread_points_kernel (dense tiles)",
+                          "tiled": "spread_kernel (+ spread_reduce_kernel)"}[variant["spread"]]}
     traffic, traffic_src = traffic_from_profiles(args.workload, kernels[dom])
     roof = {"bound": "hbm", "kernel": kernels[dom], "achieved": achieved, "peak": peak,
             "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
@@ -519,6 +537,10 @@ def run_gpu(args, w):
     cg = None
     if rank == 0 and world == 1 and not args.no_cg and w["D"] == 2:
         cg = run_cgsense(args)
+        # the groups one by one are 20 KB: not in the result line
+        per_group = cg.pop("per_group")
+        if args.cg_groups:
+            print(json.dumps({"cg_sense_per_group": per_group}), file=sys.stderr, flush=True)
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
@@ -540,7 +562,7 @@ def run_gpu(args, w):
             "gpu_launches": launches_per_step * args.steps, "clocks": clk,
             "cg_sense": cg,
         }
-        print(json.dumps(line), flush=True)
+        print(json.dumps(rounded(line), separators=(",", ":")), flush=True)
     if graph is not None:
         graph.close()
     plan.close()
@@ -702,6 +724,8 @@ def run_cgsense(args):
         per.append(res)
         A.close()
         del G, G1
+    # the reference solution: FP32 operators, FP64 inner products; within 1e-4 of the FP64
+    # solution on the parity cases
     out = {"metric": "CG-SENSE s to NRMSE 1e-3 (every problem of the batch)",
            "problems": args.cg_problems, "groups": len(per), "max_iters": args.cg_iters}
     for k in modes:
@@ -711,8 +735,7 @@ def run_cgsense(args):
         "mlp_tensor_core_ms": sum(r["mlp_tensor_core_ms"] for r in per),
         "mlp_fp32_pipes_ms": sum(r["mlp_fp32_pipes_ms"] for r in per),
         "plan_and_toeplitz_setup_s": setup_s,
-        "reference": f"{args.cg_ref} preconditioned CG iterations from zero (FP32 operators, "
-                     "FP64 inner products; within 1e-4 of the FP64 solution on the parity cases)",
+        "reference": f"{args.cg_ref} preconditioned CG iterations from zero",
         "per_group": per})
     return out
 
@@ -741,6 +764,8 @@ def main():
                     help="let the spread add with shared-memory atomics (not bitwise reproducible)")
     ap.add_argument("--cpu-seconds", type=float, default=12.0)
     ap.add_argument("--no-cg", action="store_true", help="skip the CG-SENSE comparison")
+    ap.add_argument("--cg-groups", action="store_true",
+                    help="print the CG-SENSE comparison's groups one by one on stderr")
     ap.add_argument("--cg-problems", type=int, default=64)
     ap.add_argument("--cg-iters", type=int, default=60)
     ap.add_argument("--cg-ref", type=int, default=300)
